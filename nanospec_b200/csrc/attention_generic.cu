@@ -4,7 +4,8 @@
 // accurate expf, and the keys of one query are always visited in the same order (ascending
 // from the first key it may see, 32 at a time), so a query's output does not depend on how
 // the batch was cut into steps or on what else runs beside it.  The true 32-bit path uses
-// it for every step; the bfloat16 path uses it for sizes that the tensor-core kernels refuse.
+// it for decode tokens, windows and chunks (csrc/attention_f32.cu gives the same bits for portions of prompts that see every
+// key); the bfloat16 path uses it for sizes that the tensor-core kernels refuse.
 //
 // A query at position p of request r sees the keys at positions max(0, p - window + 1) .. p
 // of the same request (window == 0: all of 0 .. p) and, with keep_first > 0, also the keys at
@@ -28,14 +29,14 @@ attention_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restr
                          const int* __restrict__ token_req, const int* __restrict__ positions, T* __restrict__ out,
                          int o_stride, int n_tokens, int nq, int nkv, int d, int dv, int page_size, float scale, int window,
                          int keep_first, int chunk, float softcap, const float* __restrict__ sink,
-                         const T* __restrict__ gate, int gate_stride, int gate_per_feature, float out_scale) {
+                         const T* __restrict__ gate, int gate_stride, int gate_per_feature, float out_scale, const int* __restrict__ rows) {
     ns_pdl_launch_dependents();  // the next kernel may be scheduled now; it waits for this one before it reads
     ns_pdl_wait();               // everything below sees the previous kernel's results
     extern __shared__ float qsm[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const long long w = (long long)blockIdx.x * kWarpsPerBlock + wib;
     if (w >= (long long)n_tokens * nq) return;
-    const int n = (int)(w / nq), h = (int)(w % nq);
+    const int n = rows ? rows[w / nq] : (int)(w / nq), h = (int)(w % nq);
     T* o = out + (size_t)n * o_stride + (size_t)h * dv;
     const int req = token_req[n];
     if (req < 0) return;
@@ -116,7 +117,7 @@ template <typename T>
 int launch(const void* q, int q_stride, const void* k_cache, const void* v_cache, const int* block_table,
            int table_stride, const int* token_req, const int* positions, void* out, int o_stride, int n_tokens, int nq,
            int nkv, int d, int dv, int page_size, float scale, int window, int keep_first, int chunk, float softcap,
-           const float* sink, const void* gate, int gate_stride, int gate_per_feature, float out_scale, cudaStream_t stream) {
+           const float* sink, const void* gate, int gate_stride, int gate_per_feature, float out_scale, const int* rows, cudaStream_t stream) {
     const long long warps = (long long)n_tokens * nq;
     const unsigned blocks = (unsigned)((warps + kWarpsPerBlock - 1) / kWarpsPerBlock);
     const size_t smem = (size_t)kWarpsPerBlock * d * sizeof(float);
@@ -127,7 +128,7 @@ int launch(const void* q, int q_stride, const void* k_cache, const void* v_cache
         NS_LAUNCH((attention_generic_kernel<T, D>), blocks, kWarpsPerBlock * 32, smem, stream,                                \
             (const T*)q, q_stride, (const T*)k_cache, (const T*)v_cache, block_table, table_stride, token_req,       \
             positions, (T*)out, o_stride, n_tokens, nq, nkv, d, dv, page_size, scale, window, keep_first, chunk, softcap, \
-            sink, (const T*)gate, gate_stride, gate_per_feature, out_scale);                                                                    \
+            sink, (const T*)gate, gate_stride, gate_per_feature, out_scale, rows);                                                                    \
         break;
     switch (dpl) {
         NS_ATTN_CASE(1) NS_ATTN_CASE(2) NS_ATTN_CASE(3) NS_ATTN_CASE(4)
@@ -144,12 +145,12 @@ int launch(const void* q, int q_stride, const void* k_cache, const void* v_cache
 // `sink` (optional, float [nq]): every query's denominator also holds exp(sink[h]), a term without key or value (zeros: "one
 // added to the denominator").  `gate` (optional, the activations' type, one number per token and head at
 // gate[n * gate_stride + h]): head h's output is multiplied by its sigmoid; with gate_per_feature every feature has its own, at
-// gate[n * gate_stride + h * dv + e].  `out_scale` multiplies every output.
+// gate[n * gate_stride + h * dv + e].  `out_scale` multiplies every output.  `rows` (or null): the n_tokens token rows to run.
 NS_API int ns_attention_generic_sink(const void* q, int q_stride, const void* k_cache, const void* v_cache,
                                 const int* block_table, int table_stride, const int* token_req, const int* positions,
                                 void* out, int o_stride, int n_tokens, int nq, int nkv, int d, int dv, int page_size,
                                 float scale, int window, int keep_first, int chunk, float softcap, const float* sink,
-                                const void* gate, int gate_stride, int gate_per_feature, float out_scale, int dtype, cudaStream_t stream) {
+                                const void* gate, int gate_stride, int gate_per_feature, float out_scale, const int* rows, int dtype, cudaStream_t stream) {
     if (n_tokens <= 0) return NS_OK;
     if (d < 1 || d > 512 || dv < 1 || dv > 512)
         NS_FAIL(NS_ERR_UNSUPPORTED, "ns_attention_generic: head sizes %d (keys) and %d (values) must lie in 1..512", d, dv);
@@ -158,10 +159,10 @@ NS_API int ns_attention_generic_sink(const void* q, int q_stride, const void* k_
     if (nkv < 1 || nq % nkv) NS_FAIL(NS_ERR_UNSUPPORTED, "ns_attention_generic: %d query heads over %d kv heads", nq, nkv);
     if (dtype == NS_F32)
         return launch<float>(q, q_stride, k_cache, v_cache, block_table, table_stride, token_req, positions, out,
-                             o_stride, n_tokens, nq, nkv, d, dv, page_size, scale, window, keep_first, chunk, softcap, sink, gate, gate_stride, gate_per_feature, out_scale, stream);
+                             o_stride, n_tokens, nq, nkv, d, dv, page_size, scale, window, keep_first, chunk, softcap, sink, gate, gate_stride, gate_per_feature, out_scale, rows, stream);
     if (dtype == NS_BF16)
         return launch<__nv_bfloat16>(q, q_stride, k_cache, v_cache, block_table, table_stride, token_req, positions,
-                                     out, o_stride, n_tokens, nq, nkv, d, dv, page_size, scale, window, keep_first, chunk, softcap, sink, gate, gate_stride, gate_per_feature, out_scale, stream);
+                                     out, o_stride, n_tokens, nq, nkv, d, dv, page_size, scale, window, keep_first, chunk, softcap, sink, gate, gate_stride, gate_per_feature, out_scale, rows, stream);
     NS_FAIL(NS_ERR_ARGUMENT, "ns_attention_generic: unknown dtype %d", dtype);
 }
 
@@ -171,5 +172,5 @@ NS_API int ns_attention_generic(const void* q, int q_stride, const void* k_cache
                                 float scale, int window, int keep_first, int chunk, float softcap, int dtype, cudaStream_t stream) {
     return ns_attention_generic_sink(q, q_stride, k_cache, v_cache, block_table, table_stride, token_req, positions, out, o_stride,
                                      n_tokens, nq, nkv, d, dv, page_size, scale, window, keep_first, chunk, softcap, nullptr, nullptr,
-                                     0, 0, 1.f, dtype, stream);
+                                     0, 0, 1.f, nullptr, dtype, stream);
 }

@@ -509,15 +509,16 @@ def attention_generic(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
                       head_dim: int, page_size: int, scale: float | None = None, window: int = 0,
                       keep_first: int = 0, v_dim: int | None = None, chunk: int = 0, softcap: float = 0.0,
                       sink: torch.Tensor | None = None, gate: torch.Tensor | None = None, feature_gate: bool = False,
-                      out_scale: float = 1.0) -> torch.Tensor:
+                      out_scale: float = 1.0, rows: torch.Tensor | None = None) -> torch.Tensor:
     """q: [N, >= nq*head_dim] rows (a view into the packed projection is fine, unit inner
     stride); out: [N, nq*v_dim] (`v_dim`: the values' head size when it differs from the keys').  `keep_first`: the
     first so many keys of a request stay visible behind the window.  `chunk` > 0: a query sees only the keys of its own
     chunk of that many positions; `softcap` > 0: scaled scores pass through softcap * tanh(s / softcap).  `sink`,
-    `gate`, `feature_gate` and `out_scale`: see `attention`.  See csrc/attention_generic.cu for the masking rule."""
+    `gate`, `feature_gate` and `out_scale`: see `attention`.  `rows` (int32): the token rows to run, all when None.  See
+    csrc/attention_generic.cu for the masking rule."""
     _cuda(q, k_cache, v_cache, block_table, token_req, positions, out, sink, gate)
     _check_sink_gate(sink, gate, nq, n_rows=out.shape[0], dtype=q.dtype, gates=nq * int(v_dim or head_dim) if feature_gate else nq)
-    _i32(positions, "positions"), _i32(token_req, "token_req")
+    _i32(positions, "positions"), _i32(token_req, "token_req"), _i32(rows, "rows")
     n = out.shape[0]
     if q.stride(1) != 1 or out.stride(1) != 1 or q.shape[0] != n or q.dtype != out.dtype:
         raise KernelError("attention: q and out must be row-major with the same rows and dtype")
@@ -527,10 +528,24 @@ def attention_generic(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
         scale = 1.0 / math.sqrt(head_dim)
     lib.call("ns_attention_generic_sink", q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
              block_table.data_ptr(), block_table.stride(0), token_req.data_ptr(), positions.data_ptr(),
-             out.data_ptr(), out.stride(0), n, nq, nkv, head_dim, int(v_dim or head_dim), page_size, float(scale), int(window),
-             int(keep_first), int(chunk), float(softcap), _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0,
-             int(bool(feature_gate)), float(out_scale), dtype_code(q.dtype), _stream())
+             out.data_ptr(), out.stride(0), n if rows is None else rows.numel(), nq, nkv, head_dim, int(v_dim or head_dim), page_size,
+             float(scale), int(window), int(keep_first), int(chunk), float(softcap), _ptr(sink), _ptr(gate),
+             gate.stride(0) if gate is not None else 0, int(bool(feature_gate)), float(out_scale), _ptr(rows), dtype_code(q.dtype), _stream())
     return out
+
+
+def _attention_f32_tiles(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, nkv: int, head_dim: int, scale: float, v_dim: int,
+                         softcap: float, sink: torch.Tensor | None, gate: torch.Tensor | None, feature_gate: bool, out_scale: float,
+                         tiles: torch.Tensor) -> None:
+    """The rows of `tiles` (int32 [n, 2]: request, offset among its tokens of this step; TILE_Q tokens each) in csrc/attention_f32.cu."""
+    _cuda(qkv, lane.k, lane.v, lane.block_table, out, sink, gate, tiles)
+    _check_sink_gate(sink, gate, nq, n_rows=out.shape[0], dtype=qkv.dtype, gates=nq * v_dim if feature_gate else nq)
+    if qkv.shape[0] != out.shape[0]:
+        raise KernelError("attention: q and out must have the same rows")
+    lib.call("ns_attention_f32_tiles", qkv.data_ptr(), qkv.stride(0), lane.k.data_ptr(), lane.v.data_ptr(), lane.block_table.data_ptr(),
+             lane.block_table.stride(0), ctx.positions.data_ptr(), ctx.qo_indptr.data_ptr(), tiles.data_ptr(), tiles.shape[0], TILE_Q,
+             out.data_ptr(), out.stride(0), nq, nkv, head_dim, v_dim, lane.page_size, float(scale), float(softcap), _ptr(sink), _ptr(gate),
+             gate.stride(0) if gate is not None else 0, int(bool(feature_gate)), float(out_scale), _stream())
 
 
 def _check_sink_gate(sink: torch.Tensor | None, gate: torch.Tensor | None, nq: int, n_rows: int, dtype: torch.dtype,
@@ -771,9 +786,21 @@ def attention(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, nkv: int
     keep_first = keep_first if window else 0
     if not _tensor_core_attention(qkv.dtype, head_dim, v_dim) or nq // nkv > 64 or (v_dim != head_dim and (nq * head_dim) % 8) \
             or (feature_gate and (gate.stride(0) % 2 or gate.data_ptr() % 4)):
+        # float32 portions of prompts with every key visible: the exact kernel's sums with keys and values shared by 32 query rows
+        # (the same bits; requests that bring one token, windows and chunks stay with the exact kernel itself)
+        rows = None
+        if qkv.dtype == torch.float32 and not window and not chunk and ctx.max_q_len > 1 and nq % nkv == 0 and nq // nkv <= 32 \
+                and lane.k.dtype == lane.v.dtype == out.dtype == qkv.dtype and all(n % 4 == 0 and 4 <= n <= 256 for n in (head_dim, v_dim)) \
+                and qkv.stride(1) == 1 and out.stride(1) == 1 and lane.k.data_ptr() % 16 == 0 and lane.v.data_ptr() % 16 == 0 \
+                and (plan := _attention_plan(ctx))["tiles"] is not None:
+            _attention_f32_tiles(qkv, lane, ctx, out, nq, nkv, head_dim, scale, v_dim, softcap, sink, gate, feature_gate, out_scale,
+                                 plan["tiles"])
+            if not plan["n_decode"]:
+                return out
+            rows = plan["decode_rows"]
         return attention_generic(qkv, lane.k, lane.v, lane.block_table, ctx.token_req, ctx.positions, out, nq, nkv,
                                  head_dim, lane.page_size, scale, window, keep_first if window else 0, v_dim, chunk, softcap, sink, gate,
-                                 feature_gate, out_scale)
+                                 feature_gate, out_scale, rows)
     _cuda(qkv, out, lane.k, lane.v, lane.block_table, sink, gate)
     _check_sink_gate(sink, gate, nq, n_rows=out.shape[0], dtype=qkv.dtype, gates=nq * v_dim if feature_gate else nq)
     if out.stride(1) != 1 or qkv.stride(1) != 1 or lane.k.dtype != qkv.dtype:
