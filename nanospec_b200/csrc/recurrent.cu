@@ -99,8 +99,8 @@ template <typename T>
 __global__ void conv_tail_kernel(const T* __restrict__ proj, int ld_proj, float* __restrict__ state, long long state_floats,
                                  long long tail_off, const int* __restrict__ qo_indptr, const int* __restrict__ state_slot,
                                  int C, int n_taps) {
-    ns_pdl_launch_dependents();
     ns_pdl_wait();
+    ns_pdl_launch_dependents();  // only now: the walk's few blocks would land unevenly among the preparation's
     const int b = blockIdx.x;
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
     if (c >= C) return;

@@ -11,43 +11,12 @@
 // Everything is float (the same operands as the token walk's: csrc/recurrent.cu), L and its differences double, so that a difference of
 // two large sums keeps its digits.  A request's chunks start at its first token of the step; requests of fewer than min_len
 // tokens are left to the token walk.  Blocks find their (request, chunk) from the step's token offsets on the device.
-#include "common.cuh"
+#include "chunks.cuh"
 
 namespace {
 
-constexpr int kQ = 64;         // tokens of a chunk
 constexpr int kThreads = 128;  // 8 x 16 threads on a 64 x 64 tile, 8 x 4 results each
 constexpr int kLd = 68;        // floats of a staged row: 16-byte aligned, rows in different banks
-
-struct Chunk {
-    int request, start, count, slot;  // count 0: no such chunk
-};
-
-// the chunk that slot number `slot` stands for; called by a whole warp
-__device__ __forceinline__ Chunk find_chunk(int slot, const int* __restrict__ qo_indptr, int n_requests, int min_len) {
-    const int lane = threadIdx.x & 31;
-    int before = 0;
-    for (int b0 = 0; b0 < n_requests; b0 += 32) {
-        const int b = b0 + lane;
-        const int start = b < n_requests ? qo_indptr[b] : 0, len = b < n_requests ? qo_indptr[b + 1] - start : 0;
-        const int chunks = len >= min_len ? (len + kQ - 1) / kQ : 0;
-        int sum = chunks;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, sum, o);
-            if (lane >= o) sum += v;
-        }
-        const int c = slot - (before + sum - chunks);
-        const unsigned who = __ballot_sync(0xffffffffu, c >= 0 && c < chunks);
-        if (who) {
-            const int src = __ffs(who) - 1;
-            return {__shfl_sync(0xffffffffu, b, src), __shfl_sync(0xffffffffu, start + c * kQ, src),
-                    __shfl_sync(0xffffffffu, min(kQ, len - c * kQ), src), slot};
-        }
-        before += __shfl_sync(0xffffffffu, sum, 31);
-    }
-    return {0, 0, 0, slot};
-}
 
 // running sums of l over the chunk (double) and the step sizes, by one warp, two tokens to a lane; tokens beyond the chunk have step 0
 __device__ __forceinline__ void chunk_logs(const float* __restrict__ step, int ld, int start, int count, float a, double* L, float* dt) {
@@ -66,8 +35,6 @@ __device__ __forceinline__ void chunk_logs(const float* __restrict__ step, int l
     dt[t0] = d0;
     dt[t1] = d1;
 }
-
-__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
 // acc[8][4] += a[8] b[4]^T
 __device__ __forceinline__ void outer(float (&acc)[8][4], const float4& a0, const float4& a1, const float4& b) {

@@ -1026,6 +1026,55 @@ def linear_scan(rec: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, 
 
 
 SCAN_MAX_DIM = 256       # rows of S that the token walk holds in registers
+LINEAR_CHUNK = 64          # tokens of a chunk in csrc/linear_chunked.cu
+# Requests of at least so many tokens in a step go a chunk at a time, shorter ones a token at a time (one request, 16 heads of 128 x 128,
+# delta rule: 128 tokens 46 us by token and 59 by chunk, 256 tokens 87 and 67, 2,048 tokens 650 and 276; retention 601 and 170) ...
+LINEAR_CHUNKED_MIN = 192
+# ... while the token walk has at most so many warps' worth of columns an SM: it needs fewer operations and wins once it fills the GPU
+# (8 requests of 256 tokens, 512 blocks of 32 columns: 261 us by token, 279 by chunk; 2 requests, 256 blocks: 1136 and 928)
+LINEAR_CHUNKED_BLOCKS = 2
+LINEAR_SCRATCH_MAX = 1 << 28  # bytes of chunk scratch; a step that would need more runs its heads in groups
+
+
+def linear_mix(rec: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, heads: int, kv_heads: int, head_dim: int, v_dim: int,
+               decay: torch.Tensor | None = None, gated: bool = False) -> torch.Tensor:
+    """Retention (`decay`) or the gated delta rule (`gated`) over each request's tokens of this step, operands as `linear_scan` takes them.
+    Long portions of prompts go 64 tokens at a time where the heads' sizes allow it (csrc/linear_chunked.cu), everything else token by
+    token."""
+    lens = [1] * ctx.n_requests if ctx.extras.get("graph") else ctx.q_lens
+    least, dp = LINEAR_CHUNKED_MIN, scan_padded_dim(head_dim)
+    chunks = sum(-(-n // LINEAR_CHUNK) for n in lens if n >= least)
+    walked = sum(n >= least for n in lens) * heads * (v_dim // 32)
+    if not chunks or walked > LINEAR_CHUNKED_BLOCKS * sm_count() or head_dim not in (64, 128) or v_dim % 64 or rec.stride(0) % 4 \
+            or rec.data_ptr() % 16:
+        return linear_scan(rec, state, ctx, out, heads, kv_heads, head_dim, v_dim, decay=decay, gated=gated)
+    off_v = 2 * kv_heads * dp
+    if rec.dtype != torch.float32 or out.dtype != torch.float32 or state.dtype != torch.float32 or rec.stride(1) != 1 or out.stride(1) != 1 \
+            or rec.shape[1] < off_v + heads * v_dim + (2 * heads if gated else 0) or out.shape[1] < heads * v_dim or not state.is_contiguous() \
+            or state.shape[1] < heads * head_dim * v_dim or (not gated and (decay is None or decay.dtype != torch.float32 or decay.numel() != heads)):
+        raise KernelError("linear_mix: float32 operands of the sizes the heads need")
+    short = max((n for n in lens if n < least), default=0)
+    if short:
+        linear_scan(rec, state, ctx, out, heads, kv_heads, head_dim, v_dim, decay=decay, gated=gated, longest=short, max_len=least - 1)
+    _cuda(rec, state, out, decay)
+    # a chunk of a head leaves its state, two factors per token and, for the delta rule, the two solved sides (csrc/linear_chunked.cu)
+    per_item = v_dim * head_dim + LINEAR_CHUNK + 4 + (LINEAR_CHUNK * (head_dim + v_dim) if gated else 0)
+    per_kv = heads // kv_heads
+    groups = min(kv_heads, max(1, LINEAR_SCRATCH_MAX // (4 * per_item * chunks * per_kv)))  # key heads to a pass
+    scratch = ctx.buffer("linear_chunks", 4, torch.float32, rows=-(-per_item * chunks * per_kv * groups // 4) + 1)
+    base, d0 = rec.data_ptr(), decay.data_ptr() if decay is not None and not gated else 0
+    for g0 in range(0, kv_heads, groups):
+        G = min(groups, kv_heads - g0)
+        h0 = g0 * per_kv
+        gates = base + 4 * (off_v + heads * v_dim + h0)
+        lib.call("ns_linear_chunked", base + 4 * g0 * dp, base + 4 * (kv_heads + g0) * dp, base + 4 * (off_v + h0 * v_dim),
+                 gates if gated else None, gates + 4 * heads if gated else None, None if gated else d0 + 4 * h0, rec.stride(0),
+                 state.data_ptr() + 4 * h0 * head_dim * v_dim, state.stride(0), ctx.qo_indptr.data_ptr(), ctx.state_slot.data_ptr(),
+                 out.data_ptr() + 4 * h0 * v_dim, out.stride(0), ctx.n_requests, least, chunks, scratch.data_ptr(), G * per_kv, G, head_dim, v_dim,
+                 _stream())
+    return out
+
+
 
 
 def ssm_padded_dim(state_dim: int) -> int:

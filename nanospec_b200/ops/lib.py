@@ -62,6 +62,7 @@ _SIGNATURES: dict[str, list] = {
                                  _P, _P, _I, _I, _F, _P],
     "ns_attention_prefill_kept": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _P, _I, _I, _I, _I, _I, _F, _I, _I, _I, _I, _F, _I, _P, _P, _I, _I, _F, _P],
     "ns_attention_generic_sink": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _F, _P, _P, _I, _I, _F, _P, _I, _P],
+    "ns_linear_chunked": [_P, _P, _P, _P, _P, _P, _I, _P, _L, _P, _P, _P, _I, _I, _I, _I, _P, _I, _I, _I, _I, _P],
     "ns_attention_f32_tiles": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P, _I, _I, _F, _P],
     "ns_add_dyt": [_P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],
     "ns_dyt_join": [_P, _P, _P, _P, _P, _P, _I, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _P],

@@ -91,8 +91,8 @@ class Retention(Part):
         ops.rotary_prepare(proj, ctx, pos.inv_freq if pos is not None and pos.dims else None, pos.magnitude if pos is not None else 1.0,
                            pos.interleaved if pos is not None else False, rec, self.heads, self.head_dim, self.v_dim,
                            1.0, self.head_dim ** -0.5)
-        read = ops.linear_scan(rec, lane.state, ctx, ctx.buffer("rec_out", self.v_size, torch.float32), self.heads, self.heads,
-                               self.head_dim, self.v_dim, decay=self._decay)
+        read = ops.linear_mix(rec, lane.state, ctx, ctx.buffer("rec_out", self.v_size, torch.float32), self.heads, self.heads,
+                              self.head_dim, self.v_dim, decay=self._decay)
         gate = proj[:, 2 * self.qk_size + self.v_size: 2 * self.qk_size + 2 * self.v_size]
         y = ops.head_norm_gate(read, gate, None, self.eps, ctx.buffer("rec_y", self.v_size), ctx, self.heads, self.v_dim)
         return ops.linear(y, self.w_o, ctx.buffer("branch", self.hidden))
@@ -166,8 +166,8 @@ class GatedDeltaRule(Part):
         rec = ctx.buffer("rec_in", self.rec_cols, torch.float32)
         ops.delta_prepare(proj, self.conv_taps, self.a_log, self.dt_bias, lane.state, self.s_floats, ctx, rec, self.kv_heads,
                           self.heads, self.head_dim, self.v_dim, self.off_b, self.off_a, self.head_dim ** -0.5, self.unit_eps)
-        read = ops.linear_scan(rec, lane.state, ctx, ctx.buffer("rec_out", self.v_size, torch.float32), self.heads, self.kv_heads,
-                               self.head_dim, self.v_dim, gated=True)
+        read = ops.linear_mix(rec, lane.state, ctx, ctx.buffer("rec_out", self.v_size, torch.float32), self.heads, self.kv_heads,
+                              self.head_dim, self.v_dim, gated=True)
         gate = proj[:, self.off_g: self.off_g + self.v_size]
         y = ops.head_norm_gate(read, gate, self.gain, self.eps, ctx.buffer("rec_y", self.v_size), ctx, self.heads, self.v_dim)
         return ops.linear(y, self.w_o, ctx.buffer("branch", self.hidden))

@@ -1,0 +1,74 @@
+"""Retention and the gated delta rule over long portions of prompts in chunks (csrc/linear_chunked.cu) against the recurrence in 64 bits."""
+
+from __future__ import annotations
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda")
+
+
+def _operands(lens, H, G, D, V, gated, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    N, cols = sum(lens), 2 * G * D + H * V + (2 * H if gated else 0)
+    rec = rnd(N, -(-(cols + G) // 4) * 4)
+    qk = rec[:, : 2 * G * D].view(N, 2 * G, D)
+    qk /= qk.norm(dim=-1, keepdim=True)
+    if gated:
+        gates = rec[:, 2 * G * D + H * V:]
+        gates[:, :H] = torch.exp(-3 * torch.rand(N, H, generator=g, device=DEV) ** 4)
+        gates[:, H // 2: H] *= (torch.rand(N, H - H // 2, generator=g, device=DEV) > 0.02)  # some decays are zero: the state is forgotten
+        gates[:, H: 2 * H] = torch.sigmoid(rnd(N, H))
+    rec[:, cols: cols + G] = (qk[:, :G] * qk[:, G:]).sum(-1)
+    decay = torch.tensor([1.0 - 2.0 ** -(5 + h % 8) for h in range(H)], device=DEV)
+    return rec, decay, 0.3 * rnd(len(lens) + 1, H * D * V + 4)
+
+
+def _walk(rec, decay, state, lens, slots, H, G, D, V, gated):
+    outs, after, at = [], state.double().clone(), 0
+    for slot, n in zip(slots, lens):
+        x = rec[at: at + n].double()
+        at += n
+        q, k = (x[:, i * G * D: (i + 1) * G * D].view(n, G, D).repeat_interleave(H // G, dim=1) for i in (0, 1))
+        v, gates = x[:, 2 * G * D: 2 * G * D + H * V].view(n, H, V), x[:, 2 * G * D + H * V:]
+        S = after[slot, : H * D * V].view(H, D, V).clone()
+        for t in range(n):
+            S = (gates[t, :H] if gated else decay.double())[:, None, None] * S
+            u = gates[t, H: 2 * H, None] * (v[t] - torch.bmm(k[t][:, None], S)[:, 0]) if gated else v[t]
+            S = S + k[t][:, :, None] * u[:, None]
+            outs.append(torch.bmm(q[t][:, None], S).reshape(-1))
+        after[slot, : H * D * V] = S.reshape(-1)
+    return torch.stack(outs), after
+
+
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("lens,H,G,D,V", [([64], 1, 1, 128, 128), ([65, 3, 129], 4, 2, 128, 128), ([63, 1, 200], 2, 2, 64, 64),
+                                          ([130, 66], 6, 2, 64, 192), ([257], 2, 1, 128, 256)])
+def test_chunked_recurrence(lens, H, G, D, V, gated, monkeypatch):
+    """Requests below and above the chunked walk's least length, remainders of one token to whole chunks, slots in another order than the
+    requests.  Bound: every sum has at most 256 + 64 terms, whose roundings (2^-24 each) add up like sqrt(n) in the 2-norm, through about
+    four products one after another; a decay of zero stays a number."""
+    from nanospec_b200 import ops
+    from nanospec_b200.parts import Workspace
+    if not gated:
+        G = H
+    monkeypatch.setattr(ops, "LINEAR_CHUNKED_MIN", 64)
+    rec, decay, state = _operands(lens, H, G, D, V, gated, sum(lens) + H)
+    slots = [len(lens) - i for i in range(len(lens))]
+    want, after = _walk(rec, decay, state, lens, slots, H, G, D, V, gated)
+    ws = Workspace(DEV)
+    ctx = SimpleNamespace(n_requests=len(lens), extras={}, q_lens=lens, max_q_len=max(lens), state_slot=torch.tensor(slots, dtype=torch.int32, device=DEV),
+                          qo_indptr=torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV),
+                          buffer=lambda name, cols, dtype, rows: ws.get(name, rows, cols, dtype))
+    for limit in (1 << 28, 1):  # all heads in one pass, and a key head at a time
+        monkeypatch.setattr(ops, "LINEAR_SCRATCH_MAX", limit)
+        S, out = state.clone(), torch.full((sum(lens), H * V + 4), 7.0, device=DEV)
+        ops.linear_mix(rec, S, ctx, out[:, : H * V], H, G, D, V, decay=None if gated else decay, gated=gated)
+        bound = 4 * 320 ** 0.5 * 2.0 ** -24
+        assert float((out[:, : H * V].double() - want).norm() / want.norm()) < bound
+        assert float((S.double() - after).norm() / after.norm()) < bound
+        assert bool((out[:, H * V:] == 7.0).all()) and torch.equal(S[0], state[0]) and torch.equal(S[:, H * D * V:], state[:, H * D * V:])
