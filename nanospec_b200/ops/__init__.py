@@ -1030,7 +1030,10 @@ LINEAR_CHUNK = 64          # tokens of a chunk in csrc/linear_chunked.cu
 # Requests of at least so many tokens in a step go a chunk at a time, shorter ones a token at a time (one request, 16 heads of 128 x 128,
 # delta rule: 128 tokens 46 us by token and 59 by chunk, 256 tokens 87 and 67, 2,048 tokens 650 and 276; retention 601 and 170) ...
 LINEAR_CHUNKED_MIN = 192
-# ... while the token walk has at most so many warps' worth of columns an SM: it needs fewer operations and wins once it fills the GPU
+# ... while the longest makes up for the pass that the shorter ones need beside it: in tokens of the walk (0.32 us each, of the longest alone)
+# a chunked pass costs about 140 and 0.36 a token (8 requests of 99 to 193 tokens: 249 us walked together, 317 with the longest in chunks) ...
+LINEAR_CHUNKED_COST = (140, 0.36)
+# ... and while the token walk has at most so many warps' worth of columns an SM: it needs fewer operations and wins once it fills the GPU
 # (8 requests of 256 tokens, 512 blocks of 32 columns: 261 us by token, 279 by chunk; 2 requests, 256 blocks: 1136 and 928)
 LINEAR_CHUNKED_BLOCKS = 2
 LINEAR_SCRATCH_MAX = 1 << 28  # bytes of chunk scratch; a step that would need more runs its heads in groups
@@ -1045,7 +1048,9 @@ def linear_mix(rec: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, h
     least, dp = LINEAR_CHUNKED_MIN, scan_padded_dim(head_dim)
     chunks = sum(-(-n // LINEAR_CHUNK) for n in lens if n >= least)
     walked = sum(n >= least for n in lens) * heads * (v_dim // 32)
-    if not chunks or walked > LINEAR_CHUNKED_BLOCKS * sm_count() or head_dim not in (64, 128) or v_dim % 64 or rec.stride(0) % 4 \
+    longest, short = max(lens, default=0), max((n for n in lens if n < least), default=0)
+    if not chunks or longest < short + LINEAR_CHUNKED_COST[0] + LINEAR_CHUNKED_COST[1] * longest \
+            or walked > LINEAR_CHUNKED_BLOCKS * sm_count() or head_dim not in (64, 128) or v_dim % 64 or rec.stride(0) % 4 \
             or rec.data_ptr() % 16:
         return linear_scan(rec, state, ctx, out, heads, kv_heads, head_dim, v_dim, decay=decay, gated=gated)
     off_v = 2 * kv_heads * dp
@@ -1053,7 +1058,6 @@ def linear_mix(rec: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, h
             or rec.shape[1] < off_v + heads * v_dim + (2 * heads if gated else 0) or out.shape[1] < heads * v_dim or not state.is_contiguous() \
             or state.shape[1] < heads * head_dim * v_dim or (not gated and (decay is None or decay.dtype != torch.float32 or decay.numel() != heads)):
         raise KernelError("linear_mix: float32 operands of the sizes the heads need")
-    short = max((n for n in lens if n < least), default=0)
     if short:
         linear_scan(rec, state, ctx, out, heads, kv_heads, head_dim, v_dim, decay=decay, gated=gated, longest=short, max_len=least - 1)
     _cuda(rec, state, out, decay)

@@ -57,6 +57,7 @@ def test_chunked_recurrence(lens, H, G, D, V, gated, monkeypatch):
     if not gated:
         G = H
     monkeypatch.setattr(ops, "LINEAR_CHUNKED_MIN", 64)
+    monkeypatch.setattr(ops, "LINEAR_CHUNKED_COST", (0, 0.0))
     rec, decay, state = _operands(lens, H, G, D, V, gated, sum(lens) + H)
     slots = [len(lens) - i for i in range(len(lens))]
     want, after = _walk(rec, decay, state, lens, slots, H, G, D, V, gated)
