@@ -52,19 +52,103 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
+// Prompts of 2,048 and 762 tokens, 32 heads of 64 over 8, a window of 1,024 with 8 kept keys, weights of 16 bits: 60 us here, 148 in the m16n8k16
+// kernel that ran them before.
+//
+// What the general instances know beside "every key at or before the query": a window, kept first keys, chunks, weights of 16 bits, a sink,
+// output gates and a scale (see csrc/attention_prefill.cu, whose masking rule this is).
+struct TcGeneral {
+    int window, keep_first, chunk, wide;
+    const float* sink;             // float [nq] or null
+    const __nv_bfloat16* gate;     // one number per token and head (or feature) or null
+    int gate_stride, per_feature;
+    float out_scale;
+};
+
+// Keys come in blocks of 64 counted from the start of the sequence: the blocks that hold kept keys, then those from the first one that the
+// block's first row sees.  lo: the first key of the first row's window (or chunk).
+struct TcKeys {
+    int lo, keep, kept_blocks, first;
+    __device__ __forceinline__ int block(int j) const { return j < kept_blocks ? j : first + j - kept_blocks; }
+};
+__device__ __forceinline__ int first_key(const TcGeneral& g, int pos) {
+    int lo = g.window > 0 && pos - g.window + 1 > 0 ? pos - g.window + 1 : 0;
+    if (g.chunk > 0) lo = max(lo, pos / g.chunk * g.chunk);
+    return lo;
+}
+__device__ __forceinline__ TcKeys tc_keys(const TcGeneral& g, int pos0) {
+    const int lo = first_key(g, pos0);
+    return {lo, g.keep_first, min((g.keep_first + kBK - 1) / kBK, lo / kBK), lo / kBK};
+}
+// the page to load for the keys of page `blk`: those past the last key, and those that nobody sees (they may have been given back), repeat the
+// last one; such keys are masked, and their values cleared before they meet a weight (clear_hidden)
+__device__ __forceinline__ int tc_page(const TcKeys& k, int blk, int last_blk, int page_size) {
+    const bool hidden = blk > last_blk || ((blk + 1) * page_size <= k.lo && blk * page_size >= k.keep);
+    return hidden ? last_blk : blk;
+}
+// Values of keys that no row of the block sees become zero: a weight of zero must not meet what happens to lie there.  One warp, before it
+// issues the product that reads them; `halves` of 64 rows x 128 bytes (the swizzle stays inside a row).
+__device__ __forceinline__ void clear_hidden(const TcKeys& k, int key0, int key_end, uint32_t v_smem, int halves) {
+    if (key0 + kBK <= key_end && (key0 >= k.lo || key0 + kBK <= k.keep)) return;
+    const int lane = threadIdx.x & 31;
+    for (int i = lane; i < halves * kBK * 8; i += 32) {
+        const int row = (i >> 3) & (kBK - 1), key = key0 + row;
+        if (key >= key_end || (key < k.lo && key >= k.keep))
+            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(v_smem + (uint32_t)i * 16u), "r"(0) : "memory");
+    }
+    fence_async_smem();
+    __syncwarp();
+}
+// scores that the row does not see become -inf; c: column of the block of keys that starts at key0
+__device__ __forceinline__ void mask_general(uint32_t (&sv)[2][32], int key0, int pos, int lo, int keep) {
+    const int last = pos - key0, from = lo - key0, kept = keep - key0;
+#pragma unroll
+    for (int c = 0; c < kBK; ++c)
+        if (c > last || (c < from && c >= kept)) sv[c >> 5][c & 31] = 0xff800000u;
+}
+__device__ __forceinline__ uint32_t pack_pair(float a, float b) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&v);
+}
+// what the rounding to a pair of bfloat16 dropped, as a pair of bfloat16
+__device__ __forceinline__ uint32_t pack_rest(uint32_t hi, float a, float b) {
+    return pack_pair(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
+}
+// the factor of the row's output, the sink's term in the denominator included; `feature` factors come on top
+__device__ __forceinline__ float general_factor(const TcGeneral& g, float m, float l, size_t token, int h) {
+    float f = 1.f;
+    if (g.sink) {
+        const float sk = g.sink[h] * kLog2eTc, mf = fmaxf(m, sk);
+        f = ex2(m - mf);
+        l = l * f + ex2(sk - mf);
+    }
+    f *= g.out_scale / l;
+    if (g.gate && !g.per_feature) f *= __fdividef(1.f, 1.f + __expf(-__bfloat162float(g.gate[token * g.gate_stride + h])));
+    return f;
+}
+__device__ __forceinline__ void gate_features(float (&v)[32], const __nv_bfloat16* gate) {
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+        const float2 z = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(gate + i));
+        v[i] *= __fdividef(1.f, 1.f + __expf(-z.x));
+        v[i + 1] *= __fdividef(1.f, 1.f + __expf(-z.y));
+    }
+}
+
 // instruction descriptors: D fp32, A and B bf16; B K-major (scores) or MN-major (values)
 __device__ __forceinline__ constexpr uint32_t idesc_tc(int n, bool b_mn_major) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn_major ? (1u << 16) : 0u) | ((uint32_t)(n >> 3) << 17) |
            ((uint32_t)(kBQ >> 4) << 24);
 }
 
-template <int kD>
+// kGeneral: the instance that knows TcGeneral
+template <int kD, bool kGeneral>
 __global__ void __launch_bounds__(kTcThreads, 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, const int* __restrict__ block_table,
                             int table_stride, const int* __restrict__ positions, const int* __restrict__ qo_indptr,
                             const int* __restrict__ tiles, __nv_bfloat16* __restrict__ out, int o_stride, int nq, int nkv,
-                            int page_size, float scale, int* __restrict__ error_flag) {
+                            int page_size, float scale, int* __restrict__ error_flag, const TcGeneral gen) {
     ns_pdl_launch_dependents();
     constexpr int kQBytes = TcSizes<kD>::kQBytes, kKBytes = TcSizes<kD>::kKBytes;
     extern __shared__ unsigned char smem_dyn[];
@@ -120,10 +204,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // per tile: its valid rows and the number of key blocks its last row sees (0 rows: the tile is idle)
     int rows_t[kTiles], nblk_t[kTiles];
     int n_blocks = 0;
+    TcKeys keys = {0, 0, 0, 0};
+    if constexpr (kGeneral) keys = tc_keys(gen, pos0);
 #pragma unroll
     for (int t = 0; t < kTiles; ++t) {
         rows_t[t] = max(0, min(kBQ, rows_all - t * kBQ));
-        nblk_t[t] = rows_t[t] > 0 ? (pos0 + t * kBQ + rows_t[t] + kBK - 1) / kBK : 0;
+        nblk_t[t] = rows_t[t] > 0 ? (pos0 + t * kBQ + rows_t[t] + kBK - 1) / kBK - keys.first + keys.kept_blocks : 0;
         n_blocks = max(n_blocks, nblk_t[t]);
     }
     const int* bt = block_table + (size_t)req * table_stride;
@@ -154,7 +240,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             const uint32_t k_dst = kv_smem + s * 2 * kKBytes, v_dst = k_dst + kKBytes;
             for (int i = 0; i < pages_per_block; ++i) {
                 // pages past the last key repeat the last page: finite values that the mask hides
-                const int blk = min(j * pages_per_block + i, last_blk);
+                const int blk = kGeneral ? tc_page(keys, keys.block(j) * pages_per_block + i, last_blk, page_size)
+                                         : min(j * pages_per_block + i, last_blk);
                 const int row = (bt[blk] * nkv + hk) * page_size;
                 const uint32_t off = (uint32_t)(i * page_size) * 128u;
                 if (elect_one()) {
@@ -208,6 +295,11 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         for (int j = 0; ok && j < n_blocks; ++j) {
             const int s = j % kKvStages, b = j & 1;
             const uint32_t v_src = kv_smem + s * 2 * kKBytes + kKBytes;
+            if constexpr (kGeneral) {
+                ok = mbar_wait_warp(kv_full(s), (uint32_t)(j / kKvStages) & 1u);
+                if (!ok) break;
+                clear_hidden(keys, keys.block(j) * kBK, pos0 + rows_all, v_src, kD / 64);
+            }
             for (int t = 0; t < kTiles && ok; ++t) {
                 if (j >= nblk_t[t]) continue;
                 if (!mbar_wait_warp(p_ready(t, b), (uint32_t)(j >> 1) & 1u)) { ok = false; break; }
@@ -217,6 +309,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     if (elect_one())
                         umma_bf16_ts(tmem_o(t), tmem_s(t, b) + kk * 8, smem_desc_mn(v_src + kk * 16 * 128, kBK * 128, 1024),
                                      idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+                if (kGeneral && gen.wide) {
+#pragma unroll
+                    for (int kk = 0; kk < kBK / 16; ++kk)
+                        if (elect_one())
+                            umma_bf16_ts(tmem_o(t), tmem_s(t, b) + 32 + kk * 8, smem_desc_mn(v_src + kk * 16 * 128, kBK * 128, 1024), idesc_o, 1u);
+                }
                 if (elect_one()) {
                     umma_commit(o_done(t));      // this tile's accumulator holds blocks 0..j
                     umma_commit(s_free(t, b));   // and S[t][b] may take the scores of block j+2
@@ -238,6 +336,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const int tile_pos0 = pos0 + t * kBQ;
         const int pos_row = tile_pos0 + min(row, max(rows, 1) - 1);
         const float sl = scale * kLog2eTc;
+        int lo_row = 0, lo_last = 0;  // the first key that this row, and the tile's last row, sees behind the kept ones
+        if constexpr (kGeneral) { lo_row = first_key(gen, pos_row); lo_last = first_key(gen, tile_pos0 + max(rows, 1) - 1); }
         float m = -INFINITY, l = 0.f;
         bool ok = true;
         for (int j = 0; j < my_blocks; ++j) {
@@ -249,14 +349,19 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             tmem_ld32(tmem_s(t, b) + lane_addr, sv[0]);
             tmem_ld32(tmem_s(t, b) + lane_addr + 32, sv[1]);
             tmem_ld_wait();
-            const int key0 = j * kBK;
-            const bool masked = key0 + kBK - 1 > tile_pos0;         // some row of the tile does not see the whole block
+            const int key0 = (kGeneral ? keys.block(j) : j) * kBK;
+            // does some row of the tile not see the whole block?
+            const bool masked = key0 + kBK - 1 > tile_pos0 || (kGeneral && key0 < lo_last && key0 + kBK > keys.keep);
             // maximum of the raw scores first (the scale is positive, so it commutes with the maximum),
             // then each weight is one fused multiply-add and one ex2
             if (masked) {
+                if constexpr (kGeneral) {
+                    mask_general(sv, key0, pos_row, lo_row, keys.keep);
+                } else {
 #pragma unroll
-                for (int c = 0; c < kBK; ++c)
-                    if (key0 + c > pos_row) sv[c >> 5][c & 31] = 0xff800000u;  // -inf
+                    for (int c = 0; c < kBK; ++c)
+                        if (key0 + c > pos_row) sv[c >> 5][c & 31] = 0xff800000u;  // -inf
+                }
             }
             // eight independent chains: one chain of 64 dependent maxima costs 64 instruction latencies
             float mx8[8];
@@ -268,24 +373,29 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             // The reference point m of the exponents follows the running maximum lazily: it moves only
             // when the maximum has grown by more than 8 (a factor 256), so the accumulator is rarely
             // rescaled; weights up to 256 are exact enough in bf16 and the sums are fp32.  Block 0
-            // holds key 0, so m is finite from the start.
+            // holds key 0, so m is finite from the start; behind a window a row may see nothing yet: then its exponents are -inf
+            // whatever is subtracted, and zero is.
             const float cand = mx * sl;
             const bool jump = cand > m + 8.f;
             const float m_new = jump ? cand : m;
             const float corr = jump ? ex2(m - m_new) : 1.f;
+            const float ref = kGeneral && m_new == -INFINITY ? 0.f : m_new;
             float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-            // weights as bf16 pairs over the first 32 columns of this row's scores
-            uint32_t pk[32];
+            // weights as bf16 pairs over the first 32 columns of this row's scores (and what the rounding dropped over the others)
+            uint32_t pk[32], rest[kGeneral ? 32 : 1];
 #pragma unroll
             for (int u = 0; u < kBK / 2; ++u) {
                 const int c = 2 * u;
-                const float p0 = ex2(fmaf(__uint_as_float(sv[c >> 5][c & 31]), sl, -m_new));
-                const float p1 = ex2(fmaf(__uint_as_float(sv[(c + 1) >> 5][(c + 1) & 31]), sl, -m_new));
+                const float p0 = ex2(fmaf(__uint_as_float(sv[c >> 5][c & 31]), sl, -ref));
+                const float p1 = ex2(fmaf(__uint_as_float(sv[(c + 1) >> 5][(c + 1) & 31]), sl, -ref));
                 sum4[u & 3] += p0 + p1;
-                __nv_bfloat162 v = __floats2bfloat162_rn(p0, p1);
-                pk[u] = *reinterpret_cast<uint32_t*>(&v);
+                pk[u] = pack_pair(p0, p1);
+                if constexpr (kGeneral) rest[u] = pack_rest(pk[u], p0, p1);
             }
             tmem_st32(tmem_s(t, b) + lane_addr, pk);
+            if constexpr (kGeneral) {
+                if (gen.wide) tmem_st32(tmem_s(t, b) + lane_addr + 32, rest);
+            }
             l = l * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
             if (j > 0 && __any_sync(0xffffffffu, jump)) {
                 // Some row's reference point moved: this warp's rows of the accumulator are rescaled.  They
@@ -314,7 +424,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             if (lane == 0) atomicExch(error_flag, kErrAttnSoftmax);
         } else if (my_blocks > 0) {
             tc_fence_after();
-            const float inv = 1.f / l;
+            const size_t token = (size_t)(tok0 + t * kBQ + min(row, rows - 1));
+            const float inv = kGeneral ? general_factor(gen, m, l, token, h) : 1.f / l;
             __nv_bfloat16* orow = out + (size_t)(tok0 + t * kBQ + row) * o_stride + (size_t)h * kD;
 #pragma unroll 1
             for (int c0 = 0; c0 < kD; c0 += 32) {
@@ -322,15 +433,14 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 tmem_ld32(tmem_o(t) + lane_addr + c0, ov);
                 tmem_ld_wait();
                 if (row < rows) {
+                    float v[32];
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        uint4 u;
-                        __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&u);
+                    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(ov[i]) * inv;
+                    if (kGeneral && gen.gate && gen.per_feature) gate_features(v, gen.gate + token * gen.gate_stride + (size_t)h * kD + c0);
 #pragma unroll
-                        for (int w = 0; w < 4; ++w)
-                            hp[w] = __floats2bfloat162_rn(__uint_as_float(ov[i + 2 * w]) * inv, __uint_as_float(ov[i + 2 * w + 1]) * inv);
-                        *reinterpret_cast<uint4*>(orow + c0 + i) = u;
-                    }
+                    for (int i = 0; i < 32; i += 8)
+                        *reinterpret_cast<uint4*>(orow + c0 + i) = make_uint4(pack_pair(v[i], v[i + 1]), pack_pair(v[i + 2], v[i + 3]),
+                                                                              pack_pair(v[i + 4], v[i + 5]), pack_pair(v[i + 6], v[i + 7]));
                 }
             }
         }
@@ -359,12 +469,13 @@ constexpr int kTiles4 = 4;
 constexpr int kTc4Threads = 96 + kTiles4 * 128;
 constexpr int kSmem4 = kTiles4 * kBQ * 64 * 2 + kKvStages * 2 * kBK * 64 * 2 + 1024 + 512;
 
+template <bool kGeneral>
 __global__ void __launch_bounds__(kTc4Threads, 1)
 attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                              const __grid_constant__ CUtensorMap map_v, const int* __restrict__ block_table,
                              int table_stride, const int* __restrict__ positions, const int* __restrict__ qo_indptr,
                              const int* __restrict__ tiles, __nv_bfloat16* __restrict__ out, int o_stride, int nq, int nkv,
-                             int page_size, float scale, int* __restrict__ error_flag) {
+                             int page_size, float scale, int* __restrict__ error_flag, const TcGeneral gen) {
     ns_pdl_launch_dependents();
     constexpr int kD = 64;
     constexpr int kQBytes = kBQ * kD * 2, kKBytes = kBK * kD * 2;
@@ -412,10 +523,12 @@ attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __
     // per row tile (tile & 1): its valid rows and the number of key blocks its last row sees (0 rows: idle)
     int rows_t[2], nblk_t[2];
     int n_blocks = 0;
+    TcKeys keys = {0, 0, 0, 0};
+    if constexpr (kGeneral) keys = tc_keys(gen, pos0);
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
         rows_t[t] = max(0, min(kBQ, rows_all - t * kBQ));
-        nblk_t[t] = rows_t[t] > 0 ? (pos0 + t * kBQ + rows_t[t] + kBK - 1) / kBK : 0;
+        nblk_t[t] = rows_t[t] > 0 ? (pos0 + t * kBQ + rows_t[t] + kBK - 1) / kBK - keys.first + keys.kept_blocks : 0;
         n_blocks = max(n_blocks, nblk_t[t]);
     }
     const int* bt = block_table + (size_t)req * table_stride;
@@ -443,7 +556,8 @@ attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __
             const uint32_t k_dst = kv_smem + s * 2 * kKBytes, v_dst = k_dst + kKBytes;
             for (int i = 0; i < pages_per_block; ++i) {
                 // pages past the last key repeat the last page: finite values that the mask hides
-                const int blk = min(j * pages_per_block + i, last_blk);
+                const int blk = kGeneral ? tc_page(keys, keys.block(j) * pages_per_block + i, last_blk, page_size)
+                                         : min(j * pages_per_block + i, last_blk);
                 const int row = (bt[blk] * nkv + hk) * page_size;
                 const uint32_t off = (uint32_t)(i * page_size) * 128u;
                 if (elect_one()) {
@@ -482,6 +596,11 @@ attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __
         for (int j = 0; ok && j < n_blocks; ++j) {
             const int s = j % kKvStages;
             const uint32_t v_src = kv_smem + s * 2 * kKBytes + kKBytes;
+            if constexpr (kGeneral) {
+                ok = mbar_wait_warp(kv_full(s), (uint32_t)(j / kKvStages) & 1u);
+                if (!ok) break;
+                clear_hidden(keys, keys.block(j) * kBK, pos0 + rows_all, v_src, kD / 64);
+            }
             for (int tt = 0; ok && tt < kTiles4; ++tt) {
                 if (j >= nblk_t[tt & 1]) continue;
                 ok = mbar_wait_warp(p_ready(tt), (uint32_t)j & 1u);
@@ -492,6 +611,12 @@ attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __
                     if (elect_one())
                         umma_bf16_ts(tmem_o(tt), tmem_s(tt) + kk * 8, smem_desc_mn(v_src + kk * 16 * 128, kBK * 128, 1024),
                                      idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+                if (kGeneral && gen.wide) {
+#pragma unroll
+                    for (int kk = 0; kk < kBK / 16; ++kk)
+                        if (elect_one())
+                            umma_bf16_ts(tmem_o(tt), tmem_s(tt) + 32 + kk * 8, smem_desc_mn(v_src + kk * 16 * 128, kBK * 128, 1024), idesc_o, 1u);
+                }
                 if (elect_one()) {
                     umma_commit(s_free(tt));                                    // the buffer may take the scores of block j+1
                     if (j == nblk_t[tt & 1] - 1) umma_commit(o_final(tt));      // the tile's accumulator is complete
@@ -513,6 +638,8 @@ attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __
         const int tile_pos0 = pos0 + t * kBQ;
         const int pos_row = tile_pos0 + min(row, max(rows, 1) - 1);
         const float sl = scale * kLog2eTc;
+        int lo_row = 0, lo_last = 0;  // the first key that this row, and the tile's last row, sees behind the kept ones
+        if constexpr (kGeneral) { lo_row = first_key(gen, pos_row); lo_last = first_key(gen, tile_pos0 + max(rows, 1) - 1); }
         float m = -INFINITY, l = 0.f;
         bool ok = true;
         for (int j = 0; j < my_blocks; ++j) {
@@ -523,11 +650,16 @@ attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __
             tmem_ld32(tmem_s(tt) + lane_addr, sv[0]);
             tmem_ld32(tmem_s(tt) + lane_addr + 32, sv[1]);
             tmem_ld_wait();
-            const int key0 = j * kBK;
-            if (key0 + kBK - 1 > tile_pos0) {                       // some row of the tile does not see the whole block
+            const int key0 = (kGeneral ? keys.block(j) : j) * kBK;
+            // does some row of the tile not see the whole block?
+            if (key0 + kBK - 1 > tile_pos0 || (kGeneral && key0 < lo_last && key0 + kBK > keys.keep)) {
+                if constexpr (kGeneral) {
+                    mask_general(sv, key0, pos_row, lo_row, keys.keep);
+                } else {
 #pragma unroll
-                for (int c = 0; c < kBK; ++c)
-                    if (key0 + c > pos_row) sv[c >> 5][c & 31] = 0xff800000u;  // -inf
+                    for (int c = 0; c < kBK; ++c)
+                        if (key0 + c > pos_row) sv[c >> 5][c & 31] = 0xff800000u;  // -inf
+                }
             }
             float mx8[8];
 #pragma unroll
@@ -540,18 +672,23 @@ attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __
             const bool jump = cand > m + 8.f;
             const float m_new = jump ? cand : m;
             const float corr = jump ? ex2(m - m_new) : 1.f;
+            const float ref = kGeneral && m_new == -INFINITY ? 0.f : m_new;  // (a row that sees nothing yet: its exponents are -inf)
+            uint32_t rest[kGeneral ? 32 : 1];
             float sum4[4] = {0.f, 0.f, 0.f, 0.f};
             // the weights of columns 2u and 2u+1 go, as a bf16 pair, where score u lay: it has been used by then
 #pragma unroll
             for (int u = 0; u < kBK / 2; ++u) {
                 const int c = 2 * u;
-                const float p0 = ex2(fmaf(__uint_as_float(sv[c >> 5][c & 31]), sl, -m_new));
-                const float p1 = ex2(fmaf(__uint_as_float(sv[(c + 1) >> 5][(c + 1) & 31]), sl, -m_new));
+                const float p0 = ex2(fmaf(__uint_as_float(sv[c >> 5][c & 31]), sl, -ref));
+                const float p1 = ex2(fmaf(__uint_as_float(sv[(c + 1) >> 5][(c + 1) & 31]), sl, -ref));
                 sum4[u & 3] += p0 + p1;
-                __nv_bfloat162 v = __floats2bfloat162_rn(p0, p1);
-                sv[0][u] = *reinterpret_cast<uint32_t*>(&v);
+                sv[0][u] = pack_pair(p0, p1);
+                if constexpr (kGeneral) rest[u] = pack_rest(sv[0][u], p0, p1);
             }
             tmem_st32(tmem_s(tt) + lane_addr, sv[0]);
+            if constexpr (kGeneral) {
+                if (gen.wide) tmem_st32(tmem_s(tt) + lane_addr + 32, rest);
+            }
             l = l * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
             if (j > 0 && __any_sync(0xffffffffu, jump)) {
                 // the accumulator holds blocks 0..j-1: this block's scores were issued after that product completed
@@ -575,7 +712,8 @@ attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __
             if (lane == 0) atomicExch(error_flag, kErrAttnSoftmax);
         } else if (my_blocks > 0) {
             tc_fence_after();
-            const float inv = 1.f / l;
+            const size_t token = (size_t)(tok0 + t * kBQ + min(row, rows - 1));
+            const float inv = kGeneral ? general_factor(gen, m, l, token, h) : 1.f / l;
             __nv_bfloat16* orow = out + (size_t)(tok0 + t * kBQ + row) * o_stride + (size_t)h * kD;
 #pragma unroll 1
             for (int c0 = 0; c0 < kD; c0 += 32) {
@@ -583,15 +721,14 @@ attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __
                 tmem_ld32(tmem_o(tt) + lane_addr + c0, ov);
                 tmem_ld_wait();
                 if (row < rows) {
+                    float v[32];
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        uint4 u;
-                        __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&u);
+                    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(ov[i]) * inv;
+                    if (kGeneral && gen.gate && gen.per_feature) gate_features(v, gen.gate + token * gen.gate_stride + (size_t)h * kD + c0);
 #pragma unroll
-                        for (int w = 0; w < 4; ++w)
-                            hp[w] = __floats2bfloat162_rn(__uint_as_float(ov[i + 2 * w]) * inv, __uint_as_float(ov[i + 2 * w + 1]) * inv);
-                        *reinterpret_cast<uint4*>(orow + c0 + i) = u;
-                    }
+                    for (int i = 0; i < 32; i += 8)
+                        *reinterpret_cast<uint4*>(orow + c0 + i) = make_uint4(pack_pair(v[i], v[i + 1]), pack_pair(v[i + 2], v[i + 3]),
+                                                                              pack_pair(v[i + 4], v[i + 5]), pack_pair(v[i + 6], v[i + 7]));
                 }
             }
         }
@@ -605,11 +742,11 @@ attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __
     }
 }
 
-template <int kD>
+template <int kD, bool kGeneral>
 int launch_prefill_tc(const void* q, int q_stride, int n_tokens, const void* k_cache, const void* v_cache, long long n_pages,
                       const int* block_table, int table_stride, const int* positions, const int* qo_indptr, const int* tiles,
                       int n_tiles, void* out, int o_stride, int nq, int nkv, int page_size, float scale, int heads_per_block,
-                      int* error_flag, cudaStream_t stream) {
+                      int* error_flag, const TcGeneral& gen, cudaStream_t stream) {
     CUtensorMap mq, mk, mv;
     int rc = ns_make_map_bf16(&mq, q, (unsigned long long)n_tokens, nq * kD, q_stride, kBQ, "ns_attention_prefill_tc");
     if (rc) return rc;
@@ -621,23 +758,23 @@ int launch_prefill_tc(const void* q, int q_stride, int n_tokens, const void* k_c
     if (kD == 64 && heads_per_block == 2) {
         static bool configured4 = false;
         if (!configured4) {
-            NS_CUDA(cudaFuncSetAttribute(attention_prefill_tc4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem4));
+            NS_CUDA(cudaFuncSetAttribute(attention_prefill_tc4_kernel<kGeneral>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem4));
             configured4 = true;
         }
-        NS_LAUNCH(attention_prefill_tc4_kernel, dim3(nq / 2, n_tiles), kTc4Threads, kSmem4, stream, mq, mk, mv, block_table,
-                  table_stride, positions, qo_indptr, tiles, (__nv_bfloat16*)out, o_stride, nq, nkv, page_size, scale, error_flag);
+        NS_LAUNCH((attention_prefill_tc4_kernel<kGeneral>), dim3(nq / 2, n_tiles), kTc4Threads, kSmem4, stream, mq, mk, mv, block_table,
+                  table_stride, positions, qo_indptr, tiles, (__nv_bfloat16*)out, o_stride, nq, nkv, page_size, scale, error_flag, gen);
         NS_CHECK_LAUNCH("ns_attention_prefill_tc");
         return NS_OK;
     }
     static bool configured = false;
     if (!configured) {
-        NS_CUDA(cudaFuncSetAttribute(attention_prefill_tc_kernel<kD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        NS_CUDA(cudaFuncSetAttribute((attention_prefill_tc_kernel<kD, kGeneral>), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      TcSizes<kD>::kSmem));
         configured = true;
     }
-    NS_LAUNCH((attention_prefill_tc_kernel<kD>), dim3(nq, n_tiles), kTcThreads, TcSizes<kD>::kSmem, stream, mq, mk, mv,
+    NS_LAUNCH((attention_prefill_tc_kernel<kD, kGeneral>), dim3(nq, n_tiles), kTcThreads, TcSizes<kD>::kSmem, stream, mq, mk, mv,
               block_table, table_stride, positions, qo_indptr, tiles, (__nv_bfloat16*)out, o_stride, nq, nkv, page_size,
-              scale, error_flag);
+              scale, error_flag, gen);
     NS_CHECK_LAUNCH("ns_attention_prefill_tc");
     return NS_OK;
 }
@@ -649,11 +786,13 @@ int launch_prefill_tc(const void* q, int q_stride, int n_tokens, const void* k_c
 // this step, a multiple of 256).  Head sizes 64 and 128; page sizes 8, 16, 32, 64; out rows 16-byte aligned.
 // heads_per_block: 1, or 2 for heads of 64 in groups of an even size (two query heads of a kv head share a block and
 // its stream of keys and values: worth it once there are more blocks than SMs).
+// window, keep_first, chunk, wide_weights, sink, gate, out_scale: as ns_attention_prefill_kept; all at rest (0, null, 1) take the plain instance.
 NS_API int ns_attention_prefill_tc(const void* q, int q_stride, int n_tokens, const void* k_cache, const void* v_cache,
                                    long long n_pages, const int* block_table, int table_stride, const int* positions,
                                    const int* qo_indptr, const int* tiles, int n_tiles, void* out, int o_stride, int nq,
-                                   int nkv, int d, int page_size, float scale, int heads_per_block, int* error_flag,
-                                   cudaStream_t stream) {
+                                   int nkv, int d, int page_size, float scale, int heads_per_block, int* error_flag, int window,
+                                   int keep_first, int chunk, int wide_weights, const float* sink, const void* gate, int gate_stride,
+                                   int gate_per_feature, float out_scale, cudaStream_t stream) {
     if (n_tiles <= 0) return NS_OK;
     if (d != 64 && d != 128) NS_FAIL(NS_ERR_UNSUPPORTED, "ns_attention_prefill_tc: head_dim=%d (64 or 128)", d);
     if (page_size != 8 && page_size != 16 && page_size != 32 && page_size != 64)
@@ -665,10 +804,15 @@ NS_API int ns_attention_prefill_tc(const void* q, int q_stride, int n_tokens, co
     if (heads_per_block != 1 && !(heads_per_block == 2 && d == 64 && (nq / nkv) % 2 == 0))
         NS_FAIL(NS_ERR_ARGUMENT, "ns_attention_prefill_tc: heads_per_block=%d (1, or 2 with heads of 64 in groups of an even size)", heads_per_block);
     if (!error_flag) NS_FAIL(NS_ERR_ARGUMENT, "ns_attention_prefill_tc: no error flag");
-    if (d == 64)
-        return launch_prefill_tc<64>(q, q_stride, n_tokens, k_cache, v_cache, n_pages, block_table, table_stride, positions,
-                                     qo_indptr, tiles, n_tiles, out, o_stride, nq, nkv, page_size, scale, heads_per_block, error_flag, stream);
-    return launch_prefill_tc<128>(q, q_stride, n_tokens, k_cache, v_cache, n_pages, block_table, table_stride, positions,
-                                  qo_indptr, tiles, n_tiles, out, o_stride, nq, nkv, page_size, scale, heads_per_block, error_flag,
-                                  stream);
+    if (window < 0 || keep_first < 0 || chunk < 0 || (chunk > 0 && keep_first > 0))
+        NS_FAIL(NS_ERR_ARGUMENT, "ns_attention_prefill_tc: window=%d keep_first=%d chunk=%d", window, keep_first, chunk);
+    if (gate && gate_per_feature && (gate_stride % 2 || (uintptr_t)gate % 4))
+        NS_FAIL(NS_ERR_UNSUPPORTED, "ns_attention_prefill_tc: a gate per feature comes in pairs");
+    const TcGeneral gen = {window, window > 0 ? keep_first : 0, chunk, wide_weights, sink, (const __nv_bfloat16*)gate, gate_stride, gate_per_feature, out_scale};
+    const bool general = window || chunk || wide_weights || sink || gate || out_scale != 1.f;
+#define NS_PREFILL_TC(D, G) launch_prefill_tc<D, G>(q, q_stride, n_tokens, k_cache, v_cache, n_pages, block_table, table_stride, positions, qo_indptr, \
+                                                    tiles, n_tiles, out, o_stride, nq, nkv, page_size, scale, heads_per_block, error_flag, gen, stream)
+    if (d == 64) return general ? NS_PREFILL_TC(64, true) : NS_PREFILL_TC(64, false);
+    return general ? NS_PREFILL_TC(128, true) : NS_PREFILL_TC(128, false);
+#undef NS_PREFILL_TC
 }

@@ -709,13 +709,13 @@ def attention_prefill(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, 
                       sink: torch.Tensor | None = None, gate: torch.Tensor | None = None, feature_gate: bool = False,
                       out_scale: float = 1.0) -> None:
     """Tensor-core attention for portions of prompts.  `tiles`: int32 [n, 2] of (request, offset
-    among its tokens of this step).  Head sizes 64 and 128 with pages of 8 to 64 tokens and no window run
+    among its tokens of this step).  Head sizes 64 and 128 with pages of 8 to 64 tokens run
     on tcgen05 (csrc/attention_prefill_tc.cu); everything else on m16n8k16 (csrc/attention_prefill.cu), also values of
-    another width than the keys (`v_dim`, both multiples of 8)."""
+    another width than the keys (`v_dim`, both multiples of 8) and capped scores."""
     v_dim = head_dim if v_dim is None else v_dim
-    if USE_TCGEN05_ATTENTION and tiles_tc is not None and head_dim in (64, 128) and window == 0 and not wide_weights \
-            and not chunk and not softcap and v_dim == head_dim and sink is None and gate is None and out_scale == 1.0 \
-            and lane.page_size in (8, 16, 32, 64) and qkv.stride(0) % 8 == 0 and out.stride(0) % 8 == 0:
+    if USE_TCGEN05_ATTENTION and tiles_tc is not None and head_dim in (64, 128) and not softcap and v_dim == head_dim and scale > 0 \
+            and lane.page_size in (8, 16, 32, 64) and qkv.stride(0) % 8 == 0 and out.stride(0) % 8 == 0 \
+            and (qkv.data_ptr() | out.data_ptr() | lane.k.data_ptr() | lane.v.data_ptr()) % 16 == 0:
         # heads of 64: two query heads of a kv head to a block (four softmax warps per sub-partition keep the exponential
         # unit busier and the keys are read once for both) - once one head to a block would give more blocks than SMs
         two_heads = head_dim == 64 and (nq // nkv) % 2 == 0 and PREFILL_TWO_HEADS != "never" and (
@@ -724,7 +724,8 @@ def attention_prefill(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, 
                  lane.v.data_ptr(), lane.k.shape[0], lane.block_table.data_ptr(), lane.block_table.stride(0),
                  ctx.positions.data_ptr(), ctx.qo_indptr.data_ptr(), tiles_tc.data_ptr(), tiles_tc.shape[0], out.data_ptr(),
                  out.stride(0), nq, nkv, head_dim, lane.page_size, float(scale), 2 if two_heads else 1,
-                 _tc(qkv.device).error.data_ptr(), _stream())
+                 _tc(qkv.device).error.data_ptr(), int(window), int(keep_first) if window else 0, int(chunk), int(bool(wide_weights)),
+                 _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0, int(bool(feature_gate)), float(out_scale), _stream())
         return
     lib.call("ns_attention_prefill_kept", qkv.data_ptr(), qkv.stride(0), lane.k.data_ptr(), lane.v.data_ptr(),
              lane.block_table.data_ptr(), lane.block_table.stride(0), ctx.positions.data_ptr(), ctx.qo_indptr.data_ptr(),
@@ -1025,7 +1026,6 @@ def linear_scan(rec: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, 
     return out
 
 
-SCAN_MAX_DIM = 256       # rows of S that the token walk holds in registers
 LINEAR_CHUNK = 64          # tokens of a chunk in csrc/linear_chunked.cu
 # Requests of at least so many tokens in a step go a chunk at a time, shorter ones a token at a time (one request, 16 heads of 128 x 128,
 # delta rule: 128 tokens 46 us by token and 59 by chunk, 256 tokens 87 and 67, 2,048 tokens 650 and 276; retention 601 and 170) ...
@@ -1079,6 +1079,7 @@ def linear_mix(rec: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, h
     return out
 
 
+SCAN_MAX_DIM = 256       # rows of S that the token walk holds in registers
 
 
 def ssm_padded_dim(state_dim: int) -> int:
