@@ -24,6 +24,7 @@
 // block winds down.  Other head sizes, page sizes other than 8/16/32/64 and windows
 // are served by the m16n8k16 kernel of attention_prefill.cu.  A second kernel below takes heads of 64 in groups
 // of an even size, two query heads to a block.
+#include "latent_flat.cuh"
 #include "tcgen05_utils.cuh"
 
 namespace {
@@ -35,12 +36,14 @@ constexpr int kKvStages = 4;     // key/value blocks in flight: later blocks are
 constexpr int kTcThreads = 96 + kTiles * 128;
 constexpr float kLog2eTc = 1.4426950408889634f;
 
-// sizes for head size D (64 or 128): tiles are halves of 64 columns = 128 bytes, the swizzle's row
-template <int D>
+// sizes for keys of DK and values of DV features (64, 128 or 192): tiles are pieces of 64 columns = 128 bytes, the swizzle's row
+template <int DK, int DV>
 struct TcSizes {
-    static constexpr int kQBytes = kBQ * D * 2;   // per tile: D / 64 halves of 128 rows x 128 B
-    static constexpr int kKBytes = kBK * D * 2;   // D / 64 halves of 64 rows x 128 B
-    static constexpr int kSmem = kTiles * kQBytes + kKvStages * 2 * kKBytes + 1024 + 256;
+    static constexpr int kQBytes = kBQ * DK * 2;   // per tile: DK / 64 pieces of 128 rows x 128 B
+    static constexpr int kKBytes = kBK * DK * 2;   // DK / 64 pieces of 64 rows x 128 B
+    static constexpr int kVBytes = kBK * DV * 2;
+    static constexpr int kStages = DK > 128 ? 3 : kKvStages;  // (two tiles of queries of 192 leave room for three)
+    static constexpr int kSmem = kTiles * kQBytes + kStages * (kKBytes + kVBytes) + 1024 + 256;
 };
 constexpr int kTmemColsTc = 512;               // S[tile][buffer] at (tile * 2 + buffer) * 64, O[tile] at 256 + tile * 128
 
@@ -141,26 +144,33 @@ __device__ __forceinline__ constexpr uint32_t idesc_tc(int n, bool b_mn_major) {
            ((uint32_t)(kBQ >> 4) << 24);
 }
 
+// Keys and values that lie side by side in scratch instead of in pages (kFlat): a request of at least min_len tokens owns the rows that
+// flat_rows() says (csrc/latent_flat.cuh), one row to a position from `from` on; keys are [a head's columns of map_k | the shared columns of
+// map_r from `shared` on].
+struct TcFlat { int n_requests, min_len, shared; };
+
 // kGeneral: the instance that knows TcGeneral
-template <int kD, bool kGeneral>
+template <int kDK, int kDV, bool kGeneral, bool kFlat>
 __global__ void __launch_bounds__(kTcThreads, 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                            const __grid_constant__ CUtensorMap map_v, const int* __restrict__ block_table,
-                            int table_stride, const int* __restrict__ positions, const int* __restrict__ qo_indptr,
-                            const int* __restrict__ tiles, __nv_bfloat16* __restrict__ out, int o_stride, int nq, int nkv,
-                            int page_size, float scale, int* __restrict__ error_flag, const TcGeneral gen) {
+                            const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_r,
+                            const int* __restrict__ block_table, int table_stride, const int* __restrict__ positions,
+                            const int* __restrict__ qo_indptr, const int* __restrict__ tiles, __nv_bfloat16* __restrict__ out,
+                            int o_stride, int nq, int nkv, int page_size, float scale, int* __restrict__ error_flag,
+                            const TcGeneral gen, const TcFlat flat) {
     ns_pdl_launch_dependents();
-    constexpr int kQBytes = TcSizes<kD>::kQBytes, kKBytes = TcSizes<kD>::kKBytes;
+    using Sz = TcSizes<kDK, kDV>;
+    constexpr int kQBytes = Sz::kQBytes, kKBytes = Sz::kKBytes, kStageBytes = Sz::kKBytes + Sz::kVBytes, kStages = Sz::kStages;
     extern __shared__ unsigned char smem_dyn[];
     const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     const uint32_t q_smem = base;                                   // [tile]
     const uint32_t kv_smem = q_smem + kTiles * kQBytes;             // [stage][K | V]
-    const uint32_t bar0 = kv_smem + kKvStages * 2 * kKBytes;
+    const uint32_t bar0 = kv_smem + kStages * kStageBytes;
     // barriers: q_full, kv_full[stage], kv_empty[stage], then per tile s_full[2], s_free[2], p_ready[2], o_done, o_final
     const uint32_t q_full = bar0;
     auto kv_full = [&](int s) { return bar0 + 8u * (1 + s); };
-    auto kv_empty = [&](int s) { return bar0 + 8u * (1 + kKvStages + s); };
-    auto tile_bar = [&](int t, int which) { return bar0 + 8u * (1 + 2 * kKvStages + t * 8 + which); };
+    auto kv_empty = [&](int s) { return bar0 + 8u * (1 + kStages + s); };
+    auto tile_bar = [&](int t, int which) { return bar0 + 8u * (1 + 2 * kStages + t * 8 + which); };
     auto s_full = [&](int t, int b) { return tile_bar(t, b); };
     auto s_free = [&](int t, int b) { return tile_bar(t, 2 + b); };
     auto p_ready = [&](int t, int b) { return tile_bar(t, 4 + b); };
@@ -169,18 +179,18 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // softmax warp may finish its last block while the product of the block before it is still waiting for the
     // tile's slower warps, and a parity wait two phases ahead of the barrier returns at once.
     auto o_final = [&](int t) { return tile_bar(t, 7); };
-    const uint32_t holder = bar0 + 8u * (1 + 2 * kKvStages + kTiles * 8);
+    const uint32_t holder = bar0 + 8u * (1 + 2 * kStages + kTiles * 8);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // heads vary fastest: the host lists the tiles with the most keys first, and blocks are
     // scheduled in that order, so the long tiles do not end up alone at the tail
     const int req = tiles[2 * blockIdx.y], q_off = tiles[2 * blockIdx.y + 1];
     const int h = blockIdx.x;
-    const int hk = h / (nq / nkv);
+    [[maybe_unused]] const int hk = h / (nq / nkv);
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
-        for (int s = 0; s < kKvStages; ++s) {
+        for (int s = 0; s < kStages; ++s) {
             mbar_init(kv_full(s), 1);
             mbar_init(kv_empty(s), 1);
         }
@@ -199,7 +209,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     if (warp == 1) tmem_alloc(holder, kTmemColsTc);
     ns_pdl_wait();  // everything below reads what earlier kernels wrote (q, the cache, the step's description)
     const int tok0 = qo_indptr[req] + q_off;
-    const int rows_all = min(kTiles * kBQ, qo_indptr[req + 1] - tok0);
+    int rows_all = min(kTiles * kBQ, qo_indptr[req + 1] - tok0);
+    if (kFlat && qo_indptr[req + 1] - tok0 + q_off < flat.min_len) rows_all = 0;  // (another kernel's)
     const int pos0 = positions[tok0];
     // per tile: its valid rows and the number of key blocks its last row sees (0 rows: the tile is idle)
     int rows_t[kTiles], nblk_t[kTiles];
@@ -212,8 +223,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         nblk_t[t] = rows_t[t] > 0 ? (pos0 + t * kBQ + rows_t[t] + kBK - 1) / kBK - keys.first + keys.kept_blocks : 0;
         n_blocks = max(n_blocks, nblk_t[t]);
     }
-    const int* bt = block_table + (size_t)req * table_stride;
-    const int last_blk = (pos0 + rows_all - 1) / page_size;  // the last page that holds one of the keys seen here
+    const int* bt = kFlat ? nullptr : block_table + (size_t)req * table_stride;
+    const int last_blk = kFlat ? 0 : (pos0 + rows_all - 1) / page_size;  // the last page that holds one of the keys seen here
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -228,16 +239,34 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             mbar_expect_tx(q_full, kTiles * kQBytes);
             for (int t = 0; t < kTiles; ++t) {  // rows past the step's tokens are zero-filled by TMA
 #pragma unroll
-                for (int hh = 0; hh < kD / 64; ++hh)
-                    tma_load_2d(q_smem + t * kQBytes + hh * (kBQ * 128), &map_q, h * kD + hh * 64, tok0 + t * kBQ, q_full);
+                for (int hh = 0; hh < kDK / 64; ++hh)
+                    tma_load_2d(q_smem + t * kQBytes + hh * (kBQ * 128), &map_q, h * kDK + hh * 64, tok0 + t * kBQ, q_full);
             }
         }
-        const int pages_per_block = kBK / page_size;
+        const int pages_per_block = kFlat ? 1 : kBK / page_size;
+        int row0 = 0;  // the scratch row of position 0
+        if constexpr (kFlat) {
+            const FlatRows f = flat_rows(req, qo_indptr, positions, flat.min_len, gen.window);
+            row0 = f.row - f.from;
+        }
         for (int j = 0; j < n_blocks; ++j) {
-            const int s = j % kKvStages;
-            if (!mbar_wait_warp(kv_empty(s), ((uint32_t)(j / kKvStages) & 1u) ^ 1u)) { if (lane == 0) atomicExch(error_flag, kErrAttnLoader); break; }
-            if (elect_one()) mbar_expect_tx(kv_full(s), 2 * kKBytes);
-            const uint32_t k_dst = kv_smem + s * 2 * kKBytes, v_dst = k_dst + kKBytes;
+            const int s = j % kStages;
+            if (!mbar_wait_warp(kv_empty(s), ((uint32_t)(j / kStages) & 1u) ^ 1u)) { if (lane == 0) atomicExch(error_flag, kErrAttnLoader); break; }
+            if (elect_one()) mbar_expect_tx(kv_full(s), kStageBytes);
+            const uint32_t k_dst = kv_smem + s * kStageBytes, v_dst = k_dst + kKBytes;
+            if constexpr (kFlat) {
+                if (elect_one()) {
+                    const int row = row0 + keys.block(j) * kBK;
+#pragma unroll
+                    for (int hh = 0; hh < kDK / 64; ++hh) {
+                        if (hh < 2) tma_load_2d(k_dst + hh * (kBK * 128), &map_k, h * 128 + hh * 64, row, kv_full(s));
+                        else tma_load_2d(k_dst + hh * (kBK * 128), &map_r, flat.shared + (hh - 2) * 64, row, kv_full(s));
+                    }
+#pragma unroll
+                    for (int hh = 0; hh < kDV / 64; ++hh) tma_load_2d(v_dst + hh * (kBK * 128), &map_v, h * kDV + hh * 64, row, kv_full(s));
+                }
+                continue;
+            }
             for (int i = 0; i < pages_per_block; ++i) {
                 // pages past the last key repeat the last page: finite values that the mask hides
                 const int blk = kGeneral ? tc_page(keys, keys.block(j) * pages_per_block + i, last_blk, page_size)
@@ -246,10 +275,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 const uint32_t off = (uint32_t)(i * page_size) * 128u;
                 if (elect_one()) {
 #pragma unroll
-                    for (int hh = 0; hh < kD / 64; ++hh) {
-                        tma_load_2d(k_dst + hh * (kBK * 128) + off, &map_k, hh * 64, row, kv_full(s));
-                        tma_load_2d(v_dst + hh * (kBK * 128) + off, &map_v, hh * 64, row, kv_full(s));
-                    }
+                    for (int hh = 0; hh < kDK / 64; ++hh) tma_load_2d(k_dst + hh * (kBK * 128) + off, &map_k, hh * 64, row, kv_full(s));
+#pragma unroll
+                    for (int hh = 0; hh < kDV / 64; ++hh) tma_load_2d(v_dst + hh * (kBK * 128) + off, &map_v, hh * 64, row, kv_full(s));
                 }
             }
         }
@@ -260,7 +288,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         constexpr uint32_t idesc_s = idesc_tc(kBK, false);
         bool ok = mbar_wait_warp(q_full, 0);
         for (int j = 0; ok && j < n_blocks; ++j) {
-            const int s = j % kKvStages, b = j & 1;
+            const int s = j % kStages, b = j & 1;
             // Three things must hold before the scores of block j are issued: its keys have landed, and for each
             // tile S[t][b] is free (it held P of block j-2, and the product that read it is done).  One lane each
             // polls one of the barriers, so the warp pays one wait, not three.
@@ -269,17 +297,17 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 const int tile = lane == 1 ? 0 : 1;
                 const bool frees = lane >= 1 && lane <= kTiles && j >= 2 && j < (tile == 0 ? nblk_t[0] : nblk_t[1]);
                 const uint32_t bar = lane == 0 ? kv_full(s) : s_free(tile, b);
-                const uint32_t par = lane == 0 ? ((uint32_t)(j / kKvStages) & 1u) : (((uint32_t)(j >> 1) & 1u) ^ 1u);
+                const uint32_t par = lane == 0 ? ((uint32_t)(j / kStages) & 1u) : (((uint32_t)(j >> 1) & 1u) ^ 1u);
                 bool mine = true;
                 if (lane == 0 || frees) mine = mbar_wait(bar, par);
                 if (!__all_sync(0xffffffffu, mine)) { ok = false; break; }
             }
             tc_fence_after();
-            const uint32_t k_src = kv_smem + s * 2 * kKBytes;
+            const uint32_t k_src = kv_smem + s * kStageBytes;
             for (int t = 0; t < kTiles; ++t) {
                 if (j >= nblk_t[t]) continue;
 #pragma unroll
-                for (int kk = 0; kk < kD / 16; ++kk) {
+                for (int kk = 0; kk < kDK / 16; ++kk) {
                     const uint32_t qa = q_smem + t * kQBytes + (kk >> 2) * (kBQ * 128) + (kk & 3) * 32;
                     const uint32_t kb = k_src + (kk >> 2) * (kBK * 128) + (kk & 3) * 32;
                     if (elect_one()) umma_bf16(tmem_s(t, b), smem_desc(qa), smem_desc(kb), idesc_s, kk > 0 ? 1u : 0u);
@@ -290,15 +318,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (!ok && lane == 0) atomicExch(error_flag, kErrAttnMma);
     } else if (warp == 2) {
         // ---------------- issuer of O += P V ----------------
-        constexpr uint32_t idesc_o = idesc_tc(kD, true);
+        constexpr uint32_t idesc_o = idesc_tc(kDV, true);
         bool ok = true;
         for (int j = 0; ok && j < n_blocks; ++j) {
-            const int s = j % kKvStages, b = j & 1;
-            const uint32_t v_src = kv_smem + s * 2 * kKBytes + kKBytes;
-            if constexpr (kGeneral) {
-                ok = mbar_wait_warp(kv_full(s), (uint32_t)(j / kKvStages) & 1u);
+            const int s = j % kStages, b = j & 1;
+            const uint32_t v_src = kv_smem + s * kStageBytes + kKBytes;
+            if constexpr (kGeneral && !kFlat) {  // (scratch rows that nobody sees are zero)
+                ok = mbar_wait_warp(kv_full(s), (uint32_t)(j / kStages) & 1u);
                 if (!ok) break;
-                clear_hidden(keys, keys.block(j) * kBK, pos0 + rows_all, v_src, kD / 64);
+                clear_hidden(keys, keys.block(j) * kBK, pos0 + rows_all, v_src, kDV / 64);
             }
             for (int t = 0; t < kTiles && ok; ++t) {
                 if (j >= nblk_t[t]) continue;
@@ -405,7 +433,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll 1
-                for (int c0 = 0; c0 < kD; c0 += 32) {
+                for (int c0 = 0; c0 < kDV; c0 += 32) {
                     uint32_t ov[32];
                     tmem_ld32(tmem_o(t) + lane_addr + c0, ov);
                     tmem_ld_wait();
@@ -426,9 +454,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             tc_fence_after();
             const size_t token = (size_t)(tok0 + t * kBQ + min(row, rows - 1));
             const float inv = kGeneral ? general_factor(gen, m, l, token, h) : 1.f / l;
-            __nv_bfloat16* orow = out + (size_t)(tok0 + t * kBQ + row) * o_stride + (size_t)h * kD;
+            __nv_bfloat16* orow = out + (size_t)(tok0 + t * kBQ + row) * o_stride + (size_t)h * kDV;
 #pragma unroll 1
-            for (int c0 = 0; c0 < kD; c0 += 32) {
+            for (int c0 = 0; c0 < kDV; c0 += 32) {
                 uint32_t ov[32];
                 tmem_ld32(tmem_o(t) + lane_addr + c0, ov);
                 tmem_ld_wait();
@@ -436,7 +464,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     float v[32];
 #pragma unroll
                     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(ov[i]) * inv;
-                    if (kGeneral && gen.gate && gen.per_feature) gate_features(v, gen.gate + token * gen.gate_stride + (size_t)h * kD + c0);
+                    if (kGeneral && gen.gate && gen.per_feature) gate_features(v, gen.gate + token * gen.gate_stride + (size_t)h * kDV + c0);
 #pragma unroll
                     for (int i = 0; i < 32; i += 8)
                         *reinterpret_cast<uint4*>(orow + c0 + i) = make_uint4(pack_pair(v[i], v[i + 1]), pack_pair(v[i + 2], v[i + 3]),
@@ -768,14 +796,32 @@ int launch_prefill_tc(const void* q, int q_stride, int n_tokens, const void* k_c
     }
     static bool configured = false;
     if (!configured) {
-        NS_CUDA(cudaFuncSetAttribute((attention_prefill_tc_kernel<kD, kGeneral>), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     TcSizes<kD>::kSmem));
+        NS_CUDA(cudaFuncSetAttribute((attention_prefill_tc_kernel<kD, kD, kGeneral, false>), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     TcSizes<kD, kD>::kSmem));
         configured = true;
     }
-    NS_LAUNCH((attention_prefill_tc_kernel<kD, kGeneral>), dim3(nq, n_tiles), kTcThreads, TcSizes<kD>::kSmem, stream, mq, mk, mv,
+    NS_LAUNCH((attention_prefill_tc_kernel<kD, kD, kGeneral, false>), dim3(nq, n_tiles), kTcThreads, (TcSizes<kD, kD>::kSmem), stream, mq, mk, mv, mv,
               block_table, table_stride, positions, qo_indptr, tiles, (__nv_bfloat16*)out, o_stride, nq, nkv, page_size,
-              scale, error_flag, gen);
+              scale, error_flag, gen, TcFlat{0, 0, 0});
     NS_CHECK_LAUNCH("ns_attention_prefill_tc");
+    return NS_OK;
+}
+
+template <int kDK>
+int launch_latent_flat(const void* q, int q_stride, int n_tokens, const void* k, const void* v, const void* lat, int lat_cols, int rows,
+                       const int* positions, const int* qo_indptr, const int* tiles, int n_tiles, void* out, int o_stride, int H, float scale,
+                       int* error_flag, const TcGeneral& gen, const TcFlat& flat, cudaStream_t stream) {
+    CUtensorMap mq, mk, mv, mr;
+    int rc = ns_make_map_bf16(&mq, q, (unsigned long long)n_tokens, H * kDK, q_stride, kBQ, "ns_attention_latent_flat");
+    if (!rc) rc = ns_make_map_bf16(&mk, k, (unsigned long long)rows, H * 128, H * 128, kBK, "ns_attention_latent_flat");
+    if (!rc) rc = ns_make_map_bf16(&mv, v, (unsigned long long)rows, H * 128, H * 128, kBK, "ns_attention_latent_flat");
+    if (!rc) rc = ns_make_map_bf16(&mr, lat, (unsigned long long)rows, lat_cols, lat_cols, kBK, "ns_attention_latent_flat");
+    if (rc) return rc;
+    constexpr int smem = TcSizes<kDK, 128>::kSmem;
+    NS_CUDA(cudaFuncSetAttribute((attention_prefill_tc_kernel<kDK, 128, true, true>), cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    NS_LAUNCH((attention_prefill_tc_kernel<kDK, 128, true, true>), dim3(H, n_tiles), kTcThreads, smem, stream, mq, mk, mv, mr, nullptr, 0, positions,
+              qo_indptr, tiles, (__nv_bfloat16*)out, o_stride, H, H, kBK, scale, error_flag, gen, flat);
+    NS_CHECK_LAUNCH("ns_attention_latent_flat");
     return NS_OK;
 }
 
@@ -815,4 +861,27 @@ NS_API int ns_attention_prefill_tc(const void* q, int q_stride, int n_tokens, co
     if (d == 64) return general ? NS_PREFILL_TC(64, true) : NS_PREFILL_TC(64, false);
     return general ? NS_PREFILL_TC(128, true) : NS_PREFILL_TC(128, false);
 #undef NS_PREFILL_TC
+}
+
+// Attention over keys and values unfolded from cached latents (csrc/latent_flat.cuh has the rows' layout): q rows [H, 128 + r] (bf16, row stride
+// q_stride, n_tokens rows), k and v [rows, H, 128], lat [rows, lat_cols] with the r (0 or 64) shared key features from column `rank` on.
+// tiles: as ns_attention_prefill_tc; requests of fewer than min_len tokens are not touched.  out rows [H, 128].  Weights keep 16 bits where they
+// meet the values; window (0: every key), sink and gate (per head) as ns_attention_prefill_tc.
+NS_API int ns_attention_latent_flat(const void* q, int q_stride, int n_tokens, const void* k, const void* v, const void* lat, int lat_cols, int rank,
+                                    int rows, const int* positions, const int* qo_indptr, int n_requests, int min_len, const int* tiles, int n_tiles,
+                                    void* out, int o_stride, int H, int r, float scale, int window, const float* sink, const void* gate,
+                                    int gate_stride, int* error_flag, cudaStream_t stream) {
+    if (n_tiles <= 0 || rows <= 0) return NS_OK;
+    if (r != 0 && r != 64) NS_FAIL(NS_ERR_UNSUPPORTED, "ns_attention_latent_flat: %d rotated features (0 or 64)", r);
+    if (H < 1 || n_tiles > 65535 || rows % kBK) NS_FAIL(NS_ERR_ARGUMENT, "ns_attention_latent_flat: %d heads, %d tiles, %d rows", H, n_tiles, rows);
+    if (q_stride % 8 || o_stride % 8 || lat_cols % 8 || rank % 8 || rank + r > lat_cols || ((uintptr_t)q | (uintptr_t)out | (uintptr_t)k | (uintptr_t)v | (uintptr_t)lat) % 16)
+        NS_FAIL(NS_ERR_UNSUPPORTED, "ns_attention_latent_flat: rows must be 16-byte aligned");
+    if (!error_flag) NS_FAIL(NS_ERR_ARGUMENT, "ns_attention_latent_flat: no error flag");
+    const TcGeneral gen = {window, 0, 0, 1, sink, (const __nv_bfloat16*)gate, gate_stride, 0, 1.f};
+    const TcFlat flat = {n_requests, min_len, rank};
+    if (r == 64)
+        return launch_latent_flat<192>(q, q_stride, n_tokens, k, v, lat, lat_cols, rows, positions, qo_indptr, tiles, n_tiles, out, o_stride, H, scale,
+                                       error_flag, gen, flat, stream);
+    return launch_latent_flat<128>(q, q_stride, n_tokens, k, v, lat, lat_cols, rows, positions, qo_indptr, tiles, n_tiles, out, o_stride, H, scale,
+                                   error_flag, gen, flat, stream);
 }

@@ -12,7 +12,7 @@
 // Masking: a query at position p sees keys p - window + 1 .. p (window 0: 0 .. p).  A sink (one learned float
 // per head) adds exp(sink) to the softmax denominator and nothing to the sum; a gate multiplies a head's
 // output by sigmoid(gate) (the projection's raw output is passed).
-#include "common.cuh"
+#include "latent_flat.cuh"
 
 namespace {
 
@@ -266,4 +266,72 @@ NS_API int ns_attention_latent(const void* q_lat, long long ql_tok, long long ql
                                            token_req, positions, sink, gate, gate_tok, out, o_tok, o_head, n_tokens, H, R, r, page_size,
                                            scale, window, stream);
     NS_FAIL(NS_ERR_ARGUMENT, "ns_attention_latent: unknown dtype %d", dtype);
+}
+
+namespace {
+
+// grid (blocks of 64 rows): the latents of the step's long requests side by side, zeros where nobody sees a key
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table, int table_stride, const int* __restrict__ positions,
+                     const int* __restrict__ qo_indptr, int n_requests, int min_len, int window, int page_size, int D, __nv_bfloat16* __restrict__ out,
+                     int rows) {
+    ns_pdl_launch_dependents();
+    ns_pdl_wait();
+    __shared__ int who, from0;
+    if (threadIdx.x < 32) {  // the request whose rows hold this block of 64
+        const int lane = threadIdx.x, want = blockIdx.x * 64;
+        int before = 0, found = -1, pos = 0;
+        for (int b0 = 0; b0 < n_requests && found < 0; b0 += 32) {
+            int from = 0;
+            const int b = b0 + lane, count = b < n_requests ? flat_count(b, qo_indptr, positions, min_len, window, &from) : 0;
+            int sum = count;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += v;
+            }
+            const int at = want - (before + sum - count);
+            const unsigned mine = __ballot_sync(0xffffffffu, at >= 0 && at < count);
+            if (mine) {
+                const int src = __ffs(mine) - 1;
+                found = __shfl_sync(0xffffffffu, b, src);
+                pos = __shfl_sync(0xffffffffu, from + at, src);
+            }
+            before += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0) { who = found; from0 = pos; }
+    }
+    __syncthreads();
+    const int b = who;
+    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)blockIdx.x * 64 * D);
+    const int pieces = D / 8;
+    int lo = 0, end = 0;
+    if (b >= 0) {
+        const int first = qo_indptr[b], pos = positions[first];
+        lo = window > 0 && pos - window + 1 > 0 ? pos - window + 1 : 0;
+        end = pos + qo_indptr[b + 1] - first;
+    }
+    for (int i = threadIdx.x; i < 64 * pieces; i += blockDim.x) {
+        const int row = i / pieces, p = from0 + row;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (b >= 0 && p >= lo && p < end) {
+            const int page = block_table[(size_t)b * table_stride + p / page_size];
+            v = *reinterpret_cast<const uint4*>(cache + ((size_t)page * page_size + p % page_size) * D + (i - row * pieces) * 8);
+        }
+        dst[i] = v;
+    }
+}
+
+}  // namespace
+
+// cache [pages, page_size, D] -> out [rows, D] (bf16, D a multiple of 8): the rows of csrc/latent_flat.cuh; rows: a multiple of 64, at least theirs.
+NS_API int ns_latent_gather(const void* cache, const int* block_table, int table_stride, const int* positions, const int* qo_indptr, int n_requests,
+                            int min_len, int window, int page_size, int D, void* out, int rows, cudaStream_t stream) {
+    if (rows <= 0 || n_requests <= 0) return NS_OK;
+    if (D % 8 || rows % 64 || page_size < 1 || ((uintptr_t)cache | (uintptr_t)out) % 16)
+        NS_FAIL(NS_ERR_ARGUMENT, "ns_latent_gather: rows of %d features must start on 16 bytes, %d rows", D, rows);
+    NS_LAUNCH(latent_gather_kernel, rows / 64, 256, 0, stream, (const __nv_bfloat16*)cache, block_table, table_stride, positions, qo_indptr, n_requests,
+              min_len, window, page_size, D, (__nv_bfloat16*)out, rows);
+    NS_CHECK_LAUNCH("ns_latent_gather");
+    return NS_OK;
 }

@@ -32,7 +32,7 @@ attention_latent_tc_kernel(const __nv_bfloat16* __restrict__ q_lat, long long ql
                            const float* __restrict__ sink, const __nv_bfloat16* __restrict__ gate, long long gate_tok,
                            __nv_bfloat16* __restrict__ out, long long o_tok, long long o_head, float* __restrict__ part_o,
                            float* __restrict__ part_ml, int H, int R, int r, int page_size, float scale, int window,
-                           int n_splits) {
+                           int n_splits, const int* __restrict__ qo_indptr, int max_len) {
     ns_pdl_launch_dependents();
     ns_pdl_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -48,7 +48,7 @@ attention_latent_tc_kernel(const __nv_bfloat16* __restrict__ q_lat, long long ql
     const int n = blockIdx.x, h0 = blockIdx.y * kRows, split = blockIdx.z;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int req = token_req[n];
-    if (req < 0) return;
+    if (req < 0 || (max_len > 0 && qo_indptr[req + 1] - qo_indptr[req] > max_len)) return;
     const int pos = positions[n];
     const int kend_all = pos + 1;
     const int kstart_all = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
@@ -266,11 +266,12 @@ attention_latent_tc_kernel(const __nv_bfloat16* __restrict__ q_lat, long long ql
 __global__ void __launch_bounds__(128)
 latent_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const int* __restrict__ token_req,
                     const float* __restrict__ sink, const __nv_bfloat16* __restrict__ gate, long long gate_tok,
-                    __nv_bfloat16* __restrict__ out, long long o_tok, long long o_head, int H, int R, int groups, int n_splits) {
+                    __nv_bfloat16* __restrict__ out, long long o_tok, long long o_head, int H, int R, int groups, int n_splits,
+                    const int* __restrict__ qo_indptr, int max_len) {
     ns_pdl_launch_dependents();
     ns_pdl_wait();
-    const int n = blockIdx.x, h = blockIdx.y;
-    if (token_req[n] < 0) return;
+    const int n = blockIdx.x, h = blockIdx.y, req = token_req[n];
+    if (req < 0 || (max_len > 0 && qo_indptr[req + 1] - qo_indptr[req] > max_len)) return;
     const int g = h / kRows, row = h % kRows;
     const size_t item0 = ((size_t)n * groups + g) * n_splits;
     float m = sink ? sink[h] * kLog2e : -INFINITY;
@@ -293,13 +294,14 @@ latent_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ 
 }  // namespace
 
 // As ns_attention_latent, bfloat16 only.  n_splits > 1: part_o [tokens * head groups * n_splits * 16 * R] and part_ml
-// [tokens * head groups * n_splits * 16 * 2] float scratch, head groups = ceil(H / 16).
+// [tokens * head groups * n_splits * 16 * 2] float scratch, head groups = ceil(H / 16).  max_len > 0: requests of more tokens in this step
+// (by qo_indptr) are left alone.
 NS_API int ns_attention_latent_tc(const void* q_lat, long long ql_tok, long long ql_head, const void* q_rot, long long qr_tok,
                                   long long qr_head, const void* cache, const int* block_table, int table_stride,
                                   const int* token_req, const int* positions, const float* sink, const void* gate,
                                   long long gate_tok, void* out, long long o_tok, long long o_head, float* part_o, float* part_ml,
                                   int n_tokens, int H, int R, int r, int page_size, float scale, int window, int n_splits,
-                                  cudaStream_t stream) {
+                                  const int* qo_indptr, int max_len, cudaStream_t stream) {
     if (n_tokens <= 0) return NS_OK;
     if (R % 16 || r % 16 || R < 16 || R > 512)
         NS_FAIL(NS_ERR_UNSUPPORTED, "ns_attention_latent_tc: a latent of %d and a rotated part of %d features (multiples of 16, the latent at most 512)", R, r);
@@ -317,7 +319,7 @@ NS_API int ns_attention_latent_tc(const void* q_lat, long long ql_tok, long long
         NS_LAUNCH((attention_latent_tc_kernel<U>), grid, kWarps * 32, smem, stream, (const __nv_bfloat16*)q_lat, ql_tok, ql_head,        \
                   (const __nv_bfloat16*)q_rot, qr_tok, qr_head, (const __nv_bfloat16*)cache, block_table, table_stride, token_req, \
                   positions, sink, (const __nv_bfloat16*)gate, gate_tok, (__nv_bfloat16*)out, o_tok, o_head, part_o, part_ml, H, R, \
-                  r, page_size, scale, window, n_splits);                                                                       \
+                  r, page_size, scale, window, n_splits, qo_indptr, max_len);                                                                       \
     }
     if (units <= 1) NS_LATENT_TC(1)
     else if (units <= 2) NS_LATENT_TC(2)
@@ -326,7 +328,7 @@ NS_API int ns_attention_latent_tc(const void* q_lat, long long ql_tok, long long
     NS_CHECK_LAUNCH("ns_attention_latent_tc");
     if (n_splits > 1) {
         NS_LAUNCH(latent_merge_kernel, dim3(n_tokens, H), 128, 0, stream, (const float*)part_o, (const float*)part_ml, token_req, sink,
-                  (const __nv_bfloat16*)gate, gate_tok, (__nv_bfloat16*)out, o_tok, o_head, H, R, groups, n_splits);
+                  (const __nv_bfloat16*)gate, gate_tok, (__nv_bfloat16*)out, o_tok, o_head, H, R, groups, n_splits, qo_indptr, max_len);
         NS_CHECK_LAUNCH("ns_latent_merge");
     }
     return NS_OK;

@@ -1260,10 +1260,11 @@ LATENT_BLOCKS_PER_SM = 2  # the tensor-core latent kernel splits a token's keys 
 
 
 def attention_latent(q_lat: torch.Tensor, q_rot: torch.Tensor, lane, ctx, out: torch.Tensor, scale: float, window: int,
-                     sink: torch.Tensor | None = None, gate: torch.Tensor | None = None) -> torch.Tensor:
+                     sink: torch.Tensor | None = None, gate: torch.Tensor | None = None, max_len: int = 0) -> torch.Tensor:
     """Attention of folded queries over a lane of cached latents.  q_lat [N, H, R] and q_rot [N, H, r] (any strides
     with a unit inner one), out [N, H, R] likewise; `sink` [H] float32 joins each head's softmax denominator; `gate`
-    [N, H] (raw, a column range of a projection is fine): the head's output times its sigmoid.
+    [N, H] (raw, a column range of a projection is fine): the head's output times its sigmoid.  `max_len` > 0: the tensor-core kernel
+    leaves requests of more tokens alone (`attention_latent_unfolded` runs them).
     bfloat16 with a latent and a rotated part in multiples of 16 (the latent up to 512): the tensor-core kernel
     (csrc/latent_tc.cu), the keys of a token split over blocks when the step has few tokens; float32 and other sizes:
     the exact kernel (csrc/latent.cu)."""
@@ -1295,13 +1296,59 @@ def attention_latent(q_lat: torch.Tensor, q_rot: torch.Tensor, lane, ctx, out: t
         lib.call("ns_attention_latent_tc", q_lat.data_ptr(), q_lat.stride(0), q_lat.stride(1), q_rot.data_ptr(), q_rot.stride(0),
                  q_rot.stride(1), lane.k.data_ptr(), bt.data_ptr(), bt.stride(0), ctx.token_req.data_ptr(), ctx.positions.data_ptr(),
                  _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0, out.data_ptr(), out.stride(0), out.stride(1),
-                 _ptr(part_o), _ptr(part_ml), n, H, R, r, lane.page_size, float(scale), int(window), n_splits, _stream())
+                 _ptr(part_o), _ptr(part_ml), n, H, R, r, lane.page_size, float(scale), int(window), n_splits, ctx.qo_indptr.data_ptr(),
+                 int(max_len), _stream())
         return out
     lib.call("ns_attention_latent", q_lat.data_ptr(), q_lat.stride(0), q_lat.stride(1), q_rot.data_ptr(), q_rot.stride(0),
              q_rot.stride(1), lane.k.data_ptr(), bt.data_ptr(), bt.stride(0), ctx.token_req.data_ptr(), ctx.positions.data_ptr(),
              _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0, out.data_ptr(), out.stride(0), out.stride(1),
              n, H, R, r, lane.page_size, float(scale), int(window), dtype_code(q_lat.dtype), _stream())
     return out
+
+
+# Requests of at least so many tokens in a step run on keys and values unfolded from the latents: the products that unfold them cost
+# 2 * rank * 256 operations a position and head, the folded form costs 2 * (2 * rank + r - 320) more a query, key and head.
+LATENT_UNFOLD_MIN = 128
+LATENT_UNFOLD_MAX = 1 << 30  # bytes of unfolded keys and values; a step that would need more runs folded
+
+
+def latent_unfold_rows(ctx, lane, heads: int, dim: int, rot_dim: int, v_dim: int, rank: int, window: int, dtype: torch.dtype, scale: float) -> tuple[int, bool]:
+    """(rows that the step's long requests need unfolded - 0: none, or the sizes do not fit -, whether every request is long)."""
+    if ctx.max_q_len < LATENT_UNFOLD_MIN or dtype != torch.bfloat16 or dim != 128 or v_dim != 128 or rot_dim not in (0, 64) or rank % 8 \
+            or scale <= 0 or lane.k.dtype != dtype or ctx.extras.get("graph") or not USE_TENSOR_CORE_LATENT or not USE_TCGEN05_ATTENTION:
+        return 0, False
+    rows = 0
+    for n, kv in zip(ctx.q_lens, ctx.kv_lens):
+        if n >= LATENT_UNFOLD_MIN:
+            first = max(0, kv - n - window + 1) if window else 0
+            rows += -(-kv // 64) * 64 - first // 64 * 64
+    if rows * heads * 512 > LATENT_UNFOLD_MAX or _attention_plan(ctx).get("tiles_tc") is None:
+        return 0, False
+    return rows, min(ctx.q_lens) >= LATENT_UNFOLD_MIN
+
+
+def attention_latent_unfolded(q: torch.Tensor, lane, ctx, out: torch.Tensor, w_uk: torch.Tensor, w_uv: torch.Tensor, rows: int, rot_dim: int, scale: float,
+                              window: int, sink: torch.Tensor | None = None, gate: torch.Tensor | None = None) -> None:
+    """Attention of the step's long requests over a lane of cached latents, keys and values formed: the latents are gathered side by side,
+    unfolded by two products, and the tcgen05 kernel reads the result (csrc/latent_flat.cuh).  `q` [N, >= H * (128 + rot_dim)], rotated;
+    `out` [N, H * 128]; `w_uk`, `w_uv` [H, 128, rank]; `rows` from `latent_unfold_rows`.  Other requests' rows of `out` stay as they are."""
+    H, R = w_uk.shape[0], w_uk.shape[2]
+    _cuda(q, out, w_uk, w_uv, lane.k, sink, gate)
+    _check_sink_gate(sink, gate, H, n_rows=out.shape[0], dtype=q.dtype, gates=H)
+    if q.dtype != torch.bfloat16 or out.dtype != q.dtype or q.stride(1) != 1 or out.stride(1) != 1 or q.shape[0] != out.shape[0] or out.shape[1] < H * 128 \
+            or q.shape[1] < H * (128 + rot_dim) or lane.k.shape[-1] != R + rot_dim:
+        raise KernelError("attention_latent_unfolded: bfloat16 rows of [H, 128 + rot_dim] queries and [H, 128] results, a cache R + rot_dim wide")
+    lat = ctx.buffer("latent_rows", R + rot_dim, rows=rows)
+    bt = lane.block_table
+    lib.call("ns_latent_gather", lane.k.data_ptr(), bt.data_ptr(), bt.stride(0), ctx.positions.data_ptr(), ctx.qo_indptr.data_ptr(), ctx.n_requests,
+             LATENT_UNFOLD_MIN, int(window), lane.page_size, R + rot_dim, lat.data_ptr(), rows, _stream())
+    k = linear(lat[:, :R], w_uk.view(H * 128, R), ctx.buffer("latent_keys", H * 128, rows=rows))
+    v = linear(lat[:, :R], w_uv.view(H * 128, R), ctx.buffer("latent_values", H * 128, rows=rows))
+    tiles = _attention_plan(ctx)["tiles_tc"]
+    lib.call("ns_attention_latent_flat", q.data_ptr(), q.stride(0), q.shape[0], k.data_ptr(), v.data_ptr(), lat.data_ptr(), R + rot_dim, R, rows,
+             ctx.positions.data_ptr(), ctx.qo_indptr.data_ptr(), ctx.n_requests, LATENT_UNFOLD_MIN, tiles.data_ptr(), tiles.shape[0], out.data_ptr(),
+             out.stride(0), H, rot_dim, float(scale), int(window), _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0,
+             _tc(q.device).error.data_ptr(), _stream())
 
 
 ACTIVATIONS = {"gelu_erf": 0, "gelu_tanh": 1, "silu": 2, "relu2": 3, "xielu": 4}

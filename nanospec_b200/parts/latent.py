@@ -9,11 +9,10 @@
     sigmoid((W_g h)_h) (gate "head", W_g [heads, hidden]), or every feature of the heads side by side times the sigmoid
     of its own gate (gate "feature", W_g [heads * v_dim, hidden]); output projection over the heads side by side.
 
-Only [c | kr] is cached (a lane with one key head of rank + rot_dim features and no values).  Keys and values are never
-formed: the plain part of the query is folded through W_uk (q_lat = W_uk,h^T q_plain, a product per head), attention runs
+Only [c | kr] is cached (a lane with one key head of rank + rot_dim features and no values).  The plain part of the query is folded through W_uk (q_lat = W_uk,h^T q_plain, a product per head), attention runs
 over the cached vectors with one shared key head whose first `rank` features are also the value (`ops.attention_latent`),
-and the result is unfolded through W_uv,h.  Prompts, portions and single tokens all take this route, so the numbers at a
-position do not depend on the cut.  The rotation, the latent's norm, scores, softmax and the gate's sigmoid are float32.
+and the result is unfolded through W_uv,h.  In bfloat16, long portions of prompts with heads of 128 form their keys and values
+instead (`ops.attention_latent_unfolded`): a fifth of the operations per query and key, the same sums rounded in other places.  The rotation, the latent's norm, scores, softmax and the gate's sigmoid are float32.
 
 params: hidden, heads, dim, rot_dim, v_dim, rank, scale, window (0: every key), eps (of the latent's norm), sink (bool),
 gate (False, True or "head", or "feature"), position (a "rotary" PartSpec over rot_dim features, or None), names (optional: tensor names after the
@@ -102,23 +101,27 @@ class LatentAttention(Part):
                               pos.magnitude if pos is not None else 1.0, self.c_gain, self.eps, H, d, r, R, write=writes)
         q = proj[:, : self.q_size].unflatten(1, (H, d + r))
         q_plain, q_rot = q[:, :, :d], q[:, :, d:]
-        # fold the plain part of every head's query through W_uk: [H, N, R]
-        q_lat = ctx.buffer("latent_q", H * R).view(-1)[: H * N * R].view(H, N, R)
-        o_lat = ctx.buffer("latent_o", H * R).view(-1)[: H * N * R].view(H, N, R)
         attn = ctx.buffer("attn_out", H * dv)
-        if self.dtype == torch.float32:  # the float32 product kernel, a head at a time
-            for h in range(H):
-                ops.linear(q_plain[:, h, :], self.w_uk_t[h], q_lat[h])
-        else:
-            torch.bmm(q_plain.permute(1, 0, 2), self.w_uk, out=q_lat)
         gate = proj[:, self.off_gate: self.off_gate + H] if self.gate_kind == "head" else None
-        ops.attention_latent(q_lat.permute(1, 0, 2), q_rot, lane, ctx, o_lat.permute(1, 0, 2), self.scale, self.window,
-                             self.sink, gate)
-        if self.dtype == torch.float32:
-            for h in range(H):
-                ops.linear(o_lat[h], self.w_uv[h], attn[:, h * dv: (h + 1) * dv])
-        else:
-            torch.bmm(o_lat, self.w_uv.transpose(1, 2), out=attn.view(N, H, dv).permute(1, 0, 2))
+        rows, all_long = ops.latent_unfold_rows(ctx, lane, H, d, r, dv, R, self.window, self.dtype, self.scale)
+        if not all_long:
+            # fold the plain part of every head's query through W_uk: [H, N, R]
+            q_lat = ctx.buffer("latent_q", H * R).view(-1)[: H * N * R].view(H, N, R)
+            o_lat = ctx.buffer("latent_o", H * R).view(-1)[: H * N * R].view(H, N, R)
+            if self.dtype == torch.float32:  # the float32 product kernel, a head at a time
+                for h in range(H):
+                    ops.linear(q_plain[:, h, :], self.w_uk_t[h], q_lat[h])
+            else:
+                torch.bmm(q_plain.permute(1, 0, 2), self.w_uk, out=q_lat)
+            ops.attention_latent(q_lat.permute(1, 0, 2), q_rot, lane, ctx, o_lat.permute(1, 0, 2), self.scale, self.window,
+                                 self.sink, gate, max_len=ops.LATENT_UNFOLD_MIN - 1 if rows else 0)
+            if self.dtype == torch.float32:
+                for h in range(H):
+                    ops.linear(o_lat[h], self.w_uv[h], attn[:, h * dv: (h + 1) * dv])
+            else:
+                torch.bmm(o_lat, self.w_uv.transpose(1, 2), out=attn.view(N, H, dv).permute(1, 0, 2))
+        if rows:  # long portions of prompts, on keys and values formed (after the product above, which writes every row)
+            ops.attention_latent_unfolded(proj[:, : self.q_size], lane, ctx, attn, self.w_uk, self.w_uv, rows, r, self.scale, self.window, self.sink, gate)
         if self.gate_kind == "feature":
             ops.sigmoid_mul(attn, proj[:, self.off_gate: self.off_gate + H * dv])
         return ops.linear(attn, self.w_o, ctx.buffer("branch", self.hidden))
