@@ -790,10 +790,10 @@ def attention(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, nkv: int
         # float32 portions of prompts with every key visible: the exact kernel's sums with keys and values shared by 32 query rows
         # (the same bits; requests that bring one token, windows and chunks stay with the exact kernel itself)
         rows = None
-        if qkv.dtype == torch.float32 and not window and not chunk and ctx.max_q_len > 1 and nq % nkv == 0 and nq // nkv <= 32 \
+        plan = getattr(ctx, "extras", {}).get("attention_plan") if qkv.dtype == torch.float32 else None  # (the step's own, if it has one)
+        if plan is not None and plan["tiles"] is not None and not window and not chunk and nq % nkv == 0 and nq // nkv <= 32 \
                 and lane.k.dtype == lane.v.dtype == out.dtype == qkv.dtype and all(n % 4 == 0 and 4 <= n <= 256 for n in (head_dim, v_dim)) \
-                and qkv.stride(1) == 1 and out.stride(1) == 1 and lane.k.data_ptr() % 16 == 0 and lane.v.data_ptr() % 16 == 0 \
-                and (plan := _attention_plan(ctx))["tiles"] is not None:
+                and qkv.stride(1) == 1 and out.stride(1) == 1 and lane.k.data_ptr() % 16 == 0 and lane.v.data_ptr() % 16 == 0:
             _attention_f32_tiles(qkv, lane, ctx, out, nq, nkv, head_dim, scale, v_dim, softcap, sink, gate, feature_gate, out_scale,
                                  plan["tiles"])
             if not plan["n_decode"]:
