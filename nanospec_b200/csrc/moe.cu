@@ -36,9 +36,10 @@ __global__ void cast_f32_kernel(const T* __restrict__ x, long long ldx, float* _
 
 constexpr int kMaxExperts = 1024;
 
-// logits[n, e] = x[n] . w[e] (+ bias[e]) in float: a block takes TOK tokens (their rows in shared memory) and eight experts, a warp per expert,
-// so a row of w is read once for TOK tokens.  The sum over a row runs in the same order whatever TOK is.
-template <typename T, int TOK>
+// logits[n, e] = x[n] . w[e] (+ bias[e]) in float: a block takes TOK tokens (their rows in shared memory) and eight warps of EPW experts each,
+// so a row of w is read once for TOK tokens and a piece of x once for EPW experts.  The sum over a row runs in the same order whatever
+// TOK and EPW are.
+template <typename T, int TOK, int EPW>
 __global__ void __launch_bounds__(256)
 router_logits_kernel(const T* __restrict__ x, long long ldx, const float* __restrict__ w, const float* __restrict__ bias,
                      float* __restrict__ logits, int n_tokens, int E, int K) {
@@ -46,7 +47,7 @@ router_logits_kernel(const T* __restrict__ x, long long ldx, const float* __rest
     ns_pdl_wait();
     extern __shared__ __align__(16) float xrow[];  // [TOK][K4]
     const int K4 = (K + 3) / 4 * 4;
-    const int n0 = blockIdx.x * TOK, lane = threadIdx.x & 31, e = blockIdx.y * 8 + (threadIdx.x >> 5);
+    const int n0 = blockIdx.x * TOK, lane = threadIdx.x & 31, e0 = (blockIdx.y * 8 + (threadIdx.x >> 5)) * EPW;
     const int cnt = min(TOK, n_tokens - n0);
     const bool vec = K % 8 == 0 && ldx % 8 == 0 && (((uintptr_t)w | (uintptr_t)x) % 16 == 0);
     if (vec) {
@@ -64,33 +65,48 @@ router_logits_kernel(const T* __restrict__ x, long long ldx, const float* __rest
         }
     }
     __syncthreads();
-    if (e >= E) return;
-    const float* wr = w + (size_t)e * K;
-    float a[TOK];
+    if (e0 >= E) return;
+    const float* wr[EPW];  // (experts beyond the last: the last one again, not written)
 #pragma unroll
-    for (int t = 0; t < TOK; ++t) a[t] = 0.f;
+    for (int i = 0; i < EPW; ++i) wr[i] = w + (size_t)min(e0 + i, E - 1) * K;
+    float a[EPW][TOK];
+#pragma unroll
+    for (int i = 0; i < EPW; ++i)
+#pragma unroll
+        for (int t = 0; t < TOK; ++t) a[i][t] = 0.f;
     if (vec) {
-#pragma unroll 4
+#pragma unroll(EPW == 1 ? 4 : 2)
         for (int k = lane * 4; k < K; k += 128) {
-            const float4 v = *reinterpret_cast<const float4*>(wr + k);
+            float4 v[EPW];
+#pragma unroll
+            for (int i = 0; i < EPW; ++i) v[i] = *reinterpret_cast<const float4*>(wr[i] + k);
 #pragma unroll
             for (int t = 0; t < TOK; ++t) {
                 const float4 u = *reinterpret_cast<const float4*>(xrow + (size_t)t * K4 + k);
-                a[t] = fmaf(v.x, u.x, a[t]); a[t] = fmaf(v.y, u.y, a[t]); a[t] = fmaf(v.z, u.z, a[t]); a[t] = fmaf(v.w, u.w, a[t]);
+#pragma unroll
+                for (int i = 0; i < EPW; ++i) {
+                    a[i][t] = fmaf(v[i].x, u.x, a[i][t]); a[i][t] = fmaf(v[i].y, u.y, a[i][t]);
+                    a[i][t] = fmaf(v[i].z, u.z, a[i][t]); a[i][t] = fmaf(v[i].w, u.w, a[i][t]);
+                }
             }
         }
     } else {
         for (int k = lane; k < K; k += 32) {
-            const float v = wr[k];
 #pragma unroll
-            for (int t = 0; t < TOK; ++t) a[t] = fmaf(v, xrow[(size_t)t * K4 + k], a[t]);
+            for (int i = 0; i < EPW; ++i) {
+                const float v = wr[i][k];
+#pragma unroll
+                for (int t = 0; t < TOK; ++t) a[i][t] = fmaf(v, xrow[(size_t)t * K4 + k], a[i][t]);
+            }
         }
     }
 #pragma unroll
-    for (int t = 0; t < TOK; ++t) {
-        const float v = ns_warp_sum(a[t]) + (bias ? bias[e] : 0.f);
-        if (lane == 0 && t < cnt) logits[(size_t)(n0 + t) * E + e] = v;
-    }
+    for (int i = 0; i < EPW; ++i)
+#pragma unroll
+        for (int t = 0; t < TOK; ++t) {
+            const float v = ns_warp_sum(a[i][t]) + (bias ? bias[min(e0 + i, E - 1)] : 0.f);
+            if (lane == 0 && t < cnt && e0 + i < E) logits[(size_t)(n0 + t) * E + e0 + i] = v;
+        }
 }
 
 struct RouteRule {
@@ -295,11 +311,12 @@ __global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict
     }
 }
 
-// out[n] = sum_k weight[n, k] * (row >= 0 ? ys[row] : x[n]), float sums in the order of the choice, rounded once; with `resid`
+// out[n] = sum_k weight[n, k] * (row >= 0 ? ys[row] : x[n]) (+ rest[n]), float sums in the order of the choice, rounded once; with `resid`
 // the sum is added to that float row instead.  VEC = 8: eight features to a thread with 16-byte accesses.
 template <typename T, int VEC>
 __global__ void moe_combine_kernel(const T* __restrict__ ys, const int* __restrict__ row_of, const float* __restrict__ weights,
-                                   const T* __restrict__ x, T* __restrict__ out, float* __restrict__ resid, int top, int width) {
+                                   const T* __restrict__ x, const T* __restrict__ rest, T* __restrict__ out, float* __restrict__ resid,
+                                   int top, int width) {
     ns_pdl_launch_dependents();
     ns_pdl_wait();
     const int n = blockIdx.x;
@@ -326,13 +343,19 @@ __global__ void moe_combine_kernel(const T* __restrict__ ys, const int* __restri
                 for (int i = 0; i < 8; ++i) a[i] += v[i];
                 st8(resid + at, a);
             } else {
+                if (rest) {
+                    float v[8];
+                    ld8(rest + at, v);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) a[i] += v[i];
+                }
                 st8(out + at, a);
             }
         } else {
             float a = 0.f;
             for (int k = 0; k < top; ++k) a = fmaf(w[k], rows[k] >= 0 ? ns_ld(ys, (size_t)rows[k] * width + h) : ns_ld(x, at), a);
             if (resid) resid[at] += a;
-            else ns_st(out, at, a);
+            else ns_st(out, at, rest ? a + ns_ld(rest, at) : a);
         }
     }
 }
@@ -488,13 +511,21 @@ NS_API int ns_router_logits(const void* x, long long ldx, const float* w, const 
     int tok = n_tokens <= 32 ? 1 : n_tokens <= 128 ? 2 : n_tokens <= 512 ? 4 : 8;
     while (tok > 1 && tok * row > 100 * 1024) tok /= 2;
     const size_t smem = tok * row;
-    const dim3 grid((n_tokens + tok - 1) / tok, (E + 7) / 8);
-#define NS_ROUTER(T, TK)                                                                                                              \
+    // experts to a warp: one while tokens alone give few blocks; in long steps as many as leave one or two groups of eight warps (2,048 tokens of
+    // 2,048 features, 36 experts: 38 us with one, 18 with five)
+    const int epw = tok < 8 ? 1 : E <= 8 ? 1 : E <= 16 ? 2 : E > 32 && E <= 40 ? 5 : 4;
+    const dim3 grid((n_tokens + tok - 1) / tok, (E + 8 * epw - 1) / (8 * epw));
+#define NS_ROUTER(T, TK, EP)                                                                                                          \
     {                                                                                                                                 \
-        if (smem > 48 * 1024) NS_CUDA(cudaFuncSetAttribute(router_logits_kernel<T, TK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); \
-        NS_LAUNCH((router_logits_kernel<T, TK>), grid, 256, smem, stream, (const T*)x, ldx, w, bias, logits, n_tokens, E, K);         \
+        if (smem > 48 * 1024) NS_CUDA(cudaFuncSetAttribute(router_logits_kernel<T, TK, EP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); \
+        NS_LAUNCH((router_logits_kernel<T, TK, EP>), grid, 256, smem, stream, (const T*)x, ldx, w, bias, logits, n_tokens, E, K);     \
     }
-#define NS_ROUTER_T(T) { if (tok == 1) NS_ROUTER(T, 1) else if (tok == 2) NS_ROUTER(T, 2) else if (tok == 4) NS_ROUTER(T, 4) else NS_ROUTER(T, 8) }
+#define NS_ROUTER_T(T)                                                                                                  \
+    {                                                                                                                   \
+        if (tok == 1) NS_ROUTER(T, 1, 1) else if (tok == 2) NS_ROUTER(T, 2, 1) else if (tok == 4) NS_ROUTER(T, 4, 1)    \
+        else if (epw == 1) NS_ROUTER(T, 8, 1) else if (epw == 2) NS_ROUTER(T, 8, 2) else if (epw == 4) NS_ROUTER(T, 8, 4) \
+        else NS_ROUTER(T, 8, 5)                                                                                         \
+    }
     if (dtype == NS_F32) NS_ROUTER_T(float)
     else NS_ROUTER_T(__nv_bfloat16)
 #undef NS_ROUTER_T
@@ -567,17 +598,17 @@ NS_API int ns_moe_gather(const void* x, const int* row_of, void* xs, int n_token
     return NS_OK;
 }
 
-// x [n, width] (only read for choices without a row); resid (float) or out receives the sum
-NS_API int ns_moe_combine(const void* ys, const int* row_of, const float* weights, const void* x, void* out, float* resid, int n_tokens,
-                          int top, int width, int dtype, cudaStream_t stream) {
+// x [n, width] (only read for choices without a row); resid (float) or out receives the sum, out that of `rest` [n, width] (or null) as well
+NS_API int ns_moe_combine(const void* ys, const int* row_of, const float* weights, const void* x, const void* rest, void* out, float* resid,
+                          int n_tokens, int top, int width, int dtype, cudaStream_t stream) {
     if (n_tokens <= 0) return NS_OK;
     if (dtype != NS_F32 && dtype != NS_BF16) NS_FAIL(NS_ERR_ARGUMENT, "ns_moe_combine: unknown dtype %d", dtype);
     if (!out && !resid) NS_FAIL(NS_ERR_ARGUMENT, "ns_moe_combine: nowhere to put the sum");
-    const bool vec = width % 8 == 0 && (((uintptr_t)ys | (uintptr_t)x | (uintptr_t)out | (uintptr_t)resid) % 16 == 0);
+    const bool vec = width % 8 == 0 && (((uintptr_t)ys | (uintptr_t)x | (uintptr_t)rest | (uintptr_t)out | (uintptr_t)resid) % 16 == 0);
     const int per_row = vec ? width / 8 : width;
     const int threads = per_row >= 256 ? 256 : (per_row + 31) / 32 * 32;
     const dim3 grid(n_tokens, vec ? (per_row + threads - 1) / threads : 1);
-#define NS_COMBINE(T, V) NS_LAUNCH((moe_combine_kernel<T, V>), grid, threads, 0, stream, (const T*)ys, row_of, weights, (const T*)x, (T*)out, resid, top, width)
+#define NS_COMBINE(T, V) NS_LAUNCH((moe_combine_kernel<T, V>), grid, threads, 0, stream, (const T*)ys, row_of, weights, (const T*)x, (const T*)rest, (T*)out, resid, top, width)
     if (dtype == NS_F32) { if (vec) NS_COMBINE(float, 8); else NS_COMBINE(float, 1); }
     else { if (vec) NS_COMBINE(__nv_bfloat16, 8); else NS_COMBINE(__nv_bfloat16, 1); }
 #undef NS_COMBINE

@@ -6,6 +6,7 @@ except `linear` in bfloat16, which may hand a plain matrix product to cuBLAS.
 from __future__ import annotations
 
 import math
+import threading
 from dataclasses import dataclass
 
 import torch
@@ -866,13 +867,19 @@ class SideLane:
 RUN_BESIDE = True  # False: one stream (measurements and tests)
 
 
-def side_lane(device: torch.device, name: str) -> SideLane | None:
-    """The device's side stream of that name, or None while kernels are timed one by one."""
+_side_of_thread = threading.local()  # gone with its thread
+
+
+def side_lane(device: torch.device, name: str, own: bool = False) -> SideLane | None:
+    """The device's side stream of that name (`own`: the calling thread's own, whose fork and join no other thread can come between), or
+    None while kernels are timed one by one."""
     if not RUN_BESIDE or lib.timing_kernels():
         return None
-    lane = _side.get((device, name))
+    lanes = _side if not own else _side_of_thread.__dict__
+    key = (device, name) if not own else f"{device}/{name}"
+    lane = lanes.get(key)
     if lane is None:
-        lane = _side[(device, name)] = SideLane(device)
+        lane = lanes[key] = SideLane(device)
     return lane
 
 
@@ -1519,10 +1526,10 @@ def moe_gather(x: torch.Tensor, row_of: torch.Tensor, xs: torch.Tensor, top: int
 
 
 def moe_combine(ys: torch.Tensor, row_of: torch.Tensor, weights: torch.Tensor, out: torch.Tensor | None, top: int,
-                x: torch.Tensor | None = None, resid: torch.Tensor | None = None) -> torch.Tensor:
+                x: torch.Tensor | None = None, resid: torch.Tensor | None = None, rest: torch.Tensor | None = None) -> torch.Tensor:
     """out[n] = sum_k weights[n, k] * ys[row_of[n, k]]; a choice without a row (-1) takes x[n].  With `resid` (float32 [N, width])
-    the sum is added to it in place of `out`."""
-    _cuda(ys, row_of, weights, out, x, resid)
+    the sum is added to it in place of `out`; with `rest` ([N, width] of ys's dtype) that is added to the float sum before it is rounded."""
+    _cuda(ys, row_of, weights, out, x, resid, rest)
     dst = resid if resid is not None else out
     n, width = dst.shape
     if ys.shape[0] < n * top or ys.shape[1] != width or not (ys.is_contiguous() and dst.is_contiguous()) \
@@ -1530,7 +1537,9 @@ def moe_combine(ys: torch.Tensor, row_of: torch.Tensor, weights: torch.Tensor, o
         raise KernelError("moe_combine: contiguous ys [at least N * top, width] and an output of its dtype, or a float32 stream")
     if x is not None and (x.shape != dst.shape or x.dtype != ys.dtype or not x.is_contiguous()):
         raise KernelError("moe_combine: x must be contiguous [N, width] of ys's dtype")
-    lib.call("ns_moe_combine", ys.data_ptr(), row_of.data_ptr(), weights.data_ptr(), _ptr(x), _ptr(out) if resid is None else None,
+    if rest is not None and (resid is not None or rest.shape != dst.shape or rest.dtype != ys.dtype or not rest.is_contiguous()):
+        raise KernelError("moe_combine: rest must be contiguous [N, width] of ys's dtype, and the result rounded")
+    lib.call("ns_moe_combine", ys.data_ptr(), row_of.data_ptr(), weights.data_ptr(), _ptr(x), _ptr(rest), _ptr(out) if resid is None else None,
              _ptr(resid), n, int(top), width, dtype_code(ys.dtype), _stream())
     return dst
 

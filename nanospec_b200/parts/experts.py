@@ -146,9 +146,31 @@ class RoutedExperts(Part):
         out = ctx.buffer("branch", self.hidden)
         if self.shared is None:
             return self._routed(x, ctx, out, None)
-        y = ops.cast_f32(self.shared.forward(x, ctx, out_name="branch_shared"), ctx.buffer("experts_sum", self.hidden, torch.float32))
-        self._routed(x, ctx, out, y)
-        return out.copy_(y)
+        if not self._combines(x.shape[0], x, self._captured(ctx)):
+            y = ops.cast_f32(self.shared.forward(x, ctx, out_name="branch_shared"), ctx.buffer("experts_sum", self.hidden, torch.float32))
+            self._routed(x, ctx, out, y)
+            return out.copy_(y)
+        # the shared expert's products on a second stream, beside the router and the plan, which are short of work; its output joins the
+        # routed sum in that sum's kernel
+        side = ops.side_lane(x.device, "shared_expert", own=True)
+        if side is None:
+            return self._routed(x, ctx, out, None, rest=lambda: self.shared.forward(x, ctx, out_name="branch_shared"))
+        self.shared.reserve(ctx, "branch_shared")
+        side.fork()
+        with side.stream():
+            rest = self.shared.forward(x, ctx, out_name="branch_shared")
+        joined = False
+
+        def join():
+            nonlocal joined
+            if not joined:
+                joined = True
+                side.join()
+            return rest
+        try:
+            return self._routed(x, ctx, out, None, rest=join)
+        finally:
+            join()
 
     def join_stream(self, x, ctx: StepContext, resid: torch.Tensor) -> None:
         """The routed experts' sum, added to the float32 stream; everything but the shared expert."""
@@ -210,10 +232,20 @@ class RoutedExperts(Part):
         ops.moe_plan(ids, self.experts, offsets, row_of, pair_of)
         return weights
 
-    def _finish(self, ys, row_of, weights, out, x, resid, summed: bool):
-        return ops.moe_combine(ys, row_of, weights, out, self.top, x=x, resid=resid) if summed else ops.RoutedSum(ys, row_of, weights)
+    def _captured(self, ctx: StepContext) -> bool:
+        return bool(ctx.extras.get("graph")) or torch.cuda.is_current_stream_capturing()
 
-    def _grouped(self, x, ids, weights, offsets, row_of, out, ctx: StepContext, resid, summed: bool = True):
+    def _combines(self, n: int, x, captured: bool) -> bool:
+        """Whether a step of n tokens ends in `ops.moe_combine` (the rows kernel sums by itself)."""
+        if self.tcgen05 or not (n <= ROWS_MAX or captured):
+            return True
+        return ops.moe_grouped_ok(x, self.hidden, self.inter) and (GROUPED_MAX is None or n <= GROUPED_MAX or captured)
+
+    def _finish(self, ys, row_of, weights, out, x, resid, summed: bool, rest=None):
+        return ops.moe_combine(ys, row_of, weights, out, self.top, x=x, resid=resid, rest=rest() if rest is not None else None) if summed \
+            else ops.RoutedSum(ys, row_of, weights)
+
+    def _grouped(self, x, ids, weights, offsets, row_of, out, ctx: StepContext, resid, summed: bool = True, rest=None):
         n = x.shape[0]
         pair_of = ctx.buffer("expert_pairs", self.top, torch.int32)
         if ids is None:
@@ -223,13 +255,14 @@ class RoutedExperts(Part):
         act = ctx.buffer("expert_act", self.inter, rows=n * self.top)
         ys = ctx.buffer("expert_out", self.hidden, rows=n * self.top)
         ops.moe_grouped(x, pair_of, offsets, self.w_gate, self.w_up, self.w_down, act, ys, self.top, self.unit)
-        return self._finish(ys, row_of, weights, out, x, resid, summed)
+        return self._finish(ys, row_of, weights, out, x, resid, summed, rest)
 
-    def _routed(self, x, ctx: StepContext, out: torch.Tensor, resid: torch.Tensor | None, summed: bool = True):
-        """The routed experts' sum in `out`, or added to the float32 `resid` when that is given; returns where it went.  `summed` False: the
+    def _routed(self, x, ctx: StepContext, out: torch.Tensor, resid: torch.Tensor | None, summed: bool = True, rest=None):
+        """The routed experts' sum in `out`, or added to the float32 `resid` when that is given; returns where it went.  `rest` (a function of
+        nothing, asked for at the end; only where `_combines`): rows added to the float sum.  `summed` False: the
         sum is left to the caller (`ops.RoutedSum`) where the route taken leaves a row per choice."""
         n = x.shape[0]
-        captured = bool(ctx.extras.get("graph")) or torch.cuda.is_current_stream_capturing()
+        captured = self._captured(ctx)
         offsets = ctx.buffer("expert_offsets", 1, torch.int32, rows=self.experts + 1).view(-1)
         row_of = ctx.buffer("expert_rows", self.top, torch.int32)
         if self.tcgen05:
@@ -237,10 +270,10 @@ class RoutedExperts(Part):
             xs = ops.moe_gather(x, row_of, ctx.buffer("expert_in", self.hidden, rows=n * self.top), self.top)
             ys = ctx.buffer("expert_out", self.hidden, rows=n * self.top)
             ops.moe_grouped_tc(xs, offsets, self.w_gate_up, self.w_down, ctx.buffer("expert_act", self.inter, rows=n * self.top), ys, self.unit)
-            return self._finish(ys, row_of, weights, out, x, resid, summed)
+            return self._finish(ys, row_of, weights, out, x, resid, summed, rest)
         grouped_ok = ops.moe_grouped_ok(x, self.hidden, self.inter)
         if grouped_ok and (GROUPED_MAX is None or n <= GROUPED_MAX or captured):
-            return self._grouped(x, None, None, offsets, row_of, out, ctx, resid, summed)
+            return self._grouped(x, None, None, offsets, row_of, out, ctx, resid, summed, rest)
         ids, weights = self.route(x, ctx)
         if n <= ROWS_MAX or captured:
             act = ctx.buffer("expert_act", self.inter, rows=n * self.top)
@@ -253,7 +286,7 @@ class RoutedExperts(Part):
             cap = max(64, -(-max(b - a for a, b in zip(bounds, bounds[1:])) // 64) * 64)
             rows = self.experts * cap
             if rows > PAD_WASTE_MAX * n * self.top:  # the tokens crowd a few experts: no layout of equal shares for them
-                return self._grouped(x, ids, weights, offsets, row_of, out, ctx, resid, summed)
+                return self._grouped(x, ids, weights, offsets, row_of, out, ctx, resid, summed, rest)
             ops.moe_pad_rows(ids, offsets, row_of, cap)
             xs = ops.moe_gather(x, row_of, ctx.buffer("expert_in", self.hidden, rows=rows), self.top)
             gu = ctx.buffer("expert_gate_up", 2 * self.inter, rows=rows)
@@ -261,7 +294,7 @@ class RoutedExperts(Part):
             act = ops.swiglu(gu, ctx.buffer("expert_act", self.inter, rows=rows), self.gate_block, self.unit)
             ys = ctx.buffer("expert_out", self.hidden, rows=rows)
             torch.bmm(act.view(self.experts, cap, self.inter), self.w_down.transpose(1, 2), out=ys.view(self.experts, cap, self.hidden))
-            return self._finish(ys, row_of, weights, out, x, resid, summed)
+            return self._finish(ys, row_of, weights, out, x, resid, summed, rest)
         xs = ops.moe_gather(x, row_of, ctx.buffer("expert_in", self.hidden, rows=n * self.top), self.top)
         ys = ctx.buffer("expert_out", self.hidden, rows=n * self.top)
         act = ctx.buffer("expert_act", self.inter, rows=n * self.top)
@@ -271,4 +304,4 @@ class RoutedExperts(Part):
             if hi > lo:
                 ops.gated_linear(xs[lo:hi], self.w_gate_up[e], act[lo:hi], scratch[lo:hi], self.gate_block, self.unit)
                 ops.linear(act[lo:hi], self.w_down[e], ys[lo:hi])
-        return self._finish(ys, row_of, weights, out, x, resid, summed)
+        return self._finish(ys, row_of, weights, out, x, resid, summed, rest)

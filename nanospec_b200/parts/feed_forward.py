@@ -68,6 +68,11 @@ class SwiGLU(Part):
                                self.gate_block, self.unit)
         return ops.linear(act, self.w_down, ctx.buffer(out_name, self.hidden), sink=sink)
 
+    def reserve(self, ctx: StepContext, out_name: str = "branch") -> None:
+        """The step's buffers that `forward` uses: a caller that runs it on another stream makes them on its own first."""
+        for name, cols in (("ffn_act", self.inter), ("gate_up", 2 * self.inter), (out_name, self.hidden)):
+            ctx.buffer(name, cols)
+
     # ---- optional: an arrangement that runs the two products inside larger ones of its own (see `GQAAttention.packs_projections`)
     packs_projections = True
 

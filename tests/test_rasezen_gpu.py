@@ -867,3 +867,17 @@ def test_command_line(tmp_path):
                         "--max-tokens", "128"], input="\n".join(json.dumps(s) for s in steps) + "\n", capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and "done 0" in r.stdout and "done 1" in r.stdout, r.stderr
     assert (tmp_path / "o" / "0.f32").stat().st_size == 4 * full_config()["vocab"]
+
+
+@pytest.mark.parametrize("n,E", [(513, 5), (600, 16), (515, 33), (520, 40), (514, 41), (1000, 70)])  # the experts to a warp, and remainders of them
+def test_router_of_long_steps(n, E):
+    """Long steps give a warp several experts; the sums keep their order: the bits of the same rows in short steps."""
+    from nanospec_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(n + E)
+    x = torch.randn(n, 264, generator=g, device="cuda").to(torch.bfloat16)
+    w, bias = torch.randn(E, 264, generator=g, device="cuda"), torch.randn(E, generator=g, device="cuda")
+    got = ops.router_logits(x, w, torch.full((n, E), 9.0, device="cuda"), bias=bias)
+    parts = [ops.router_logits(x[i: i + 100], w, torch.empty(min(100, n - i), E, device="cuda"), bias=bias) for i in range(0, n, 100)]
+    assert torch.equal(got, torch.cat(parts))
+    # K roundings of a partial sum below sum |x w|
+    assert bool(((got.double() - x.double() @ w.double().T - bias.double()).abs() <= x.double().abs() @ w.double().abs().T * 300 * 2.0 ** -24 + 1e-6).all())
