@@ -268,6 +268,232 @@ chunk_outputs_kernel(const float* __restrict__ C, const float* __restrict__ B, c
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// The same two kernels for heads of 64 features in groups of a multiple of four and states of 64 or 128 rows: a block takes four heads of a
+// group, so that B, and C and the scores C B^T, are staged and made once for them, and threads of 8 x 8 results (16 words of shared memory to 64
+// FMAs; 12 to 32 above).  The same sums in the same order, bit for bit.  Prompts of 2,471 tokens in all, 64 heads of 64, a state of 128 rows, 8
+// groups: sums 103 us above, 80 here; read-out 242 above, 190 here.
+// ---------------------------------------------------------------------------------------
+constexpr int kHeads = 4, kLd4 = 68;
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int G> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(G) : "memory"); }
+
+// acc += a b^T, 8 x 8
+__device__ __forceinline__ void outer8(float (&acc)[8][8], const float4& a0, const float4& a1, const float4& b0, const float4& b1) {
+    const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+}
+
+// grid (chunk slots, H / 4), 256 threads: N / 8 x 8 threads to a head, 256 / N heads at a time
+template <int N>
+__global__ void __launch_bounds__(256, 2)
+chunk_states4_kernel(const float* __restrict__ B, const float* __restrict__ x, const float* __restrict__ step, int ld,
+                     const float* __restrict__ a_log, const int* __restrict__ qo_indptr, int n_requests, int min_len,
+                     float* __restrict__ states, float* __restrict__ decays, int H, int G) {
+    ns_pdl_wait();
+    constexpr int kAtOnce = 256 / N, kPasses = kHeads / kAtOnce, kLdB = N + 4;
+    extern __shared__ __align__(16) float states_smem[];
+    float* Bs = states_smem;              // [64][N + 4]
+    float* xs = Bs + kQ * kLdB;           // [kHeads][64][68]
+    __shared__ double L[kHeads][kQ];
+    __shared__ float dt[kHeads][kQ], w[kHeads][kQ];
+    __shared__ Chunk chunk;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h0 = blockIdx.y * kHeads, g = h0 / (H / G);
+    if (warp == 0) {
+        const Chunk c = find_chunk(blockIdx.x, qo_indptr, n_requests, min_len);
+        if (lane == 0) chunk = c;
+    }
+    __syncthreads();
+    const Chunk c = chunk;
+    if (c.count == 0) return;
+    const float* B0 = B + (size_t)c.start * ld + (size_t)g * N;
+    for (int i = tid; i < kQ * (N / 4); i += 256) {
+        const int t = i / (N / 4), e = (i % (N / 4)) * 4;
+        cp_async16(Bs + t * kLdB + e, B0 + (size_t)(t < c.count ? t : 0) * ld + e, t < c.count);
+    }
+    const float* x0 = x + (size_t)c.start * ld + (size_t)h0 * 64;
+    for (int p = 0; p < kPasses; ++p) {  // a group of copies to a pass, so that the first heads do not wait for the others
+        for (int i = tid; i < kAtOnce * kQ * 16; i += 256) {
+            const int hh = p * kAtOnce + i / (kQ * 16), t = (i >> 4) % kQ, e = (i & 15) * 4;
+            cp_async16(xs + (hh * kQ + t) * kLd4 + e, x0 + (size_t)(t < c.count ? t : 0) * ld + hh * 64 + e, t < c.count);
+        }
+        cp_async_commit();
+    }
+    if (warp < kHeads) {
+        const int h = h0 + warp;
+        chunk_logs(step + h, ld, c.start, c.count, expf(a_log[h]), L[warp], dt[warp]);
+        __syncwarp();
+        for (int t = lane; t < kQ; t += 32) w[warp][t] = expf((float)(L[warp][kQ - 1] - L[warp][t])) * dt[warp][t];  // (tokens beyond the chunk: step 0)
+        if (lane == 0) decays[(size_t)c.slot * H + h] = expf((float)L[warp][kQ - 1]);
+    }
+    const int mine = tid / N, n4 = ((tid % N) >> 3) * 4, v4 = (tid & 7) * 4;  // rows n4 .. + 3 and N / 2 + n4 .. + 3, columns v4 .. + 3 and 32 + v4 .. + 3
+    for (int p = 0; p < kPasses; ++p) {
+        if (kPasses == 2 && p == 0) cp_async_wait<1>();
+        else cp_async_wait<0>();
+        __syncthreads();
+        const int hh = p * kAtOnce + mine;
+        const float* xh = xs + hh * kQ * kLd4;
+        float acc[8][8] = {};
+#pragma unroll 2
+        for (int s = 0; s < c.count; ++s) {
+            const float f = w[hh][s];
+            float4 b0 = ld4(xh + s * kLd4 + v4), b1 = ld4(xh + s * kLd4 + 32 + v4);
+            b0.x *= f; b0.y *= f; b0.z *= f; b0.w *= f;
+            b1.x *= f; b1.y *= f; b1.z *= f; b1.w *= f;
+            outer8(acc, ld4(Bs + s * kLdB + n4), ld4(Bs + s * kLdB + N / 2 + n4), b0, b1);
+        }
+        if (p == kPasses - 1) ns_pdl_launch_dependents();
+        float* dst = states + ((size_t)c.slot * H + h0 + hh) * N * 64;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float* row = dst + (size_t)((i < 4 ? n4 + i : N / 2 + n4 + i - 4)) * 64 + v4;
+            *reinterpret_cast<float4*>(row) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+            *reinterpret_cast<float4*>(row + 32) = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+        }
+    }
+}
+
+// grid (chunk slots, H / 4), 256 threads, two warps to a head: the first tokens 0 .. 31, the second 32 .. 63
+template <int N>
+__global__ void __launch_bounds__(256, 2)
+chunk_outputs4_kernel(const float* __restrict__ C, const float* __restrict__ B, const float* __restrict__ x, const float* __restrict__ step,
+                      int ld, const float* __restrict__ a_log, const int* __restrict__ qo_indptr, int n_requests, int min_len,
+                      const float* __restrict__ states, float* __restrict__ out, int ld_out, int H, int G) {
+    ns_pdl_wait();
+    constexpr int kRows = 16;  // rows of the state to a slice
+    constexpr int kSlices = 2 * kHeads * kRows * kLd4, kCt = N * kLd4;
+    extern __shared__ __align__(16) float outputs_smem[];
+    float* Sc = outputs_smem;       // the scores, [s][t]
+    float* Ct = Sc + kQ * kLd4;     // C transposed, [k][t]
+    float* slices = Ct + kCt;       // first B transposed, [k][s]; then slices of the heads' states, [2][head][16][68]
+    float* M = Ct;                  // at last, over both: the heads' weights of x, [head][s][t]
+    static_assert(kSlices >= kCt, "B transposed takes the slices' place");
+    __shared__ double L[kHeads][kQ];
+    __shared__ float dt[kHeads][kQ];
+    __shared__ Chunk chunk;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h0 = blockIdx.y * kHeads, g = h0 / (H / G);
+    if (warp == 0) {
+        const Chunk c = find_chunk(blockIdx.x, qo_indptr, n_requests, min_len);
+        if (lane == 0) chunk = c;
+    }
+    __syncthreads();
+    const Chunk c = chunk;
+    if (c.count == 0) return;
+    {
+        const float* C0 = C + (size_t)c.start * ld + (size_t)g * N;
+        const float* B0 = B + (size_t)c.start * ld + (size_t)g * N;
+#pragma unroll 4
+        for (int i = tid; i < kQ * (N / 4); i += 256) {
+            const int t = (i >> 2) % kQ, k = ((i >> 2) / kQ * 4 + (i & 3)) * 4;
+            float4 u = make_float4(0.f, 0.f, 0.f, 0.f), v = u;
+            if (t < c.count) {
+                u = ld4(C0 + (size_t)t * ld + k);
+                v = ld4(B0 + (size_t)t * ld + k);
+            }
+            float* a = Ct + k * kLd4 + t;
+            float* b = slices + k * kLd4 + t;
+            a[0] = u.x; a[kLd4] = u.y; a[2 * kLd4] = u.z; a[3 * kLd4] = u.w;
+            b[0] = v.x; b[kLd4] = v.y; b[2 * kLd4] = v.z; b[3 * kLd4] = v.w;
+        }
+    }
+    if (warp < kHeads) chunk_logs(step + h0 + warp, ld, c.start, c.count, expf(a_log[h0 + warp]), L[warp], dt[warp]);
+    __syncthreads();
+    {  // the scores: four tokens t and four s to a thread
+        const int t4 = (tid >> 4) * 4, s4 = (tid & 15) * 4;
+        float z[4][4] = {};
+#pragma unroll 4
+        for (int k = 0; k < N; ++k) {
+            const float4 a = ld4(Ct + k * kLd4 + t4), b = ld4(slices + k * kLd4 + s4);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) z[i][j] = fmaf(av[i], bv[j], z[i][j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(Sc + (s4 + j) * kLd4 + t4) = make_float4(z[0][j], z[1][j], z[2][j], z[3][j]);
+    }
+    __syncthreads();  // B has been read
+    const int hh = warp >> 1, h = h0 + hh, id = tid & 63;
+    const int ta = 32 * (warp & 1) + (lane >> 3) * 4, va = (lane & 7) * 4;  // tokens ta .. + 3 and ta + 16 .. + 19, features va .. + 3 and va + 32 .. + 35
+    const float* S0 = states + ((size_t)c.slot * H + h) * N * 64;
+    auto issue = [&](int sl) {
+        float* dst = slices + ((sl & 1) * kHeads + hh) * kRows * kLd4;
+        for (int i = id; i < kRows * 16; i += 64) cp_async16(dst + (i >> 4) * kLd4 + (i & 15) * 4, S0 + (size_t)(sl * kRows + (i >> 4)) * 64 + (i & 15) * 4, true);
+        cp_async_commit();
+    };
+    auto head_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + hh) : "memory"); };  // the two warps of a head
+    float y[8][8] = {};
+    issue(0);
+    for (int sl = 0; sl < N / kRows; ++sl) {
+        if (sl + 1 < N / kRows) { issue(sl + 1); cp_async_wait<1>(); }
+        else cp_async_wait<0>();
+        head_sync();
+        const float* Sl = slices + ((sl & 1) * kHeads + hh) * kRows * kLd4;
+        const float* Ck = Ct + sl * kRows * kLd4;
+#pragma unroll 4
+        for (int k = 0; k < kRows; ++k)
+            outer8(y, ld4(Ck + k * kLd4 + ta), ld4(Ck + k * kLd4 + ta + 16), ld4(Sl + k * kLd4 + va), ld4(Sl + k * kLd4 + va + 32));
+        head_sync();  // the slice may be filled again
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float f = expf((float)L[hh][i < 4 ? ta + i : ta + 12 + i]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) y[i][j] *= f;
+    }
+    __syncthreads();  // C and the slices have been read by every head
+    float* Mh = M + hh * kQ * kLd4;
+    {
+        const double Lt = L[hh][id];
+#pragma unroll 4
+        for (int s = 0; s < kQ; ++s) Mh[s * kLd4 + id] = s <= id ? Sc[s * kLd4 + id] * (expf((float)(Lt - L[hh][s])) * dt[hh][s]) : 0.f;
+    }
+    head_sync();
+    const float* xh = x + (size_t)c.start * ld + (size_t)h * 64 + va;
+    const int s_end = min(c.count, 32 * (warp & 1) + 32);  // no weight of this warp's tokens lies beyond
+#pragma unroll 4
+    for (int s = 0; s < s_end; ++s)
+        outer8(y, ld4(Mh + s * kLd4 + ta), ld4(Mh + s * kLd4 + ta + 16), ld4(xh + (size_t)s * ld), ld4(xh + (size_t)s * ld + 32));
+    ns_pdl_launch_dependents();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int t = i < 4 ? ta + i : ta + 12 + i;
+        if (t >= c.count) continue;
+        float* dst = out + (size_t)(c.start + t) * ld_out + (size_t)h * 64 + va;
+        *reinterpret_cast<float4*>(dst) = make_float4(y[i][0], y[i][1], y[i][2], y[i][3]);
+        *reinterpret_cast<float4*>(dst + 32) = make_float4(y[i][4], y[i][5], y[i][6], y[i][7]);
+    }
+}
+
+template <int N>
+int launch_states4(const float* B, const float* x, const float* step, int ld, const float* a_log, const int* qo_indptr, int n_requests, int min_len,
+                   int chunks, float* states, float* decays, int H, int G, cudaStream_t stream) {
+    constexpr int smem = 4 * (kQ * (N + 4) + kHeads * kQ * kLd4);
+    NS_CUDA(cudaFuncSetAttribute(chunk_states4_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    NS_LAUNCH(chunk_states4_kernel<N>, dim3(chunks, H / kHeads), 256, smem, stream, B, x, step, ld, a_log, qo_indptr, n_requests, min_len, states, decays, H, G);
+    NS_CHECK_LAUNCH("ns_ssm_chunked");
+    return NS_OK;
+}
+template <int N>
+int launch_outputs4(const float* C, const float* B, const float* x, const float* step, int ld, const float* a_log, const int* qo_indptr, int n_requests,
+                    int min_len, int chunks, const float* states, float* out, int ld_out, int H, int G, cudaStream_t stream) {
+    constexpr int both = N * kLd4 + 2 * kHeads * 16 * kLd4, weights = kHeads * kQ * kLd4;
+    constexpr int smem = 4 * (kQ * kLd4 + (both > weights ? both : weights));
+    NS_CUDA(cudaFuncSetAttribute(chunk_outputs4_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    NS_LAUNCH(chunk_outputs4_kernel<N>, dim3(chunks, H / kHeads), 256, smem, stream, C, B, x, step, ld, a_log, qo_indptr, n_requests, min_len, states, out,
+              ld_out, H, G);
+    NS_CHECK_LAUNCH("ns_ssm_chunked");
+    return NS_OK;
+}
+
 }  // namespace
 
 // C, B, x, step: the columns of the preparation's rows (row stride ld floats; groups of C and B Np apart, heads of x V, one step size
@@ -283,8 +509,15 @@ NS_API int ns_ssm_chunked(const float* C, const float* B, const float* x, const 
         NS_FAIL(NS_ERR_ARGUMENT, "ns_ssm_chunked: rows must start on 16 bytes");
     const int n_tiles = (N + 63) / 64, v_tiles = (V + 63) / 64;
     if (H > 65535 || n_tiles * v_tiles > 65535) NS_FAIL(NS_ERR_UNSUPPORTED, "ns_ssm_chunked: %d heads, state of %d x %d exceed the grid", H, N, V);
-    NS_LAUNCH(chunk_states_kernel, dim3(chunks, H, n_tiles * v_tiles), kThreads, 0, stream, B, x, step, ld, a_log, qo_indptr, n_requests, min_len,
-              states, decays, H, G, N, Np, V);
+    const bool four = V == 64 && (N == 64 || N == 128) && Np == N && (H / G) % kHeads == 0 && ld_out % 4 == 0;
+#define NS_SSM_FOUR(F, ...) (N == 128 ? F<128>(__VA_ARGS__) : F<64>(__VA_ARGS__))
+    if (four) {
+        const int rc = NS_SSM_FOUR(launch_states4, B, x, step, ld, a_log, qo_indptr, n_requests, min_len, chunks, states, decays, H, G, stream);
+        if (rc) return rc;
+    } else {
+        NS_LAUNCH(chunk_states_kernel, dim3(chunks, H, n_tiles * v_tiles), kThreads, 0, stream, B, x, step, ld, a_log, qo_indptr, n_requests, min_len,
+                  states, decays, H, G, N, Np, V);
+    }
     NS_CHECK_LAUNCH("ns_ssm_chunked");
     const long long total = (long long)H * N * V;
     const bool vec = (N * V) % 4 == 0 && state_floats % 4 == 0 && (uintptr_t)state % 16 == 0;
@@ -297,6 +530,9 @@ NS_API int ns_ssm_chunked(const float* C, const float* B, const float* x, const 
         NS_LAUNCH((chunk_pass_kernel<1>), dim3(n_requests, (unsigned)blocks), 256, 0, stream, states, decays, state, state_floats, qo_indptr, state_slot,
                   min_len, H, N * V);
     NS_CHECK_LAUNCH("ns_ssm_chunked");
+    if (four)
+        return NS_SSM_FOUR(launch_outputs4, C, B, x, step, ld, a_log, qo_indptr, n_requests, min_len, chunks, states, out, ld_out, H, G, stream);
+#undef NS_SSM_FOUR
     NS_LAUNCH(chunk_outputs_kernel, dim3(chunks, H, v_tiles), kThreads, 0, stream, C, B, x, step, ld, a_log, qo_indptr, n_requests, min_len,
               states, out, ld_out, H, G, N, Np, V);
     NS_CHECK_LAUNCH("ns_ssm_chunked");
