@@ -12,7 +12,7 @@ DEV = torch.device("cuda")
 
 
 @pytest.mark.parametrize("N", [64, 128])
-@pytest.mark.parametrize("lens,H,G", [([96], 4, 1), ([97, 3, 191], 8, 2), ([128, 65, 160], 12, 1), ([511], 16, 4)])
+@pytest.mark.parametrize("lens,H,G", [([96], 4, 1), ([97, 3, 191], 8, 2), ([128, 65, 160], 12, 1), ([511], 16, 4), ([577, 1153], 4, 1)])
 def test_four_heads_to_a_block(lens, H, G, N):
     from nanospec_b200 import ops
     from nanospec_b200.parts import Workspace
