@@ -49,6 +49,12 @@ from .base import Part, WeightSpec
 from .context import StepContext
 from .registry import build_part, register_part
 
+# An eager step runs the shared expert on a second stream from so many us of work on: the fork and the join cost the host 40 us, and a step
+# below is bound by its launches (32 experts of 4 chosen, 1,024 over 2,048 features, a shared one of 2,048: 128 us on one stream against 158
+# on two for 400 tokens, 148 / 156 for 800, 183 / 175 for 1,200, 257 / 224 for 2,048; 2 chosen, 512 over 4,096: 145 / 156 for 400, 180 / 165 for
+# 800; 4 of 1,024 over 4,096: 173 / 165 for 24).  Captured steps have no launches to wait for and always take two.
+BESIDE_MIN_US = 130
+
 USE_TCGEN05 = True # False: parts built from now on take the m16n8k16 kernel and the library's batched products (measurements)
 ROWS_MAX = 16      # steps of up to this many tokens stream the chosen experts' rows (float32, or widths that are no multiple of 8)
 # bfloat16 steps of up to this many tokens run every expert over its tokens in one tensor-core kernel that reads the counts on the
@@ -152,7 +158,8 @@ class RoutedExperts(Part):
             return out.copy_(y)
         # the shared expert's products on a second stream, beside the router and the plan, which are short of work; its output joins the
         # routed sum in that sum's kernel
-        side = ops.side_lane(x.device, "shared_expert", own=True)
+        beside = self._captured(ctx) or self._outlasts_launches(x)
+        side = ops.side_lane(x.device, "shared_expert", own=True) if beside else None
         if side is None:
             return self._routed(x, ctx, out, None, rest=lambda: self.shared.forward(x, ctx, out_name="branch_shared"))
         self.shared.reserve(ctx, "branch_shared")
@@ -234,6 +241,14 @@ class RoutedExperts(Part):
 
     def _captured(self, ctx: StepContext) -> bool:
         return bool(ctx.extras.get("graph")) or torch.cuda.is_current_stream_capturing()
+
+    def _outlasts_launches(self, x: torch.Tensor) -> bool:
+        """Whether the part's work on the rows of x (the chosen weights at 6.5 TB/s and the products at 1 PFLOP/s) covers the launches of an
+        eager step with a second stream."""
+        n = x.shape[0]
+        weights = 3 * self.hidden * (min(self.experts, n * self.top) * self.inter + self.shared.inter) * x.element_size()
+        flops = 6 * n * self.hidden * (self.top * self.inter + self.shared.inter)
+        return weights / 6.5e6 + flops / 1e9 >= BESIDE_MIN_US
 
     def _combines(self, n: int, x, captured: bool) -> bool:
         """Whether a step of n tokens ends in `ops.moe_combine` (the rows kernel sums by itself)."""

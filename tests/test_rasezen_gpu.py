@@ -881,3 +881,24 @@ def test_router_of_long_steps(n, E):
     assert torch.equal(got, torch.cat(parts))
     # K roundings of a partial sum below sum |x w|
     assert bool(((got.double() - x.double() @ w.double().T - bias.double()).abs() <= x.double().abs() @ w.double().abs().T * 300 * 2.0 ** -24 + 1e-6).all())
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("n,ff", [(2, 64), (65, 64), (600, 64), (40, 16), (600, 16)])
+def test_shared_expert_on_one_stream_or_two(n, ff, dtype, tmp_path, monkeypatch):
+    """The rule that gives an eager step a second stream changes no bit, and long steps of heavy experts pass it."""
+    from nanospec_b200.engine.step import StepEntry
+    from nanospec_b200.parts import experts
+
+    cfg = config([attn(moe(ff=ff, shared=16), size=40)])
+    runner, _ = make(tmp_path, cfg, seed=91, dtype=dtype, blocks=160, page=4)
+    runner.begin(0)
+    ctx, _, _ = runner.build_context([StepEntry(0, tokens(n, cfg["vocab"], 92), [])])
+    part = runner.model.blocks[0].feed_forward
+    x = torch.randn(n, part.hidden, generator=torch.Generator().manual_seed(93)).to("cuda", dtype)
+    runs = []
+    for least in (0, 1 << 30, 0):
+        monkeypatch.setattr(experts, "BESIDE_MIN_US", least)
+        assert part._outlasts_launches(x) == (least == 0)
+        runs.append(part.forward(x, ctx).clone())
+    assert torch.equal(runs[0], runs[1]) and torch.equal(runs[0], runs[2])
