@@ -21,8 +21,8 @@
 // waited for the softmax left the tensor core idle during its waits.
 //
 // Every mbarrier wait is bounded (two seconds); a wait that runs out sets *error_flag and the
-// block winds down.  Other head sizes, page sizes other than 8/16/32/64 and windows
-// are served by the m16n8k16 kernel of attention_prefill.cu.  A second kernel below takes heads of 64 in groups
+// block winds down.  Other head sizes, page sizes other than 8/16/32/64, capped scores and
+// values of another width than the keys are served by the m16n8k16 kernel of attention_prefill.cu.  A second kernel below takes heads of 64 in groups
 // of an even size, two query heads to a block.
 #include "latent_flat.cuh"
 #include "tcgen05_utils.cuh"

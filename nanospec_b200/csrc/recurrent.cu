@@ -11,8 +11,9 @@
 // from one token to the next; k . q per token and key head comes from the preparation.
 // The columns of S never meet: column e needs only v[e], so the scan runs one column per group of four
 // lanes (each lane holds a quarter of the column's D entries in registers), walks the request's tokens of
-// this step in order, and leaves the state where the next step finds it.  A request's result therefore
-// does not depend on how its tokens were cut into steps: the operations per token are the same.
+// this step in order, and leaves the state where the next step finds it.  The operations per
+// token are the same however a request's tokens are cut into steps (long portions of prompts go in chunks instead, linear_chunked.cu and
+// ssm_chunked.cu, which sum in another order).
 //
 // Everything that enters the recurrence is prepared in float by a kernel with one block per token
 // (`*_prepare`): q, k (a head's row padded with zeros to a multiple of 4 * R floats), v, and for the delta

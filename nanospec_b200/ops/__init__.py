@@ -711,7 +711,7 @@ def attention_prefill(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, 
                       out_scale: float = 1.0) -> None:
     """Tensor-core attention for portions of prompts.  `tiles`: int32 [n, 2] of (request, offset
     among its tokens of this step).  Head sizes 64 and 128 with pages of 8 to 64 tokens run
-    on tcgen05 (csrc/attention_prefill_tc.cu); everything else on m16n8k16 (csrc/attention_prefill.cu), also values of
+    on tcgen05, windows, kept keys, chunks, wide weights, sinks and gates included (csrc/attention_prefill_tc.cu); everything else on m16n8k16 (csrc/attention_prefill.cu), also values of
     another width than the keys (`v_dim`, both multiples of 8) and capped scores."""
     v_dim = head_dim if v_dim is None else v_dim
     if USE_TCGEN05_ATTENTION and tiles_tc is not None and head_dim in (64, 128) and not softcap and v_dim == head_dim and scale > 0 \
@@ -776,14 +776,15 @@ def attention(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, nkv: int
     bfloat16 with a head size that the tensor-core kernels take: the decode kernel for requests
     that bring one token, the prefill kernel for the others.  `wide_weights`: the softmax weights meet the values
     with about 16 bits each (two bfloat16 products per weight) instead of 8, for designs that state their weights in
-    float32; the m16n8k16 kernels have it.  `chunk` > 0: a query sees only the keys of its own chunk of that many
+    float32; the tcgen05 prefill kernel and the m16n8k16 kernels have it.  `chunk` > 0: a query sees only the keys of its own chunk of that many
     positions, counted from the start of the sequence; `softcap` > 0: a scaled score s becomes softcap * tanh(s / softcap) (the exact and
     the m16n8k16 kernels); `v_dim`: values of another width than the keys (the same kernels, widths in multiples of 8).
     `sink` (float32 [nq]): the softmax's denominator also holds exp(sink[h]), a term that has no key and no value and counts once
     (zeros: "one added to the denominator"); `gate` ([N, >= nq] in the activations' dtype, a column range of the packed projection
     is fine): head h's output is multiplied by sigmoid(gate[n, h]), or, with `feature_gate` ([N, >= nq * v_dim]), every output feature
-    by the sigmoid of its own; `out_scale` multiplies the output before it is rounded.  They run in the exact and the m16n8k16 kernels.  float32, and head
-    sizes those kernels refuse: the exact kernel, one warp per (token, head)."""
+    by the sigmoid of its own; `out_scale` multiplies the output before it is rounded.  They run in the exact, the tcgen05 prefill
+    and the m16n8k16 kernels.  float32, and head sizes those kernels refuse: the exact kernel, one warp per (token, head); float32 portions of
+    prompts its sums with keys and values shared (csrc/attention_f32.cu)."""
     v_dim = head_dim if v_dim is None else v_dim
     keep_first = keep_first if window else 0
     if not _tensor_core_attention(qkv.dtype, head_dim, v_dim) or nq // nkv > 64 or (v_dim != head_dim and (nq * head_dim) % 8) \

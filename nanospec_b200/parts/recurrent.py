@@ -1,7 +1,7 @@
 """Mixers whose memory is a matrix per head instead of a growing cache: retention (linear attention with a fixed decay
 per head), the gated delta rule and the state space of Mamba-2.  All keep S [heads, head_dim, v_dim] in float32 in the request's state slot and walk
-a step's tokens in order (csrc/recurrent.cu), so portions of a prompt, single decoded tokens and whole prompts give the
-same numbers; under CUDA graphs they address the state through the device's `qo_indptr` and `state_slot`.
+a step's tokens in order (csrc/recurrent.cu), or long portions of prompts in chunks of 64 tokens (csrc/linear_chunked.cu, csrc/ssm_chunked.cu:
+products over a chunk's tokens, the state carried between chunks; the same sums in another order); under CUDA graphs they address the state through the device's `qo_indptr` and `state_slot`.
 
     retention   S_t = decay_h S_(t-1) + k_t v_t^T,  o_t = S_t^T q_t;  q and k rotated by position, k times head_dim^-1/2;
                 per head o / rms(o), all heads times silu(gate), output projection.
@@ -13,8 +13,6 @@ same numbers; under CUDA graphs they address the state through the device's `qo_
                 a = softplus(dt + dt_bias) is the step size of a head and exp(-exp(A_log) a) its decay g;
                 S_t = g S_(t-1) + B_t (a x_t)^T,  o_t = S_t^T C_t + D x_t, B and C shared by the heads of a group;
                 (o silu(z)) normed in equal parts, each by its own root mean square, times a gain, output projection.
-                Long portions of prompts run in chunks of 64 tokens (csrc/ssm_chunked.cu: products over the chunk's tokens, the state
-                carried between chunks), the same sums in another order.
 
 The projections are one packed product; the convolution, the rotation, the unit norms, the decay and the read-out's norm are
 float32.
