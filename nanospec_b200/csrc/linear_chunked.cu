@@ -12,6 +12,8 @@
 //     chunk_solve    every chunk and head at once: A, T (blocks of 16 by substitution, joined by products), W and T (beta V)
 //     chunk_walk     the chunks of a request in order, 16 columns of S to a block: U, S_out, and S_in left for the next kernel
 //     chunk_read     every chunk and head at once: the read-out
+// A weight that the masks above leave out is skipped, not multiplied as a zero: a NaN or an infinity of one token stays out of the tokens
+// before it, as in the walk by token.
 // Everything is float, L and its differences double; products are fp32 FMAs on the CUDA cores.  The products' bound is what shared
 // memory can return: 12 words to 32 FMAs a thread (8 x 4 tiles).  The kernels let their successor in when their products are done (blocks
 // placed earlier would land unevenly).
@@ -73,7 +75,8 @@ __device__ __forceinline__ void gate_logs(const float* __restrict__ gate, int ld
         const double v = __shfl_up_sync(0xffffffffu, sum, o);
         if (lane >= o) sum += v;
     }
-    L[t0] = sum - l1;
+    const double before = __shfl_up_sync(0xffffffffu, sum, 1);
+    L[t0] = lane ? before + l0 : l0;  // (not sum - l1, which a later token's infinity would make a NaN)
     L[t1] = sum;
 }
 
@@ -181,7 +184,8 @@ chunk_solve_kernel(const float* __restrict__ k, const float* __restrict__ v, con
             const int bi = n + off, bj = n;
             float sum = 0.f;
 #pragma unroll
-            for (int kk = 0; kk < 16; ++kk) sum = fmaf(Ts[(bi * 16 + r) * kLdT + bi * 16 + kk], tmp[(n * 16 + kk) * 17 + cc], sum);
+            for (int kk = 0; kk < 16; ++kk)
+                if (kk <= r) sum = fmaf(Ts[(bi * 16 + r) * kLdT + bi * 16 + kk], tmp[(n * 16 + kk) * 17 + cc], sum);
             Ts[(bi * 16 + r) * kLdT + bj * 16 + cc] = -sum;
         }
         __syncthreads();
@@ -190,23 +194,28 @@ chunk_solve_kernel(const float* __restrict__ k, const float* __restrict__ v, con
     auto product = [&](const float* x, int ldx, int cols, float* dst, int ld_dst) {
         if (lane * 4 < cols) {
             float acc[8][4] = {};
-            for (int s = 0; s < 8 * warp + 8; s += 4) {
+            auto add = [&](int s, int first) {  // columns s .. s + 3 of T; in the diagonal block row i ends at its own column, first + i
                 float4 b[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) b[u] = ld4(x + (s + u) * ldx + lane * 4);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
+                    if (first + i < 0) continue;
                     const float4 a = ld4(Ts + (8 * warp + i) * kLdT + s);
                     const float av[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
+                        if (u > first + i) break;
                         acc[i][0] = fmaf(av[u], b[u].x, acc[i][0]);
                         acc[i][1] = fmaf(av[u], b[u].y, acc[i][1]);
                         acc[i][2] = fmaf(av[u], b[u].z, acc[i][2]);
                         acc[i][3] = fmaf(av[u], b[u].w, acc[i][3]);
                     }
                 }
-            }
+            };
+            for (int s = 0; s < 8 * warp; s += 4) add(s, 3);
+            add(8 * warp, 0);
+            add(8 * warp + 4, -4);
 #pragma unroll
             for (int i = 0; i < 8; ++i)
                 *reinterpret_cast<float4*>(dst + (size_t)(8 * warp + i) * ld_dst + lane * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
@@ -478,24 +487,32 @@ chunk_read_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     __syncthreads();
     for (int s0 = 0; s0 < tr + 32; s0 += 32) {
         float run[8][kTN] = {};
-#pragma unroll 2
-        for (int s = s0; s < s0 + 32; s += 4) {
+        // tokens s0 + 4 m .. + 3; in the diagonal block a row t = ly + 4 i (counted from s0) ends at its own token
+        auto add = [&](int m, bool diagonal) {
             float b[4][kTN];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
 #pragma unroll
-                for (int j = 0; j < kTN; ++j) b[u][j] = Xs[(s + u) * kLdU + vc + lx + 8 * j];
+                for (int j = 0; j < kTN; ++j) b[u][j] = Xs[(s0 + 4 * m + u) * kLdU + vc + lx + 8 * j];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const float4 a = ld4(Ms + (tr + ly + 4 * i) * kLdT + s);
+                if (diagonal && i < m) continue;
+                const float4 a = ld4(Ms + (tr + ly + 4 * i) * kLdT + s0 + 4 * m);
+                const float av[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-                for (int j = 0; j < kTN; ++j) {
-                    run[i][j] = fmaf(a.x, b[0][j], run[i][j]);
-                    run[i][j] = fmaf(a.y, b[1][j], run[i][j]);
-                    run[i][j] = fmaf(a.z, b[2][j], run[i][j]);
-                    run[i][j] = fmaf(a.w, b[3][j], run[i][j]);
-                }
+                for (int u = 0; u < 4; ++u)
+                    if (!diagonal || i > m || u <= ly) {
+#pragma unroll
+                        for (int j = 0; j < kTN; ++j) run[i][j] = fmaf(av[u], b[u][j], run[i][j]);
+                    }
             }
+        };
+        if (s0 < tr) {
+#pragma unroll 2
+            for (int m = 0; m < 8; ++m) add(m, false);
+        } else {
+#pragma unroll
+            for (int m = 0; m < 8; ++m) add(m, true);
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i)

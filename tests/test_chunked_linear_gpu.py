@@ -2,6 +2,7 @@
 
 from __future__ import annotations
 
+import math
 from types import SimpleNamespace
 
 import pytest
@@ -45,6 +46,12 @@ def _walk(rec, decay, state, lens, slots, H, G, D, V, gated):
     return torch.stack(outs), after
 
 
+def _context(lens, slots, ws):
+    return SimpleNamespace(n_requests=len(lens), extras={}, q_lens=lens, max_q_len=max(lens), state_slot=torch.tensor(slots, dtype=torch.int32, device=DEV),
+                           qo_indptr=torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV),
+                           buffer=lambda name, cols, dtype, rows: ws.get(name, rows, cols, dtype))
+
+
 @pytest.mark.parametrize("gated", [True, False])
 @pytest.mark.parametrize("lens,H,G,D,V", [([64], 1, 1, 128, 128), ([65, 3, 129], 4, 2, 128, 128), ([63, 1, 200], 2, 2, 64, 64),
                                           ([130, 66], 6, 2, 64, 192), ([257], 2, 1, 128, 256)])
@@ -61,10 +68,7 @@ def test_chunked_recurrence(lens, H, G, D, V, gated, monkeypatch):
     rec, decay, state = _operands(lens, H, G, D, V, gated, sum(lens) + H)
     slots = [len(lens) - i for i in range(len(lens))]
     want, after = _walk(rec, decay, state, lens, slots, H, G, D, V, gated)
-    ws = Workspace(DEV)
-    ctx = SimpleNamespace(n_requests=len(lens), extras={}, q_lens=lens, max_q_len=max(lens), state_slot=torch.tensor(slots, dtype=torch.int32, device=DEV),
-                          qo_indptr=torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV),
-                          buffer=lambda name, cols, dtype, rows: ws.get(name, rows, cols, dtype))
+    ctx = _context(lens, slots, Workspace(DEV))
     for limit in (1 << 28, 1):  # all heads in one pass, and a key head at a time
         monkeypatch.setattr(ops, "LINEAR_SCRATCH_MAX", limit)
         S, out = state.clone(), torch.full((sum(lens), H * V + 4), 7.0, device=DEV)
@@ -73,3 +77,43 @@ def test_chunked_recurrence(lens, H, G, D, V, gated, monkeypatch):
         assert float((out[:, : H * V].double() - want).norm() / want.norm()) < bound
         assert float((S.double() - after).norm() / after.norm()) < bound
         assert bool((out[:, H * V:] == 7.0).all()) and torch.equal(S[0], state[0]) and torch.equal(S[:, H * D * V:], state[:, H * D * V:])
+
+
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("H,G,D,V", [(2, 1, 128, 128), (4, 2, 64, 192)])
+@pytest.mark.parametrize("bad", [0, 1, 15, 70, 77, 127, 149])
+def test_a_token_that_is_no_number_leaves_earlier_ones_alone(bad, H, G, D, V, gated, monkeypatch):
+    """A NaN or an infinity in one operand of token `bad` of the first request: everything before it, the other request and the heads and
+    columns that it does not enter keep their bits; what the recurrence makes non-finite is non-finite."""
+    from nanospec_b200 import ops
+    from nanospec_b200.parts import Workspace
+    if not gated:
+        G = H
+    lens, slots = [150, 70], [1, 2]
+    monkeypatch.setattr(ops, "LINEAR_CHUNKED_MIN", 64)
+    monkeypatch.setattr(ops, "LINEAR_CHUNKED_COST", (0, 0.0))
+    rec, decay, state = _operands(lens, H, G, D, V, gated, bad + H)
+    ctx = _context(lens, slots, Workspace(DEV))
+
+    def run(r):
+        S, out = state.clone(), torch.empty(sum(lens), H * V, device=DEV)
+        ops.linear_mix(r, S, ctx, out, H, G, D, V, decay=None if gated else decay, gated=gated)
+        return out, S
+    clean, S_clean = run(rec)
+    v0 = 2 * G * D
+    for col, value in [(v0 + V + 5, math.nan), (v0 + V + 5, math.inf), (G * D + 3, math.nan), (G * D + 3, -math.inf), (3, math.nan)] \
+            + ([(v0 + H * V + H, math.nan)] if gated else []):
+        worse = rec.clone()
+        worse[bad, col] = value
+        out, S = run(worse)
+        want, after = _walk(worse, decay, state, lens, slots, H, G, D, V, gated)
+        untouched = torch.ones_like(out, dtype=torch.bool)
+        if col >= v0 + H * V:
+            untouched[bad: 150, :V] = False                      # the first head's write strength
+        elif col >= v0:
+            untouched[bad: 150, V + 5] = False                   # one column of the second head's values
+        else:
+            untouched[bad: 150, : H // G * V] = False            # the first key head
+        assert torch.equal(out[untouched], clean[untouched]), (col, value)
+        assert not bool(out[~want.isfinite()].isfinite().any()) and not bool(S[~after.isfinite()].isfinite().any()), (col, value)
+        assert torch.equal(S[2], S_clean[2])
