@@ -61,12 +61,13 @@ __device__ __forceinline__ void dot_rows(float (&acc)[TM][TN], const float* a, i
 }
 
 // L of the chunk's tokens by one warp, two to a lane; tokens beyond the chunk do not decay.  `gate`: decays per token (row stride ld), or
-// null: `fixed`.  A decay of 0 counts as exp(-200), whose float is 0, so that differences stay numbers.
+// null: `fixed`.  A decay of 0 counts as exp(-200), whose float is 0, so that differences stay numbers; one that is no number, or negative, has no
+// logarithm and makes what it enters a NaN.
 __device__ __forceinline__ void gate_logs(const float* __restrict__ gate, int ld, float fixed, int start, int count, double* L) {
     const int lane = threadIdx.x & 31, t0 = 2 * lane, t1 = t0 + 1;
     auto log_of = [&](int t) {
         const float g = t >= count ? 1.f : gate ? gate[(size_t)(start + t) * ld] : fixed;
-        return g > 0.f ? log((double)g) : -200.0;
+        return g == 0.f ? -200.0 : log((double)g);
     };
     const double l0 = log_of(t0), l1 = log_of(t1);
     double sum = l0 + l1;

@@ -1049,7 +1049,8 @@ LINEAR_SCRATCH_MAX = 1 << 28  # bytes of chunk scratch; a step that would need m
 
 def linear_mix(rec: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, heads: int, kv_heads: int, head_dim: int, v_dim: int,
                decay: torch.Tensor | None = None, gated: bool = False) -> torch.Tensor:
-    """Retention (`decay`) or the gated delta rule (`gated`) over each request's tokens of this step, operands as `linear_scan` takes them.
+    """Retention (`decay`, none of them negative) or the gated delta rule (`gated`) over each request's tokens of this step, operands as
+    `linear_scan` takes them.
     Long portions of prompts go 64 tokens at a time where the heads' sizes allow it (csrc/linear_chunked.cu), everything else token by
     token."""
     lens = [1] * ctx.n_requests if ctx.extras.get("graph") else ctx.q_lens

@@ -51,6 +51,7 @@ class Retention(Part):
         if len(decay) != self.heads:
             raise ValueError(f"retention: {len(decay)} decays for {self.heads} heads")
         self.decay_host = torch.tensor(decay, dtype=torch.float32)
+        self.mix = ops.linear_mix if all(d >= 0.0 for d in decay) else ops.linear_scan  # (the chunks take logarithms of the decays)
         self._decay: torch.Tensor | None = None
         self.position = build_part("position", p["position"], dtype, device) if p.get("position") is not None else None
         names = dict(p.get("names") or {})
@@ -89,8 +90,8 @@ class Retention(Part):
         ops.rotary_prepare(proj, ctx, pos.inv_freq if pos is not None and pos.dims else None, pos.magnitude if pos is not None else 1.0,
                            pos.interleaved if pos is not None else False, rec, self.heads, self.head_dim, self.v_dim,
                            1.0, self.head_dim ** -0.5)
-        read = ops.linear_mix(rec, lane.state, ctx, ctx.buffer("rec_out", self.v_size, torch.float32), self.heads, self.heads,
-                              self.head_dim, self.v_dim, decay=self._decay)
+        read = self.mix(rec, lane.state, ctx, ctx.buffer("rec_out", self.v_size, torch.float32), self.heads, self.heads,
+                        self.head_dim, self.v_dim, decay=self._decay)
         gate = proj[:, 2 * self.qk_size + self.v_size: 2 * self.qk_size + 2 * self.v_size]
         y = ops.head_norm_gate(read, gate, None, self.eps, ctx.buffer("rec_y", self.v_size), ctx, self.heads, self.v_dim)
         return ops.linear(y, self.w_o, ctx.buffer("branch", self.hidden))

@@ -117,3 +117,44 @@ def test_a_token_that_is_no_number_leaves_earlier_ones_alone(bad, H, G, D, V, ga
         assert torch.equal(out[untouched], clean[untouched]), (col, value)
         assert not bool(out[~want.isfinite()].isfinite().any()) and not bool(S[~after.isfinite()].isfinite().any()), (col, value)
         assert torch.equal(S[2], S_clean[2])
+
+
+@pytest.mark.parametrize("gated", [True, False])
+def test_a_decay_that_is_no_number_is_carried_on(gated, monkeypatch):
+    """A NaN among the decays enters everything from its token (retention: of its head) on, and a decay of zero next to it stays a number."""
+    from nanospec_b200 import ops
+    from nanospec_b200.parts import Workspace
+    H, D, V, lens = 2, 64, 64, [150]
+    monkeypatch.setattr(ops, "LINEAR_CHUNKED_MIN", 64)
+    monkeypatch.setattr(ops, "LINEAR_CHUNKED_COST", (0, 0.0))
+    rec, decay, state = _operands(lens, H, H, D, V, gated, 3)
+    at = 2 * H * D + H * V
+    if gated:
+        rec[60, at: at + 2] = 0.0
+        rec[77, at + 1] = math.nan
+    else:
+        decay[:] = torch.tensor([0.0, math.nan])
+    S, out = state.clone(), torch.empty(150, H * V, device=DEV)
+    ops.linear_mix(rec, S, _context(lens, [1], Workspace(DEV)), out, H, H, D, V, decay=None if gated else decay, gated=gated)
+    want, after = _walk(rec, decay, state, lens, [1], H, H, D, V, gated)
+    assert torch.equal(out.isfinite(), want.isfinite()) and torch.equal(S.isfinite(), after.isfinite())
+    sound = want.isfinite()
+    assert float((out[sound].double() - want[sound]).norm() / want[sound].norm()) < 4 * 320 ** 0.5 * 2.0 ** -24
+
+
+def test_negative_decays_are_walked():
+    """The sign of a fixed decay alternates from token to token, which a sum of logarithms does not hold: such a layer goes token by token."""
+    from nanospec_b200 import ops
+    from nanospec_b200.config import PartSpec
+    from nanospec_b200.parts import Workspace, build_part
+    spec = {"hidden": 128, "heads": 2, "head_dim": 64, "v_dim": 64, "eps": 1e-6, "position": None}
+    for decay, mix in (((0.5, -0.25), ops.linear_scan), ((0.5, 0.0), ops.linear_mix), ((math.nan, 0.5), ops.linear_scan)):
+        part = build_part("mixer", PartSpec("retention", {**spec, "decay": decay}), torch.float32, DEV)
+        assert part.mix is mix
+    rec, _, state = _operands([300], 2, 2, 64, 64, False, 1)
+    decay = torch.tensor([0.9, -0.95], device=DEV)
+    part = build_part("mixer", PartSpec("retention", {**spec, "decay": decay.tolist()}), torch.float32, DEV)
+    S, out = state.clone(), torch.empty(300, 128, device=DEV)
+    part.mix(rec, S, _context([300], [1], Workspace(DEV)), out, 2, 2, 64, 64, decay=decay)
+    want, _ = _walk(rec, decay, state, [300], [1], 2, 2, 64, 64, False)
+    assert float((out.double() - want).norm() / want.norm()) < 4 * 320 ** 0.5 * 2.0 ** -24
