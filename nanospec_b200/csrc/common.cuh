@@ -150,7 +150,8 @@ __device__ __forceinline__ float ns_block_max(float v, float* scratch) {
 // which covers the grid directly before it only, would no longer mean "everything earlier is done".
 // A launch right after streams have forked or joined is made without it (ns_full_launch_next): such a kernel has prerequisites
 // beside its predecessor in the stream, and starts when all of them are complete.
-extern int ns_pdl_enabled, ns_pdl_skip_one;
+extern int ns_pdl_enabled;
+extern thread_local int ns_pdl_skip_one;  // of the thread that forked or joined: another thread's launch must not take it
 inline bool ns_take_pdl() {
     const bool use = ns_pdl_enabled && !ns_pdl_skip_one;
     ns_pdl_skip_one = 0;

@@ -8,13 +8,16 @@
 thread_local char ns_error_text[512] = "";
 NS_API const char* ns_last_error() { return ns_error_text; }
 
-int ns_pdl_enabled = 1, ns_pdl_skip_one = 0;
+int ns_pdl_enabled = 1;
+thread_local int ns_pdl_skip_one = 0;
 
-// The next kernel launch (on whatever stream) starts only when everything before it is complete.
+// The calling thread's next kernel launch (on whatever stream) starts only when everything before it is complete.
 NS_API int ns_full_launch_next() {
     ns_pdl_skip_one = 1;
     return NS_OK;
 }
+// Whether that is still to come (1) or has been taken by a launch of this thread (0).
+NS_API int ns_full_launch_pending() { return ns_pdl_skip_one; }
 // 1 (default): kernels are launched so that they may overlap the tail of their predecessor
 // (programmatic dependent launch); 0: plain stream order.
 NS_API int ns_set_pdl(int enabled) {

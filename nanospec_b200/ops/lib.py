@@ -52,6 +52,7 @@ _SIGNATURES: dict[str, list] = {
                              _P, _P],
     "ns_set_pdl": [_I],
     "ns_full_launch_next": [],
+    "ns_full_launch_pending": [],
     "ns_attention_decode_stages": [_I],
     "ns_gemm_bf16_tc": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "ns_gemm_bf16_tc_gated": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
