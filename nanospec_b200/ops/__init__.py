@@ -1044,7 +1044,16 @@ LINEAR_CHUNKED_COST = (140, 0.36)
 # ... and while the token walk has at most so many warps' worth of columns an SM: it needs fewer operations and wins once it fills the GPU
 # (8 requests of 256 tokens, 512 blocks of 32 columns: 261 us by token, 279 by chunk; 2 requests, 256 blocks: 1136 and 928)
 LINEAR_CHUNKED_BLOCKS = 2
-LINEAR_SCRATCH_MAX = 1 << 28  # bytes of chunk scratch; a step that would need more runs its heads in groups
+LINEAR_SCRATCH_MAX = 1 << 28  # bytes of chunk scratch; a step that would need more runs its heads in groups, one of which a head exceeds by token
+
+
+def head_passes(heads: int, kv_heads: int, limit: int) -> list[tuple[int, int, int, int]]:
+    """(first head, heads, first key head, key heads) of passes of at most `limit` heads each: whole key heads, or parts of one."""
+    per_kv = heads // kv_heads
+    if limit >= per_kv:
+        step = limit // per_kv
+        return [(g * per_kv, min(step, kv_heads - g) * per_kv, g, min(step, kv_heads - g)) for g in range(0, kv_heads, step)]
+    return [(g * per_kv + h, min(limit, per_kv - h), g, 1) for g in range(kv_heads) for h in range(0, per_kv, limit)]
 
 
 def linear_mix(rec: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, heads: int, kv_heads: int, head_dim: int, v_dim: int,
@@ -1056,9 +1065,12 @@ def linear_mix(rec: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, h
     lens = [1] * ctx.n_requests if ctx.extras.get("graph") else ctx.q_lens
     least, dp = LINEAR_CHUNKED_MIN, scan_padded_dim(head_dim)
     chunks = sum(-(-n // LINEAR_CHUNK) for n in lens if n >= least)
+    # floats that a chunk of a head leaves: its state, two factors per token and, for the delta rule, the two solved sides (csrc/linear_chunked.cu)
+    per_item = v_dim * head_dim + LINEAR_CHUNK + 4 + (LINEAR_CHUNK * (head_dim + v_dim) if gated else 0)
+    at_once = min(heads, LINEAR_SCRATCH_MAX // (4 * per_item * max(chunks, 1)))  # heads to a pass
     walked = sum(n >= least for n in lens) * heads * (v_dim // 32)
     longest, short = max(lens, default=0), max((n for n in lens if n < least), default=0)
-    if not chunks or longest < short + LINEAR_CHUNKED_COST[0] + LINEAR_CHUNKED_COST[1] * longest \
+    if not chunks or not at_once or longest < short + LINEAR_CHUNKED_COST[0] + LINEAR_CHUNKED_COST[1] * longest \
             or walked > LINEAR_CHUNKED_BLOCKS * sm_count() or head_dim not in (64, 128) or v_dim % 64 or rec.stride(0) % 4 \
             or rec.data_ptr() % 16:
         return linear_scan(rec, state, ctx, out, heads, kv_heads, head_dim, v_dim, decay=decay, gated=gated)
@@ -1070,20 +1082,15 @@ def linear_mix(rec: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, h
     if short:
         linear_scan(rec, state, ctx, out, heads, kv_heads, head_dim, v_dim, decay=decay, gated=gated, longest=short, max_len=least - 1)
     _cuda(rec, state, out, decay)
-    # a chunk of a head leaves its state, two factors per token and, for the delta rule, the two solved sides (csrc/linear_chunked.cu)
-    per_item = v_dim * head_dim + LINEAR_CHUNK + 4 + (LINEAR_CHUNK * (head_dim + v_dim) if gated else 0)
-    per_kv = heads // kv_heads
-    groups = min(kv_heads, max(1, LINEAR_SCRATCH_MAX // (4 * per_item * chunks * per_kv)))  # key heads to a pass
-    scratch = ctx.buffer("linear_chunks", 4, torch.float32, rows=-(-per_item * chunks * per_kv * groups // 4) + 1)
+    passes = head_passes(heads, kv_heads, at_once)
+    scratch = ctx.buffer("linear_chunks", 4, torch.float32, rows=-(-per_item * chunks * max(n for _, n, _, _ in passes) // 4) + 1)
     base, d0 = rec.data_ptr(), decay.data_ptr() if decay is not None and not gated else 0
-    for g0 in range(0, kv_heads, groups):
-        G = min(groups, kv_heads - g0)
-        h0 = g0 * per_kv
+    for h0, H, g0, G in passes:
         gates = base + 4 * (off_v + heads * v_dim + h0)
         lib.call("ns_linear_chunked", base + 4 * g0 * dp, base + 4 * (kv_heads + g0) * dp, base + 4 * (off_v + h0 * v_dim),
                  gates if gated else None, gates + 4 * heads if gated else None, None if gated else d0 + 4 * h0, rec.stride(0),
                  state.data_ptr() + 4 * h0 * head_dim * v_dim, state.stride(0), ctx.qo_indptr.data_ptr(), ctx.state_slot.data_ptr(),
-                 out.data_ptr() + 4 * h0 * v_dim, out.stride(0), ctx.n_requests, least, chunks, scratch.data_ptr(), G * per_kv, G, head_dim, v_dim,
+                 out.data_ptr() + 4 * h0 * v_dim, out.stride(0), ctx.n_requests, least, chunks, scratch.data_ptr(), H, G, head_dim, v_dim,
                  _stream())
     return out
 

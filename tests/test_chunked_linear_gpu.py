@@ -69,7 +69,8 @@ def test_chunked_recurrence(lens, H, G, D, V, gated, monkeypatch):
     slots = [len(lens) - i for i in range(len(lens))]
     want, after = _walk(rec, decay, state, lens, slots, H, G, D, V, gated)
     ctx = _context(lens, slots, Workspace(DEV))
-    for limit in (1 << 28, 1):  # all heads in one pass, and a key head at a time
+    one = 4 * sum(-(-n // 64) for n in lens if n >= 64) * (V * D + 68 + (64 * (D + V) if gated else 0))  # bytes of a head's chunks
+    for limit in (1 << 28, one):  # all heads in one pass, and a head at a time
         monkeypatch.setattr(ops, "LINEAR_SCRATCH_MAX", limit)
         S, out = state.clone(), torch.full((sum(lens), H * V + 4), 7.0, device=DEV)
         ops.linear_mix(rec, S, ctx, out[:, : H * V], H, G, D, V, decay=None if gated else decay, gated=gated)
@@ -158,3 +159,28 @@ def test_negative_decays_are_walked():
     part.mix(rec, S, _context([300], [1], Workspace(DEV)), out, 2, 2, 64, 64, decay=decay)
     want, _ = _walk(rec, decay, state, [300], [1], 2, 2, 64, 64, False)
     assert float((out.double() - want).norm() / want.norm()) < 4 * 320 ** 0.5 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("H,G,limit,calls", [(6, 1, 6, 1), (6, 1, 4, 2), (6, 1, 1, 6), (6, 2, 5, 2), (6, 2, 2, 4), (6, 2, 0, 0)])
+def test_chunk_scratch_stays_below_its_limit(H, G, limit, calls, monkeypatch):
+    """Several heads to a key head: passes of parts of one, no more bytes than the limit, the same bits, and the walk where not even one
+    head's chunks fit."""
+    from nanospec_b200 import ops
+    from nanospec_b200.parts import Workspace
+    D = V = 64
+    lens, one = [200], 4 * 4 * (V * D + 68 + 64 * (D + V))
+    monkeypatch.setattr(ops, "LINEAR_CHUNKED_COST", (0, 0.0))
+    rec, _, state = _operands(lens, H, G, D, V, True, 7)
+    names, call = [], ops.lib.call
+    monkeypatch.setattr(ops.lib, "call", lambda name, *a: (names.append(name), call(name, *a)))
+    outs = []
+    for most in (1 << 28, limit * one + 15):
+        monkeypatch.setattr(ops, "LINEAR_SCRATCH_MAX", most)
+        names.clear()
+        ws, S, out = Workspace(DEV), state.clone(), torch.empty(200, H * V, device=DEV)
+        ops.linear_mix(rec, S, _context(lens, [1], ws), out, H, G, D, V, gated=True)
+        outs.append((out, S))
+        assert sum(b.numel() * b.element_size() for b in ws._bufs.values()) <= most + 32
+    assert names == ["ns_linear_chunked"] * calls or (not calls and names == ["ns_linear_scan"])
+    if calls:
+        assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
