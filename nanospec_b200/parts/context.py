@@ -20,6 +20,10 @@ class LaneView:
     state: torch.Tensor | None = None  # [slots, *state_shape] when the mixer asked for state
 
 
+# A buffer that grows is doubled, so that steps of slowly growing size do not each allocate, but by no more bytes than this beyond what is asked.
+GROWTH_SPARE_MAX = 64 << 20
+
+
 class Workspace:
     """Scratch activations keyed by (name, columns, dtype), sized for the largest step seen.
     Buffers are reused by every layer, so a model's activations cost one layer's worth."""
@@ -37,10 +41,12 @@ class Workspace:
         if buf is None or buf.shape[0] < rows:
             if self.frozen and buf is not None:
                 raise RuntimeError(f"workspace buffer {name!r} would have to grow while CUDA graphs point into it")
-            cap = max(rows, 16 if buf is None else 2 * buf.shape[0])
+            spare = GROWTH_SPARE_MAX // max(1, cols * dtype.itemsize)
+            cap = max(rows, 16 if buf is None else min(2 * buf.shape[0], rows + spare))
             make = torch.zeros if zero else torch.empty
-            buf = make((cap, cols), dtype=dtype, device=self.device)
-            self._bufs[key] = buf
+            buf = self._bufs.pop(key, None)
+            del buf  # the old one is free again before the new one is made
+            buf = self._bufs[key] = make((cap, cols), dtype=dtype, device=self.device)
         return buf[:rows]
 
     def reserve(self, rows: int) -> None:
