@@ -1036,14 +1036,49 @@ def linear_scan(rec: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, 
 
 LINEAR_CHUNK = 64          # tokens of a chunk in csrc/linear_chunked.cu
 # Requests of at least so many tokens in a step go a chunk at a time, shorter ones a token at a time (one request, 16 heads of 128 x 128,
-# delta rule: 128 tokens 46 us by token and 59 by chunk, 256 tokens 87 and 67, 2,048 tokens 650 and 276; retention 601 and 170) ...
+# delta rule: 128 tokens 46 us by token and 59 by chunk, 256 tokens 80 and 65, 2,048 tokens 620 and 272; retention 574 and 166) ...
 LINEAR_CHUNKED_MIN = 192
-# ... while the longest makes up for the pass that the shorter ones need beside it: in tokens of the walk (0.32 us each, of the longest alone)
-# a chunked pass costs about 140 and 0.36 a token (8 requests of 99 to 193 tokens: 249 us walked together, 317 with the longest in chunks) ...
-LINEAR_CHUNKED_COST = (140, 0.36)
-# ... and while the token walk has at most so many warps' worth of columns an SM: it needs fewer operations and wins once it fills the GPU
-# (8 requests of 256 tokens, 512 blocks of 32 columns: 261 us by token, 279 by chunk; 2 requests, 256 blocks: 1136 and 928)
+# ... while the chunks, with a pass of the walk for the shorter ones beside them, are expected to take less than the walk of all: (us, factor) ...
+LINEAR_CHUNKED_COST = (5, 1.05)
+# ... and while the token walk has at most so many warps' worth of columns an SM
 LINEAR_CHUNKED_BLOCKS = 2
+# us a token of the walk by blocks of 32 columns side by side: the chain of a token, the GPU filling up, the GPU full (D 128: 0.30 with 64 blocks,
+# 0.40 with 128, 0.55 with 256, 0.99 with 512; D 64: 0.25, 0.30, 0.41, 0.68)
+LINEAR_WALK_US = {64: (0.248, (0.19, 0.0008), 0.00133), 128: (0.30, (0.25, 0.0012), 0.0019)}
+
+
+def _walk_us(lens: list[int], heads: int, head_dim: int, v_dim: int) -> float:
+    longest = max(lens, default=0)
+    if not longest:
+        return 0.0
+    blocks = sum(lens) / longest * heads * v_dim / 32
+    chain, (filling, more), full = LINEAR_WALK_US[head_dim]
+    return longest * max(chain, filling + more * blocks, full * blocks)
+
+
+def _chunks_us(lens: list[int], heads: int, head_dim: int, v_dim: int, gated: bool) -> float:
+    """The chain from chunk to chunk of the longest request, or every chunk of every head, whichever takes longer (delta rule, 128 x 128: 8 heads
+    and 32 chunks 199 us, 16 heads and 128 chunks 1,089; 64 x 64: 4 heads and 32 chunks 127, 16 heads and 128 chunks 554)."""
+    chunks = [-(-n // LINEAR_CHUNK) for n in lens]
+    items = sum(chunks) * heads
+    if gated:
+        return max(22 + 0.2 * head_dim + (1.1 + 0.028 * head_dim) * max(chunks), 15 + (0.2 + 2e-5 * head_dim * v_dim) * items)
+    return max(14 + 0.094 * head_dim + (0.5 + 0.019 * head_dim) * max(chunks), 15 + (0.05 + 1.2e-5 * head_dim * v_dim) * items)
+
+
+def chunks_pay(lens: list[int], heads: int, head_dim: int, v_dim: int, gated: bool) -> bool:
+    """Whether a step whose requests bring `lens` tokens runs those of LINEAR_CHUNKED_MIN and more in chunks (15 steps through 12 layers measured:
+    nowhere more than 3 % above the walk)."""
+    if head_dim not in LINEAR_WALK_US:
+        return False
+    long = [n for n in lens if n >= LINEAR_CHUNKED_MIN]
+    if not long or len(long) * heads * (v_dim // 32) > LINEAR_CHUNKED_BLOCKS * sm_count():
+        return False
+    short = [n for n in lens if n < LINEAR_CHUNKED_MIN]
+    cost = _chunks_us(long, heads, head_dim, v_dim, gated) + _walk_us(short, heads, head_dim, v_dim)
+    return LINEAR_CHUNKED_COST[0] + LINEAR_CHUNKED_COST[1] * cost < _walk_us(lens, heads, head_dim, v_dim)
+
+
 LINEAR_SCRATCH_MAX = 1 << 28  # bytes of chunk scratch; a step that would need more runs its heads in groups, one of which a head exceeds by token
 
 
@@ -1068,11 +1103,8 @@ def linear_mix(rec: torch.Tensor, state: torch.Tensor, ctx, out: torch.Tensor, h
     # floats that a chunk of a head leaves: its state, two factors per token and, for the delta rule, the two solved sides (csrc/linear_chunked.cu)
     per_item = v_dim * head_dim + LINEAR_CHUNK + 4 + (LINEAR_CHUNK * (head_dim + v_dim) if gated else 0)
     at_once = min(heads, LINEAR_SCRATCH_MAX // (4 * per_item * max(chunks, 1)))  # heads to a pass
-    walked = sum(n >= least for n in lens) * heads * (v_dim // 32)
-    longest, short = max(lens, default=0), max((n for n in lens if n < least), default=0)
-    if not chunks or not at_once or longest < short + LINEAR_CHUNKED_COST[0] + LINEAR_CHUNKED_COST[1] * longest \
-            or walked > LINEAR_CHUNKED_BLOCKS * sm_count() or head_dim not in (64, 128) or v_dim % 64 or rec.stride(0) % 4 \
-            or rec.data_ptr() % 16:
+    short = max((n for n in lens if n < least), default=0)
+    if not chunks or not at_once or not chunks_pay(lens, heads, head_dim, v_dim, gated) or v_dim % 64 or rec.stride(0) % 4 or rec.data_ptr() % 16:
         return linear_scan(rec, state, ctx, out, heads, kv_heads, head_dim, v_dim, decay=decay, gated=gated)
     off_v = 2 * kv_heads * dp
     if rec.dtype != torch.float32 or out.dtype != torch.float32 or state.dtype != torch.float32 or rec.stride(1) != 1 or out.stride(1) != 1 \

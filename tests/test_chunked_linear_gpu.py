@@ -8,7 +8,6 @@ from types import SimpleNamespace
 import pytest
 import torch
 
-pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda")
 
 
@@ -52,6 +51,7 @@ def _context(lens, slots, ws):
                            buffer=lambda name, cols, dtype, rows: ws.get(name, rows, cols, dtype))
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("gated", [True, False])
 @pytest.mark.parametrize("lens,H,G,D,V", [([64], 1, 1, 128, 128), ([65, 3, 129], 4, 2, 128, 128), ([63, 1, 200], 2, 2, 64, 64),
                                           ([130, 66], 6, 2, 64, 192), ([257], 2, 1, 128, 256)])
@@ -70,16 +70,21 @@ def test_chunked_recurrence(lens, H, G, D, V, gated, monkeypatch):
     want, after = _walk(rec, decay, state, lens, slots, H, G, D, V, gated)
     ctx = _context(lens, slots, Workspace(DEV))
     one = 4 * sum(-(-n // 64) for n in lens if n >= 64) * (V * D + 68 + (64 * (D + V) if gated else 0))  # bytes of a head's chunks
-    for limit in (1 << 28, one):  # all heads in one pass, and a head at a time
+    names, call = [], ops.lib.call
+    monkeypatch.setattr(ops.lib, "call", lambda name, *a: (names.append(name), call(name, *a)))
+    for limit, passes in ((1 << 28, 1), (one, H)):  # all heads in one pass, and a head at a time
         monkeypatch.setattr(ops, "LINEAR_SCRATCH_MAX", limit)
+        names.clear()
         S, out = state.clone(), torch.full((sum(lens), H * V + 4), 7.0, device=DEV)
         ops.linear_mix(rec, S, ctx, out[:, : H * V], H, G, D, V, decay=None if gated else decay, gated=gated)
+        assert names.count("ns_linear_chunked") == passes and names.count("ns_linear_scan") == (min(lens) < 64)
         bound = 4 * 320 ** 0.5 * 2.0 ** -24
         assert float((out[:, : H * V].double() - want).norm() / want.norm()) < bound
         assert float((S.double() - after).norm() / after.norm()) < bound
         assert bool((out[:, H * V:] == 7.0).all()) and torch.equal(S[0], state[0]) and torch.equal(S[:, H * D * V:], state[:, H * D * V:])
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("gated", [True, False])
 @pytest.mark.parametrize("H,G,D,V", [(2, 1, 128, 128), (4, 2, 64, 192)])
 @pytest.mark.parametrize("bad", [0, 1, 15, 70, 77, 127, 149])
@@ -120,6 +125,7 @@ def test_a_token_that_is_no_number_leaves_earlier_ones_alone(bad, H, G, D, V, ga
         assert torch.equal(S[2], S_clean[2])
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("gated", [True, False])
 def test_a_decay_that_is_no_number_is_carried_on(gated, monkeypatch):
     """A NaN among the decays enters everything from its token (retention: of its head) on, and a decay of zero next to it stays a number."""
@@ -143,6 +149,7 @@ def test_a_decay_that_is_no_number_is_carried_on(gated, monkeypatch):
     assert float((out[sound].double() - want[sound]).norm() / want[sound].norm()) < 4 * 320 ** 0.5 * 2.0 ** -24
 
 
+@pytest.mark.gpu
 def test_negative_decays_are_walked():
     """The sign of a fixed decay alternates from token to token, which a sum of logarithms does not hold: such a layer goes token by token."""
     from nanospec_b200 import ops
@@ -161,6 +168,7 @@ def test_negative_decays_are_walked():
     assert float((out.double() - want).norm() / want.norm()) < 4 * 320 ** 0.5 * 2.0 ** -24
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("H,G,limit,calls", [(6, 1, 6, 1), (6, 1, 4, 2), (6, 1, 1, 6), (6, 2, 5, 2), (6, 2, 2, 4), (6, 2, 0, 0)])
 def test_chunk_scratch_stays_below_its_limit(H, G, limit, calls, monkeypatch):
     """Several heads to a key head: passes of parts of one, no more bytes than the limit, the same bits, and the walk where not even one
@@ -184,3 +192,50 @@ def test_chunk_scratch_stays_below_its_limit(H, G, limit, calls, monkeypatch):
     assert names == ["ns_linear_chunked"] * calls or (not calls and names == ["ns_linear_scan"])
     if calls:
         assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("lens,H,D,V,gated,chunked", [
+    # us by token, in chunks (B200)
+    ([1000], 16, 128, 128, True, True),              # 304, 134
+    ([256], 32, 128, 128, True, True),               # 106, 90
+    ([600, 100], 16, 128, 128, True, True),          # 228, 143
+    ([2048, 2048], 16, 128, 128, True, True),        # 818, 538
+    ([2000] + [1] * 7, 32, 128, 128, True, True),    # 1056, 540
+    ([300] * 4, 4, 64, 64, True, True),              # 77, 51
+    ([300] * 4, 16, 128, 128, False, True),          # 153, 103
+    ([192, 191], 16, 128, 128, True, False),         # 81, 147
+    ([300, 150], 16, 128, 128, True, False),         # 120, 142
+    ([300] * 4, 16, 128, 128, True, False),          # 171, 199
+    ([2048, 2048], 32, 128, 128, True, False),       # 1134, 1184
+    ([300] * 4, 16, 64, 64, True, False),            # 88, 106
+    ([1000] * 8, 16, 64, 64, True, False),           # 413, 545
+    ([300] * 16, 4, 64, 64, True, False),            # 89, 107
+    ([192, 191], 4, 64, 64, False, False),           # 47, 69
+    ([191], 4, 64, 64, False, False), ([2048], 16, 256, 64, True, False), ([], 16, 64, 64, True, False),
+])
+def test_chunks_are_taken_where_they_are_faster(lens, H, D, V, gated, chunked, monkeypatch):
+    from nanospec_b200 import ops
+    monkeypatch.setattr(ops, "sm_count", lambda: 148)
+    assert ops.chunks_pay(lens, H, D, V, gated) == chunked
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("others,chunked", [([], True), ([1], True), ([190], False), ([300] * 7, False)])
+def test_a_long_request_beside_others(others, chunked, gated, monkeypatch):
+    """The rule as it stands, on both its sides: a request's numbers depend on its neighbours by the roundings of its sums alone (the walk and the
+    chunks each within the bound of `test_chunked_recurrence` of the recurrence in 64 bits)."""
+    from nanospec_b200 import ops
+    from nanospec_b200.parts import Workspace
+    H, G, D, V = 16, 8 if gated else 16, 128, 128
+    lens = [300, *others]
+    names, call = [], ops.lib.call
+    monkeypatch.setattr(ops.lib, "call", lambda name, *a: (names.append(name), call(name, *a)))
+    rec, decay, state = _operands(lens, H, G, D, V, gated, len(others))
+    want, after = _walk(rec[:300], decay, state, [300], [1], H, G, D, V, gated)
+    S, out = state.clone(), torch.empty(sum(lens), H * V, device=DEV)
+    ops.linear_mix(rec, S, _context(lens, [i + 1 for i in range(len(lens))], Workspace(DEV)), out, H, G, D, V, decay=None if gated else decay, gated=gated)
+    assert ("ns_linear_chunked" in names) == chunked
+    bound = 4 * 320 ** 0.5 * 2.0 ** -24
+    assert float((out[:300].double() - want).norm() / want.norm()) < bound
+    assert float((S[1].double() - after[1]).norm() / after[1].norm()) < bound
