@@ -3,7 +3,7 @@
 // No tensor cores and no reduced-precision mode: every product and sum is an fp32 FMA.
 // Each output element is accumulated by one thread over k = 0..K-1 in ascending order, so
 // its value does not depend on M, on the tile it falls in, or on what else is in the batch
-// (the three kernels below give the same bits).
+// (the three kernels below give the same bits).  Rows that do not start on 16 bytes, and K that is no multiple of 4, run in the wide tiles.
 //
 // Microseconds on a B200, one 64 x 64 kernel with 4 x 4 results a thread before -> now (an FMA loop in registers reaches 72 TFLOP/s here):
 //     M x N x K         3 x 32768 x 2048   8 x 2048 x 2048   128 x 2048 x 2048   641 x 2048 x 2048   641 x 2048 x 8192   641 x 16384 x 2048
@@ -47,8 +47,7 @@ constexpr int BK = 16;
 // ---------------------------------------------------------------------------------------
 constexpr int kBM = 32, kBN = 64, kTM = 8, kTN = 4, kStages = 4, kLd = BK + 4, kTileThreads = 64;
 
-template <bool kAligned>  // rows start on 16 bytes and K is a multiple of 4
-__global__ void __launch_bounds__(kTileThreads)
+__global__ void __launch_bounds__(kTileThreads)  // rows start on 16 bytes and K is a multiple of 4
 gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int M, int N, int K,
                 int ldx, int ldw, int ldy) {
     ns_pdl_wait();  // everything below sees the previous kernel's results
@@ -66,14 +65,9 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
                 const int row = p >> 2, k = t * BK + (p & 3) * 4;
                 const bool is_x = row < kBM;
                 const int g = is_x ? m0 + row : n0 + row - kBM;
-                float* dst = st + row * kLd + (p & 3) * 4;
-                if (kAligned) {
-                    const bool in = g < (is_x ? M : N) && k < K;
-                    const float* src = is_x ? x + (size_t)g * ldx + k : w + (size_t)g * ldw + k;
-                    cp_async16(dst, in ? src : w, in ? 16 : 0);
-                } else {
-                    *reinterpret_cast<float4*>(dst) = is_x ? load_k4<false>(x, g, M, ldx, k, K) : load_k4<false>(w, g, N, ldw, k, K);
-                }
+                const bool in = g < (is_x ? M : N) && k < K;
+                const float* src = is_x ? x + (size_t)g * ldx + k : w + (size_t)g * ldw + k;
+                cp_async16(st + row * kLd + (p & 3) * 4, in ? src : w, in ? 16 : 0);
             }
         }
         cp_async_commit();
@@ -332,15 +326,17 @@ NS_API int ns_gemm_f32(const float* x, const float* w, float* y, int M, int N, i
         if (M <= 16) return launch_rows<4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
         return launch_rows<8>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
     }
-    // six and more rounds of the wide kernel's blocks, two an SM (below that its last round costs more than it wins: 641 x 3072 x 2048
-    // 236 against 233 us, 641 x 2048 x 2048 235 against 179); and more rows than the small tiles' grid can hold
+    // Wide tiles from six blocks an SM on (below that the last round costs more than it wins: 641 x 3072 x 2048
+    // 236 against 233 us, 641 x 2048 x 2048 235 against 179), with more rows than the small tiles' grid can hold, and whenever the small
+    // tiles' 16-byte copies cannot be had: their loads go through registers a tile ahead (rows of 2,049, 16 x 2048 124 us, 300 x 2048
+    // 129, 1500 x 2048 314; small tiles filled by plain loads 190, 261, 632).
     const dim3 wide((N + kWideN - 1) / kWideN, (M + kWideM - 1) / kWideM), small((N + kBN - 1) / kBN, (M + kBM - 1) / kBM);
-    if ((long long)wide.x * wide.y >= 6 * kSMs || small.y > 65535) {
+    const bool pieces = aligned && K % 4 == 0;
+    if (!pieces || (long long)wide.x * wide.y >= 6 * kSMs || small.y > 65535) {
         if (aligned) NS_LAUNCH((gemm_f32_wide_kernel<true>), wide, kWideThreads, 0, stream, x, w, y, M, N, K, ldx, ldw, ldy);
         else NS_LAUNCH((gemm_f32_wide_kernel<false>), wide, kWideThreads, 0, stream, x, w, y, M, N, K, ldx, ldw, ldy);
     } else {
-        if (aligned && K % 4 == 0) NS_LAUNCH((gemm_f32_kernel<true>), small, kTileThreads, 0, stream, x, w, y, M, N, K, ldx, ldw, ldy);
-        else NS_LAUNCH((gemm_f32_kernel<false>), small, kTileThreads, 0, stream, x, w, y, M, N, K, ldx, ldw, ldy);
+        NS_LAUNCH(gemm_f32_kernel, small, kTileThreads, 0, stream, x, w, y, M, N, K, ldx, ldw, ldy);
     }
     NS_CHECK_LAUNCH("ns_gemm_f32");
     return NS_OK;
