@@ -112,7 +112,7 @@ chunk_states_kernel(const float* __restrict__ B, const float* __restrict__ x, co
 }
 
 // grid (requests, elements of the state / (256 * VEC)); states[slot] becomes the state before the chunk
-template <int VEC>
+template <int VEC, bool AHEAD>
 __global__ void __launch_bounds__(256)
 chunk_pass_kernel(float* __restrict__ states, const float* __restrict__ decays, float* __restrict__ state, long long state_floats,
                   const int* __restrict__ qo_indptr, const int* __restrict__ state_slot, int min_len, int H, int per_head) {
@@ -140,38 +140,65 @@ chunk_pass_kernel(float* __restrict__ states, const float* __restrict__ decays, 
     float S[VEC];
 #pragma unroll
     for (int k = 0; k < VEC; ++k) S[k] = S_mem[k];
-    // Four chunks' loads are in flight while the four before are passed on: what bounds this is the latency of a chain of loads (three prompts of
-    // 2,471 tokens in all, 64 heads of 128 x 64: 67 us with the loads and the sums of four chunks in turn, 33 so).
-    float add[2][4][VEC], d[2][4];
-    auto fetch = [&](int c0, int st) {
+    // AHEAD: four chunks' loads are in flight while the four before are passed on.  What bounds this is the latency of a chain of loads (three prompts
+    // of 2,471 tokens in all, 64 heads of 128 x 64: 67 us with the loads and the sums of four chunks in turn, 33 so); short prompts of few
+    // heads have no chain, and the wider kernel leaves the next one's blocks less room (96 tokens, 32 heads, the whole step: 45 us in turn, 52 ahead).
+    if constexpr (AHEAD) {
+        float add[2][4][VEC], d[2][4];
+        auto fetch = [&](int c0, int st) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (c0 + u < chunks) {
-                d[st][u] = dec[(size_t)(c0 + u) * H];
-                if constexpr (VEC == 4) {
-                    const float4 v = ld4(at + (size_t)(c0 + u) * total);
-                    add[st][u][0] = v.x; add[st][u][1] = v.y; add[st][u][2] = v.z; add[st][u][3] = v.w;
-                } else {
-                    add[st][u][0] = at[(size_t)(c0 + u) * total];
+            for (int u = 0; u < 4; ++u)
+                if (c0 + u < chunks) {
+                    d[st][u] = dec[(size_t)(c0 + u) * H];
+                    if constexpr (VEC == 4) {
+                        const float4 v = ld4(at + (size_t)(c0 + u) * total);
+                        add[st][u][0] = v.x; add[st][u][1] = v.y; add[st][u][2] = v.z; add[st][u][3] = v.w;
+                    } else {
+                        add[st][u][0] = at[(size_t)(c0 + u) * total];
+                    }
                 }
-            }
-    };
-    auto pass = [&](int c0, int st) {
+        };
+        auto pass = [&](int c0, int st) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (c0 + u < chunks) {
-                if constexpr (VEC == 4) *reinterpret_cast<float4*>(at + (size_t)(c0 + u) * total) = make_float4(S[0], S[1], S[2], S[3]);
-                else at[(size_t)(c0 + u) * total] = S[0];
+            for (int u = 0; u < 4; ++u)
+                if (c0 + u < chunks) {
+                    if constexpr (VEC == 4) *reinterpret_cast<float4*>(at + (size_t)(c0 + u) * total) = make_float4(S[0], S[1], S[2], S[3]);
+                    else at[(size_t)(c0 + u) * total] = S[0];
 #pragma unroll
-                for (int k = 0; k < VEC; ++k) S[k] = fmaf(d[st][u], S[k], add[st][u][k]);
-            }
-    };
-    fetch(0, 0);
-    for (int c0 = 0; c0 < chunks; c0 += 8) {
-        fetch(c0 + 4, 1);
-        pass(c0, 0);
-        fetch(c0 + 8, 0);
-        pass(c0 + 4, 1);
+                    for (int k = 0; k < VEC; ++k) S[k] = fmaf(d[st][u], S[k], add[st][u][k]);
+                }
+        };
+        fetch(0, 0);
+        for (int c0 = 0; c0 < chunks; c0 += 8) {
+            fetch(c0 + 4, 1);
+            pass(c0, 0);
+            fetch(c0 + 8, 0);
+            pass(c0 + 4, 1);
+        }
+    } else {
+        for (int c0 = 0; c0 < chunks; c0 += 4) {  // four chunks' loads are in flight together
+            float add[4][VEC], d[4];
+            const int cnt = min(4, chunks - c0);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (u < cnt) {
+                    d[u] = dec[(size_t)(c0 + u) * H];
+                    if constexpr (VEC == 4) {
+                        const float4 v = ld4(at + (size_t)(c0 + u) * total);
+                        add[u][0] = v.x; add[u][1] = v.y; add[u][2] = v.z; add[u][3] = v.w;
+                    } else {
+                        add[u][0] = at[(size_t)(c0 + u) * total];
+                    }
+                }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (u < cnt) {
+                    if constexpr (VEC == 4) *reinterpret_cast<float4*>(at + (size_t)(c0 + u) * total) = make_float4(S[0], S[1], S[2], S[3]);
+                    else at[(size_t)(c0 + u) * total] = S[0];
+#pragma unroll
+                    for (int k = 0; k < VEC; ++k) S[k] = fmaf(d[u], S[k], add[u][k]);
+                }
+        }
     }
 #pragma unroll
     for (int k = 0; k < VEC; ++k) S_mem[k] = S[k];
@@ -509,17 +536,19 @@ int launch_outputs4(const float* C, const float* B, const float* x, const float*
 // C, B, x, step: the columns of the preparation's rows (row stride ld floats; groups of C and B Np apart, heads of x V, one step size
 // per head); a_log [H]; state [slots, state_floats] with S [H, N, V] at the start of a row; states: scratch for `chunks` chunks of
 // H * N * V floats, decays: H floats each, where `chunks` is at least the number of chunks of all requests of min_len tokens or more.
-// Requests of fewer tokens are not touched.
+// Requests of fewer tokens are not touched.  Four heads go to a block, where they can, once that makes more than
+// `four_from` blocks.
 NS_API int ns_ssm_chunked(const float* C, const float* B, const float* x, const float* step, int ld, const float* a_log, float* state,
                           long long state_floats, const int* qo_indptr, const int* state_slot, float* out, int ld_out, int n_requests,
-                          int min_len, int chunks, float* states, float* decays, int H, int G, int N, int Np, int V, cudaStream_t stream) {
+                          int min_len, int chunks, float* states, float* decays, int H, int G, int N, int Np, int V, int four_from, cudaStream_t stream) {
     if (n_requests <= 0 || chunks <= 0) return NS_OK;
     if (G < 1 || H % G || N < 1 || V < 1 || Np < N) NS_FAIL(NS_ERR_ARGUMENT, "ns_ssm_chunked: %d heads in %d groups, state %d (%d), features %d", H, G, N, Np, V);
     if (ld % 4 || Np % 4 || (((uintptr_t)C | (uintptr_t)B | (uintptr_t)x | (uintptr_t)states) % 16) || (V % 4 == 0 && (uintptr_t)out % 16))
         NS_FAIL(NS_ERR_ARGUMENT, "ns_ssm_chunked: rows must start on 16 bytes");
     const int n_tiles = (N + 63) / 64, v_tiles = (V + 63) / 64;
     if (H > 65535 || n_tiles * v_tiles > 65535) NS_FAIL(NS_ERR_UNSUPPORTED, "ns_ssm_chunked: %d heads, state of %d x %d exceed the grid", H, N, V);
-    const bool four = V == 64 && (N == 64 || N == 128) && Np == N && (H / G) % kHeads == 0 && ld_out % 4 == 0;
+    const bool many = (long long)chunks * H > (long long)four_from * kHeads;
+    const bool four = many && V == 64 && (N == 64 || N == 128) && Np == N && (H / G) % kHeads == 0 && ld_out % 4 == 0;
 #define NS_SSM_FOUR(F, ...) (N == 128 ? F<128>(__VA_ARGS__) : F<64>(__VA_ARGS__))
     if (four) {
         const int rc = NS_SSM_FOUR(launch_states4, B, x, step, ld, a_log, qo_indptr, n_requests, min_len, chunks, states, decays, H, G, stream);
@@ -533,12 +562,12 @@ NS_API int ns_ssm_chunked(const float* C, const float* B, const float* x, const 
     const bool vec = (N * V) % 4 == 0 && state_floats % 4 == 0 && (uintptr_t)state % 16 == 0;
     const long long blocks = (total + 256 * (vec ? 4 : 1) - 1) / (256 * (vec ? 4 : 1));
     if (blocks > 65535) NS_FAIL(NS_ERR_UNSUPPORTED, "ns_ssm_chunked: a state of %lld floats exceeds the grid", total);
-    if (vec)
-        NS_LAUNCH((chunk_pass_kernel<4>), dim3(n_requests, (unsigned)blocks), 256, 0, stream, states, decays, state, state_floats, qo_indptr, state_slot,
-                  min_len, H, N * V);
-    else
-        NS_LAUNCH((chunk_pass_kernel<1>), dim3(n_requests, (unsigned)blocks), 256, 0, stream, states, decays, state, state_floats, qo_indptr, state_slot,
-                  min_len, H, N * V);
+#define NS_SSM_PASS(VC, AH)                                                                                                                \
+    NS_LAUNCH((chunk_pass_kernel<VC, AH>), dim3(n_requests, (unsigned)blocks), 256, 0, stream, states, decays, state, state_floats, qo_indptr, \
+              state_slot, min_len, H, N * V)
+    if (vec) { if (many) NS_SSM_PASS(4, true); else NS_SSM_PASS(4, false); }
+    else { if (many) NS_SSM_PASS(1, true); else NS_SSM_PASS(1, false); }
+#undef NS_SSM_PASS
     NS_CHECK_LAUNCH("ns_ssm_chunked");
     if (four)
         return NS_SSM_FOUR(launch_outputs4, C, B, x, step, ld, a_log, qo_indptr, n_requests, min_len, chunks, states, out, ld_out, H, G, stream);

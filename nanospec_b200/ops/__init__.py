@@ -1138,6 +1138,10 @@ def ssm_padded_dim(state_dim: int) -> int:
 SSM_CHUNK = 64           # tokens of a chunk in csrc/ssm_chunked.cu
 # requests of at least so many tokens in a step go a chunk at a time, shorter ones (and decoding) a token at a time
 SSM_CHUNKED_MIN = 96
+# Blocks of four heads above which the chunks take them (None: as many as there are SMs); below, one head to a block has four times as many in
+# flight (states of 64 x 128, a head to a block against four: 64 heads, 500 tokens, 128 blocks of four 77 us / 94, 1,000 tokens, 256 blocks
+# 143 / 107; 128 heads, 300 tokens, 160 blocks 114 / 97; 32 heads, 96 tokens, 16 blocks 45 / 78)
+SSM_FOUR_HEADS_FROM: int | None = None
 SSM_SCRATCH_MAX = 1 << 31  # bytes of chunk states; a step that would need more walks token by token
 
 
@@ -1168,7 +1172,8 @@ def ssm_scan(rec: torch.Tensor, a_log: torch.Tensor, state: torch.Tensor, ctx, o
     base = rec.data_ptr()
     lib.call("ns_ssm_chunked", base, base + 4 * groups * dp, base + 4 * off_x, base + 4 * (off_x + heads * v_dim + heads), rec.stride(0),
              a_log.data_ptr(), state.data_ptr(), state.stride(0), ctx.qo_indptr.data_ptr(), ctx.state_slot.data_ptr(), out.data_ptr(), out.stride(0),
-             ctx.n_requests, least, chunks, states.data_ptr(), decays.data_ptr(), heads, groups, state_dim, dp, v_dim, _stream())
+             ctx.n_requests, least, chunks, states.data_ptr(), decays.data_ptr(), heads, groups, state_dim, dp, v_dim,
+             sm_count() if SSM_FOUR_HEADS_FROM is None else SSM_FOUR_HEADS_FROM, _stream())
     return out
 
 

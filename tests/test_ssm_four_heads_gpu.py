@@ -13,8 +13,9 @@ DEV = torch.device("cuda")
 
 @pytest.mark.parametrize("N", [64, 128])
 @pytest.mark.parametrize("lens,H,G", [([96], 4, 1), ([97, 3, 191], 8, 2), ([128, 65, 160], 12, 1), ([511], 16, 4), ([577, 1153], 4, 1)])
-def test_four_heads_to_a_block(lens, H, G, N):
+def test_four_heads_to_a_block(lens, H, G, N, monkeypatch):
     from nanospec_b200 import ops
+    monkeypatch.setattr(ops, "SSM_FOUR_HEADS_FROM", 0)  # also where they are too few to be worth it
     from nanospec_b200.parts import Workspace
     V = 64
     g = torch.Generator(device=DEV).manual_seed(sum(lens) + H + N)
@@ -42,3 +43,31 @@ def test_four_heads_to_a_block(lens, H, G, N):
         assert torch.equal(out[:, h * V: (h + 1) * V], o1), h
         assert torch.equal(S[:, h * N * V: (h + 1) * N * V], S1), h
     assert bool((out[:, H * V:] == 7.0).all())
+
+
+@pytest.mark.parametrize("tokens,heads,blocks", [(96, 32, 16), (500, 64, 128), (300, 128, 160)])
+def test_both_sides_of_the_rule_give_the_same_bits(tokens, heads, blocks, monkeypatch):
+    """A step below and above the number of SMs in blocks of four heads, as the rule has it and with the other choice."""
+    from nanospec_b200 import ops
+    from nanospec_b200.parts import Workspace
+    assert -(-tokens // 64) * heads // 4 == blocks
+    N, V, G = 64, 64, 8
+    g = torch.Generator(device=DEV).manual_seed(tokens)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    off = 2 * G * N + heads * V
+    rec, a_log, step = rnd(tokens, off + 2 * heads + G), 0.5 * rnd(heads), torch.nn.functional.softplus(rnd(tokens, heads))
+    rec[:, off: off + heads], rec[:, off + heads: off + 2 * heads] = torch.exp(-torch.exp(a_log) * step), step
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    ws, state = Workspace(DEV), 0.3 * rnd(2, heads * N * V)
+    ctx = SimpleNamespace(n_requests=1, extras={}, q_lens=[tokens], max_q_len=tokens, state_slot=i32([1]), qo_indptr=i32([0, tokens]),
+                          buffer=lambda name, cols, dtype, rows: ws.get(name, rows, cols, dtype))
+    seen, call = [], ops.lib.call
+    monkeypatch.setattr(ops.lib, "call", lambda name, *a: (seen.append((name, a[-2])), call(name, *a)))
+    outs = []
+    for least in (None, 0, 1 << 20):
+        monkeypatch.setattr(ops, "SSM_FOUR_HEADS_FROM", least)
+        S, out = state.clone(), torch.empty(tokens, heads * V, device=DEV)
+        ops.ssm_scan(rec, a_log, S, ctx, out, heads, G, N, V)
+        outs.append((out, S))
+    assert seen == [("ns_ssm_chunked", ops.sm_count()), ("ns_ssm_chunked", 0), ("ns_ssm_chunked", 1 << 20)]
+    assert all(torch.equal(a, b) for other in outs[1:] for a, b in zip(outs[0], other))
