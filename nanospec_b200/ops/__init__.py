@@ -535,6 +535,22 @@ def attention_generic(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     return out
 
 
+F32_TILES: bool | None = None  # None: by the rule below (measurements and tests set it)
+
+
+def f32_tiles_pay(ctx, nq: int, dim: int) -> bool:
+    """Whether a float32 step's portions take csrc/attention_f32.cu: us of the exact kernel (a warp's chain over its keys, or all pairs of rows and
+    keys) against those of a block's chain over groups of 32 keys (one request, 32 heads of 64 over 8: a prompt of 2 tokens 6.2 us against 13.4,
+    of 40 23.4 / 23.0, of 300 434 / 87; 2 tokens behind 1,500 488 / 312; 4 heads of 32 over 1, a prompt of 128 26 / 33; of 450 such points the
+    rule takes a kernel slower by more than 5 % at 27, by 4 us in the mean of all but one).  The bits are the same."""
+    if F32_TILES is not None:
+        return F32_TILES
+    prompts = _prompts(ctx)
+    keys = prompts["keys"]
+    by_row = max(2 + keys * (0.08 + 0.0032 * dim), 6e-6 * dim * nq * prompts["pairs"])
+    return by_row > 6 + 0.04 * dim + -(-keys // 32) * (5.5 + 0.01 * dim)
+
+
 def _attention_f32_tiles(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, nkv: int, head_dim: int, scale: float, v_dim: int,
                          softcap: float, sink: torch.Tensor | None, gate: torch.Tensor | None, feature_gate: bool, out_scale: float,
                          tiles: torch.Tensor) -> None:
@@ -767,6 +783,18 @@ def _attention_plan(ctx) -> dict:
     return plan
 
 
+def _prompts(ctx) -> dict:
+    """Once per step, of the requests that bring more than one token: the most keys that a row sees, and what all rows see together."""
+    found = ctx.extras.get("attention_prompts")
+    if found is None:
+        sizes = [(n, kv) for n, kv in zip(ctx.q_lens, ctx.kv_lens) if n > 1]
+        found = ctx.extras["attention_prompts"] = {
+            "keys": max((kv for _, kv in sizes), default=0),
+            "pairs": sum(n * (2 * kv - n + 1) // 2 for n, kv in sizes),
+        }
+    return found
+
+
 def attention(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, nkv: int, head_dim: int, scale: float,
               window: int = 0, keep_first: int = 0, v_dim: int | None = None, wide_weights: bool = False, chunk: int = 0,
               softcap: float = 0.0, sink: torch.Tensor | None = None, gate: torch.Tensor | None = None, feature_gate: bool = False,
@@ -795,7 +823,8 @@ def attention(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, nkv: int
         plan = getattr(ctx, "extras", {}).get("attention_plan") if qkv.dtype == torch.float32 else None  # (the step's own, if it has one)
         if plan is not None and plan["tiles"] is not None and not window and not chunk and nq % nkv == 0 and nq // nkv <= 32 \
                 and lane.k.dtype == lane.v.dtype == out.dtype == qkv.dtype and all(n % 4 == 0 and 4 <= n <= 256 for n in (head_dim, v_dim)) \
-                and qkv.stride(1) == 1 and out.stride(1) == 1 and lane.k.data_ptr() % 16 == 0 and lane.v.data_ptr() % 16 == 0:
+                and qkv.stride(1) == 1 and out.stride(1) == 1 and lane.k.data_ptr() % 16 == 0 and lane.v.data_ptr() % 16 == 0 \
+                and f32_tiles_pay(ctx, nq, max(head_dim, v_dim)):
             _attention_f32_tiles(qkv, lane, ctx, out, nq, nkv, head_dim, scale, v_dim, softcap, sink, gate, feature_gate, out_scale,
                                  plan["tiles"])
             if not plan["n_decode"]:

@@ -44,7 +44,7 @@ def test_gemm_f32_kernels_give_the_same_bits(M, N, K):
 @pytest.mark.parametrize("nq,nkv,d,dv,page", [(4, 4, 32, 32, 8), (8, 2, 64, 64, 16), (24, 8, 128, 128, 16), (32, 1, 20, 20, 8), (5, 1, 36, 100, 16),
                                              (6, 2, 256, 8, 8), (2, 1, 4, 256, 16), (66, 2, 16, 16, 8)])  # (the last: 33 heads to a kv head, the exact kernel's)
 @pytest.mark.parametrize("options", ["plain", "sink", "gate", "features"])
-def test_attention_f32_portions_give_the_exact_kernels_bits(nq, nkv, d, dv, page, options):
+def test_attention_f32_portions_give_the_exact_kernels_bits(nq, nkv, d, dv, page, options, monkeypatch):
     """Portions of unlike lengths on unlike contexts beside decode tokens through `ops.attention`, against the one-warp kernel over the
     same rows, bit for bit (that kernel is tested against plain attention); pages that nobody wrote hold NaN."""
     from nanospec_b200 import ops
@@ -70,6 +70,7 @@ def test_attention_f32_portions_give_the_exact_kernels_bits(nq, nkv, d, dv, page
     qkv = torch.randn(N, nq * d + 8, generator=g, device=DEV)
     extra = {"sink": dict(sink=torch.randn(nq, generator=g, device=DEV)), "gate": dict(gate=torch.randn(N, nq, generator=g, device=DEV)),
              "features": dict(gate=torch.randn(N, nq * dv, generator=g, device=DEV), feature_gate=True, out_scale=0.5, softcap=2.0)}.get(options, {})
+    monkeypatch.setattr(ops, "F32_TILES", True)  # also where so few rows do not take them
     got, want = torch.empty(N, nq * dv, device=DEV), torch.empty(N, nq * dv, device=DEV)
     ops.attention(qkv, lane, ctx, got, nq, nkv, d, 0.3, v_dim=dv, **extra)
     ops.attention_generic(qkv, lane.k, lane.v, lane.block_table, ctx.token_req, ctx.positions, want, nq, nkv, d, page, 0.3, v_dim=dv, **extra)
