@@ -720,6 +720,20 @@ def attention_decode(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, n
 PREFILL_TWO_HEADS = "auto"  # "always" / "never": tests run both kernels whatever the size of the grid
 
 
+def many_short_portions(ctx, blocks: int, head_dim: int, two_heads: bool, sms: int) -> bool:
+    """Whether a step's portions fill so little of the tiles of the tcgen05 kernel's `blocks` (256 rows, a block an SM) that the m16n8k16 kernel, which holds
+    several blocks of 128 rows an SM, is faster: more blocks than SMs, heads of 64, on average at most 64 rows a request - 128 where they see
+    no more than 128 keys -, and with two heads to a block no more than 128 keys (us on m16n8k16 / tcgen05, a window of 1,024, wide weights: 64
+    prompts of 2 tokens, 8 heads over 8 11.2 / 19.9, 32 over 8 37 / 45; 32 portions of 60 behind 100, 8 over 8 13.1 / 14.8, 32 over 8 48 / 41;
+    32 prompts of 120, 8 over 8 12.0 / 13.1; 32 portions of 120 behind 100 19.8 / 17.4)."""
+    if head_dim != 64 or blocks <= sms or getattr(ctx, "kv_lens", None) is None:
+        return False
+    prompts = _prompts(ctx)
+    requests = max(1, prompts["requests"])
+    rows, keys = prompts["rows"] / requests, prompts["held"] / requests
+    return (rows <= 64 and (keys <= 128 or not two_heads)) or (rows <= 128 and keys <= 128 and not two_heads)
+
+
 def attention_prefill(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, nkv: int, head_dim: int, scale: float,
                       window: int, tiles: torch.Tensor, tiles_tc: torch.Tensor | None = None, keep_first: int = 0,
                       wide_weights: bool = False, chunk: int = 0, softcap: float = 0.0, v_dim: int | None = None,
@@ -737,13 +751,15 @@ def attention_prefill(qkv: torch.Tensor, lane, ctx, out: torch.Tensor, nq: int, 
         # unit busier and the keys are read once for both) - once one head to a block would give more blocks than SMs
         two_heads = head_dim == 64 and (nq // nkv) % 2 == 0 and PREFILL_TWO_HEADS != "never" and (
             PREFILL_TWO_HEADS == "always" or nq * tiles_tc.shape[0] > sm_count())
-        lib.call("ns_attention_prefill_tc", qkv.data_ptr(), qkv.stride(0), qkv.shape[0], lane.k.data_ptr(),
-                 lane.v.data_ptr(), lane.k.shape[0], lane.block_table.data_ptr(), lane.block_table.stride(0),
-                 ctx.positions.data_ptr(), ctx.qo_indptr.data_ptr(), tiles_tc.data_ptr(), tiles_tc.shape[0], out.data_ptr(),
-                 out.stride(0), nq, nkv, head_dim, lane.page_size, float(scale), 2 if two_heads else 1,
-                 _tc(qkv.device).error.data_ptr(), int(window), int(keep_first) if window else 0, int(chunk), int(bool(wide_weights)),
-                 _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0, int(bool(feature_gate)), float(out_scale), _stream())
-        return
+        general = window or chunk or wide_weights or sink is not None or gate is not None or out_scale != 1.0
+        if not general or not many_short_portions(ctx, tiles_tc.shape[0] * (nq // 2 if two_heads else nq), head_dim, two_heads, sm_count()):
+            lib.call("ns_attention_prefill_tc", qkv.data_ptr(), qkv.stride(0), qkv.shape[0], lane.k.data_ptr(),
+                     lane.v.data_ptr(), lane.k.shape[0], lane.block_table.data_ptr(), lane.block_table.stride(0),
+                     ctx.positions.data_ptr(), ctx.qo_indptr.data_ptr(), tiles_tc.data_ptr(), tiles_tc.shape[0], out.data_ptr(),
+                     out.stride(0), nq, nkv, head_dim, lane.page_size, float(scale), 2 if two_heads else 1,
+                     _tc(qkv.device).error.data_ptr(), int(window), int(keep_first) if window else 0, int(chunk), int(bool(wide_weights)),
+                     _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0, int(bool(feature_gate)), float(out_scale), _stream())
+            return
     lib.call("ns_attention_prefill_kept", qkv.data_ptr(), qkv.stride(0), lane.k.data_ptr(), lane.v.data_ptr(),
              lane.block_table.data_ptr(), lane.block_table.stride(0), ctx.positions.data_ptr(), ctx.qo_indptr.data_ptr(),
              tiles.data_ptr(), tiles.shape[0], out.data_ptr(), out.stride(0), nq, nkv, head_dim, lane.page_size,
@@ -784,13 +800,15 @@ def _attention_plan(ctx) -> dict:
 
 
 def _prompts(ctx) -> dict:
-    """Once per step, of the requests that bring more than one token: the most keys that a row sees, and what all rows see together."""
+    """Once per step, of the requests that bring more than one token: the most keys that a row sees, what all rows see together, requests,
+    rows, and the positions that they hold after the step."""
     found = ctx.extras.get("attention_prompts")
     if found is None:
         sizes = [(n, kv) for n, kv in zip(ctx.q_lens, ctx.kv_lens) if n > 1]
         found = ctx.extras["attention_prompts"] = {
             "keys": max((kv for _, kv in sizes), default=0),
             "pairs": sum(n * (2 * kv - n + 1) // 2 for n, kv in sizes),
+            "requests": len(sizes), "rows": sum(n for n, _ in sizes), "held": sum(kv for _, kv in sizes),
         }
     return found
 

@@ -28,3 +28,52 @@ def _step(held, brings):
 def test_float32_portions(held, brings, nq, dim, tiles):
     from nanospec_b200 import ops
     assert ops.f32_tiles_pay(_step(held, brings), nq, dim) == tiles
+
+
+@pytest.mark.parametrize("held,brings,nq,two,m16", [
+    ([0] * 64, [2] * 64, 8, False, True),            # 11.2 on m16n8k16, 19.9 on tcgen05
+    ([0] * 64, [2] * 64, 32, True, True),            # 37.3, 45.1
+    ([100] * 32, [60] * 32, 8, False, True),         # 13.1, 14.8
+    ([0] * 32, [120] * 32, 8, False, True),          # 12.0, 13.1
+    ([100] * 32, [60] * 32, 32, True, False),        # 47.8, 40.6
+    ([100] * 32, [120] * 32, 8, False, False),       # 19.8, 17.4
+    ([1000] * 16, [2] * 16, 32, True, False),        # 75.6, 55.2
+    ([0] * 16, [2] * 16, 8, False, False),           # 5.9, 5.8: a block an SM
+    ([0] * 16, [180] * 16, 32, True, False),         # 43.0, 26.7
+    ([1000] * 16, [1] * 16, 32, True, False),        # nothing but decoding
+])
+def test_prefill_of_many_short_portions(held, brings, nq, two, m16):
+    from nanospec_b200 import ops
+    ctx, blocks = _step(held, brings), sum(-(-n // 256) for n in brings if n > 1) * (nq // 2 if two else nq)
+    assert ops.many_short_portions(ctx, blocks, 64, two, 148) == m16
+    assert not ops.many_short_portions(ctx, blocks, 128, two, 148)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nq,nkv,brings,entry", [(8, 8, 24, "ns_attention_prefill_kept"), (16, 2, 24, "ns_attention_prefill_kept"),
+                                                 (8, 8, 200, "ns_attention_prefill_tc")])
+def test_prefill_of_many_requests(nq, nkv, brings, entry, monkeypatch):
+    """Windowed prompts of 24 requests through `ops.attention` on both sides of the rule; the two kernels agree to the roundings of the weights
+    (16 bits) and of the output (2^-9 of itself)."""
+    from nanospec_b200 import ops
+    from nanospec_b200.engine import ModelRunner, StepEntry
+    from nanospec_b200.parts import CacheNeed
+    from test_parts_gpu import _Shell
+    d, B = 64, 24
+    runner = ModelRunner(_Shell(torch.bfloat16, [(CacheNeed(nkv, d, 0, 0, None), None)], 1024), B * (brings // 16 + 1), 16, B)
+    for r in range(B):
+        runner.begin(r)
+    ctx, _, _ = runner.build_context([StepEntry(r, [1] * brings) for r in range(B)])
+    lane, g = ctx.lanes[0], torch.Generator(device="cuda").manual_seed(nq)
+    for store in (lane.k, lane.v):
+        store.copy_(torch.randn(store.shape, generator=g, device="cuda"))
+    qkv = torch.randn(B * brings, nq * d, generator=g, device="cuda").to(torch.bfloat16)
+    names, call, outs = [], ops.lib.call, []
+    monkeypatch.setattr(ops.lib, "call", lambda name, *a: (names.append(name), call(name, *a)))
+    for rule in (ops.many_short_portions, lambda *a: entry == "ns_attention_prefill_tc"):  # the rule, and the other kernel
+        monkeypatch.setattr(ops, "many_short_portions", rule)
+        outs.append(torch.zeros(B * brings, nq * d, device="cuda", dtype=torch.bfloat16))
+        ops.attention(qkv, lane, ctx, outs[-1], nq, nkv, d, d ** -0.5, window=100, keep_first=3, wide_weights=True)
+    ops.check_kernel_errors()
+    assert names[0] == entry and names[0] != names[1]
+    assert float((outs[0].double() - outs[1].double()).norm() / outs[1].double().norm()) < 2.0 ** -8
