@@ -1407,8 +1407,14 @@ def attention_latent(q_lat: torch.Tensor, q_rot: torch.Tensor, lane, ctx, out: t
 
 
 # Requests of at least so many tokens in a step run on keys and values unfolded from the latents: the products that unfold them cost
-# 2 * rank * 256 operations a position and head, the folded form costs 2 * (2 * rank + r - 320) more a query, key and head.
+# 2 * rank * 256 operations a position and head, the folded form costs 2 * (2 * rank + r - 320) more a query, key and head, on the older tensor
+# path (a layer of 16 heads, rank 512, folded / unfolded us: a prompt of 64 tokens 39 / 56, of 128 40 / 37, of 256 53 / 45; 128 behind 2,000
+# 124 / 71, behind 32,000 1,369 / 607; behind 32,000 under a window of 1,024 79 / 54; rank 128, a prompt of 128 31 / 32).
 LATENT_UNFOLD_MIN = 128
+# Beside shorter requests, whose folded products run over every row of the step, only where the long ones' folded attention is at least so many
+# operations (16 heads, rank 512: 130 tokens behind 500 beside 8 that decode, 2.5e9, 66 / 90 us; 256 behind 8,000 under a window of 1,024
+# beside one, 9.1e9, 119 / 117; 512 behind 2,000 so, 18e9, 214 / 135; rank 256 without rotation, 4.3e9, 82 / 109).
+LATENT_UNFOLD_MIXED = 9e9
 LATENT_UNFOLD_MAX = 1 << 30  # bytes of unfolded keys and values; a step that would need more runs folded
 
 
@@ -1424,7 +1430,14 @@ def latent_unfold_rows(ctx, lane, heads: int, dim: int, rot_dim: int, v_dim: int
             rows += -(-kv // 64) * 64 - first // 64 * 64
     if rows * heads * 512 > LATENT_UNFOLD_MAX or _attention_plan(ctx).get("tiles_tc") is None:
         return 0, False
-    return rows, min(ctx.q_lens) >= LATENT_UNFOLD_MIN
+    all_long = min(ctx.q_lens) >= LATENT_UNFOLD_MIN
+    return (rows, all_long) if all_long or _latent_folded_ops(ctx, heads, rot_dim, rank, window) >= LATENT_UNFOLD_MIXED else (0, False)
+
+
+def _latent_folded_ops(ctx, heads: int, rot_dim: int, rank: int, window: int) -> float:
+    """Operations of the folded attention of the step's long requests."""
+    pairs = sum(n * min(kv - n // 2, window or kv) for n, kv in zip(ctx.q_lens, ctx.kv_lens) if n >= LATENT_UNFOLD_MIN)
+    return 2.0 * (2 * rank + rot_dim) * heads * pairs
 
 
 def attention_latent_unfolded(q: torch.Tensor, lane, ctx, out: torch.Tensor, w_uk: torch.Tensor, w_uv: torch.Tensor, rows: int, rot_dim: int, scale: float,

@@ -49,6 +49,25 @@ def test_prefill_of_many_short_portions(held, brings, nq, two, m16):
     assert not ops.many_short_portions(ctx, blocks, 128, two, 148)
 
 
+@pytest.mark.parametrize("held,brings,heads,rank,rot,window,unfolded", [
+    # folded, unfolded
+    ([500] + [300] * 8, [130] + [1] * 8, 16, 512, 64, 0, False),      # 65.6, 90.1
+    ([8000, 500], [256, 1], 16, 256, 0, 1024, False),                 # 81.9, 109.0
+    ([2000, 500], [512, 1], 16, 256, 0, 1024, False),                 # 122, 129
+    ([2000, 500], [512, 1], 16, 512, 64, 1024, True),                 # 214, 135
+    ([500] + [300] * 8, [130] + [1] * 8, 128, 512, 64, 0, True),      # 311, 199
+    ([0, 500], [1500, 1], 16, 128, 64, 0, True),                      # 220, 123
+    ([500], [130], 16, 512, 64, 0, True),                             # alone: 65, 46
+    ([0], [127], 16, 512, 64, 0, False),
+])
+def test_latents_of_long_portions(held, brings, heads, rank, rot, window, unfolded):
+    from nanospec_b200 import ops
+    ctx = _step(held, brings)
+    lane = SimpleNamespace(k=torch.empty(0, dtype=torch.bfloat16))
+    rows, all_long = ops.latent_unfold_rows(ctx, lane, heads, 128, rot, 128, rank, window, torch.bfloat16, 0.1)
+    assert (rows > 0) == unfolded and all_long == (unfolded and min(brings) >= 128)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("nq,nkv,brings,entry", [(8, 8, 24, "ns_attention_prefill_kept"), (16, 2, 24, "ns_attention_prefill_kept"),
                                                  (8, 8, 200, "ns_attention_prefill_tc")])
