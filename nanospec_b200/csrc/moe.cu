@@ -36,15 +36,71 @@ __global__ void cast_f32_kernel(const T* __restrict__ x, long long ldx, float* _
 
 constexpr int kMaxExperts = 1024;
 
-// logits[n, e] = x[n] . w[e] (+ bias[e]) in float: a block takes TOK tokens (their rows in shared memory) and eight warps of EPW experts each,
-// so a row of w is read once for TOK tokens and a piece of x once for EPW experts.  The sum over a row runs in the same order whatever
-// TOK and EPW are.
-template <typename T, int TOK, int EPW>
+// logits[n, e] = x[n] . w[e] (+ bias[e]) in float: a block takes TOK tokens (their rows in shared memory) and eight experts, a warp per expert,
+// so a row of w is read once for TOK tokens.  The sum over a row runs in the same order whatever TOK is, here and below.
+template <typename T, int TOK>
 __global__ void __launch_bounds__(256)
 router_logits_kernel(const T* __restrict__ x, long long ldx, const float* __restrict__ w, const float* __restrict__ bias,
                      float* __restrict__ logits, int n_tokens, int E, int K) {
     ns_pdl_launch_dependents();
     ns_pdl_wait();
+    extern __shared__ __align__(16) float xrow[];  // [TOK][K4]
+    const int K4 = (K + 3) / 4 * 4;
+    const int n0 = blockIdx.x * TOK, lane = threadIdx.x & 31, e = blockIdx.y * 8 + (threadIdx.x >> 5);
+    const int cnt = min(TOK, n_tokens - n0);
+    const bool vec = K % 8 == 0 && ldx % 8 == 0 && (((uintptr_t)w | (uintptr_t)x) % 16 == 0);
+    if (vec) {
+        const int per_row = K / 8;
+        for (int i = threadIdx.x; i < TOK * per_row; i += blockDim.x) {
+            const int t = i / per_row, k = (i - t * per_row) * 8;
+            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (t < cnt) ld8(x + (size_t)(n0 + t) * ldx + k, v);
+            st8(xrow + (size_t)t * K4 + k, v);
+        }
+    } else {
+        for (int i = threadIdx.x; i < TOK * K; i += blockDim.x) {
+            const int t = i / K, k = i - t * K;
+            xrow[(size_t)t * K4 + k] = t < cnt ? ns_ld(x, (size_t)(n0 + t) * ldx + k) : 0.f;
+        }
+    }
+    __syncthreads();
+    if (e >= E) return;
+    const float* wr = w + (size_t)e * K;
+    float a[TOK];
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) a[t] = 0.f;
+    if (vec) {
+#pragma unroll 4
+        for (int k = lane * 4; k < K; k += 128) {
+            const float4 v = *reinterpret_cast<const float4*>(wr + k);
+#pragma unroll
+            for (int t = 0; t < TOK; ++t) {
+                const float4 u = *reinterpret_cast<const float4*>(xrow + (size_t)t * K4 + k);
+                a[t] = fmaf(v.x, u.x, a[t]); a[t] = fmaf(v.y, u.y, a[t]); a[t] = fmaf(v.z, u.z, a[t]); a[t] = fmaf(v.w, u.w, a[t]);
+            }
+        }
+    } else {
+        for (int k = lane; k < K; k += 32) {
+            const float v = wr[k];
+#pragma unroll
+            for (int t = 0; t < TOK; ++t) a[t] = fmaf(v, xrow[(size_t)t * K4 + k], a[t]);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < TOK; ++t) {
+        const float v = ns_warp_sum(a[t]) + (bias ? bias[e] : 0.f);
+        if (lane == 0 && t < cnt) logits[(size_t)(n0 + t) * E + e] = v;
+    }
+}
+
+// The same with eight tokens to a block and EPW experts to a warp, so that a piece of x is read once for EPW experts.
+template <typename T, int EPW>
+__global__ void __launch_bounds__(256)
+router_logits_wide_kernel(const T* __restrict__ x, long long ldx, const float* __restrict__ w, const float* __restrict__ bias,
+                     float* __restrict__ logits, int n_tokens, int E, int K) {
+    ns_pdl_launch_dependents();
+    ns_pdl_wait();
+    constexpr int TOK = 8;
     extern __shared__ __align__(16) float xrow[];  // [TOK][K4]
     const int K4 = (K + 3) / 4 * 4;
     const int n0 = blockIdx.x * TOK, lane = threadIdx.x & 31, e0 = (blockIdx.y * 8 + (threadIdx.x >> 5)) * EPW;
@@ -75,7 +131,7 @@ router_logits_kernel(const T* __restrict__ x, long long ldx, const float* __rest
 #pragma unroll
         for (int t = 0; t < TOK; ++t) a[i][t] = 0.f;
     if (vec) {
-#pragma unroll(EPW == 1 ? 4 : 2)
+#pragma unroll 2
         for (int k = lane * 4; k < K; k += 128) {
             float4 v[EPW];
 #pragma unroll
@@ -502,7 +558,7 @@ NS_API int ns_cast_f32(const void* x, long long ldx, float* out, int n_rows, int
 
 // x [n, K] (row stride ldx) in the compute type, w [E, K] and bias [E] (or null) float, logits [n, E] float
 NS_API int ns_router_logits(const void* x, long long ldx, const float* w, const float* bias, float* logits, int n_tokens, int E, int K, int dtype,
-                            cudaStream_t stream) {
+                            int n_sms, cudaStream_t stream) {
     if (n_tokens <= 0) return NS_OK;
     const size_t row = (size_t)(K + 3) / 4 * 4 * sizeof(float);
     if (row > 200 * 1024) NS_FAIL(NS_ERR_UNSUPPORTED, "ns_router_logits: a row of %d floats does not fit shared memory", K);
@@ -511,20 +567,26 @@ NS_API int ns_router_logits(const void* x, long long ldx, const float* w, const 
     int tok = n_tokens <= 32 ? 1 : n_tokens <= 128 ? 2 : n_tokens <= 512 ? 4 : 8;
     while (tok > 1 && tok * row > 100 * 1024) tok /= 2;
     const size_t smem = tok * row;
-    // experts to a warp: one while tokens alone give few blocks; in long steps as many as leave one or two groups of eight warps (2,048 tokens of
-    // 2,048 features, 36 experts: 38 us with one, 18 with five)
-    const int epw = tok < 8 ? 1 : E <= 8 ? 1 : E <= 16 ? 2 : E > 32 && E <= 40 ? 5 : 4;
-    const dim3 grid((n_tokens + tok - 1) / tok, (E + 8 * epw - 1) / (8 * epw));
-#define NS_ROUTER(T, TK, EP)                                                                                                          \
-    {                                                                                                                                 \
-        if (smem > 48 * 1024) NS_CUDA(cudaFuncSetAttribute(router_logits_kernel<T, TK, EP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); \
-        NS_LAUNCH((router_logits_kernel<T, TK, EP>), grid, 256, smem, stream, (const T*)x, ldx, w, bias, logits, n_tokens, E, K);     \
+    // Experts to a warp: one in short steps; in long ones the most, up to five, that leave a block for every SM and no more than a fifth of the warps'
+    // places empty (us with one and with the rule's: 2,048 tokens of 2,048 features 36 experts 38 / 18 (5), 64 57 / 26 (4), 100 84 / 43; 513 tokens of
+    // 3,072 features, 32 experts, which five or four would give 65 blocks, 13).
+    int epw = 1;
+    for (int w = 2; w <= 5 && tok == 8; ++w) {
+        const int groups = (E + 8 * w - 1) / (8 * w);
+        if (groups * ((n_tokens + tok - 1) / tok) >= n_sms && groups * 8 * w * 4 <= E * 5) epw = w;
     }
-#define NS_ROUTER_T(T)                                                                                                  \
-    {                                                                                                                   \
-        if (tok == 1) NS_ROUTER(T, 1, 1) else if (tok == 2) NS_ROUTER(T, 2, 1) else if (tok == 4) NS_ROUTER(T, 4, 1)    \
-        else if (epw == 1) NS_ROUTER(T, 8, 1) else if (epw == 2) NS_ROUTER(T, 8, 2) else if (epw == 4) NS_ROUTER(T, 8, 4) \
-        else NS_ROUTER(T, 8, 5)                                                                                         \
+    const dim3 grid((n_tokens + tok - 1) / tok, (E + 8 * epw - 1) / (8 * epw));
+#define NS_ROUTER(T, ...)                                                                                                             \
+    {                                                                                                                                 \
+        if (smem > 48 * 1024) NS_CUDA(cudaFuncSetAttribute((__VA_ARGS__), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));    \
+        NS_LAUNCH((__VA_ARGS__), grid, 256, smem, stream, (const T*)x, ldx, w, bias, logits, n_tokens, E, K);                         \
+    }
+#define NS_ROUTER_T(T)                                                                                                                \
+    {                                                                                                                                 \
+        if (tok == 1) NS_ROUTER(T, router_logits_kernel<T, 1>) else if (tok == 2) NS_ROUTER(T, router_logits_kernel<T, 2>)            \
+        else if (tok == 4) NS_ROUTER(T, router_logits_kernel<T, 4>) else if (epw == 1) NS_ROUTER(T, router_logits_kernel<T, 8>)       \
+        else if (epw == 2) NS_ROUTER(T, router_logits_wide_kernel<T, 2>) else if (epw == 3) NS_ROUTER(T, router_logits_wide_kernel<T, 3>) \
+        else if (epw == 4) NS_ROUTER(T, router_logits_wide_kernel<T, 4>) else NS_ROUTER(T, router_logits_wide_kernel<T, 5>)           \
     }
     if (dtype == NS_F32) NS_ROUTER_T(float)
     else NS_ROUTER_T(__nv_bfloat16)

@@ -1512,7 +1512,7 @@ def router_logits(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, scratch=N
     if bias is not None and (bias.dtype != torch.float32 or bias.numel() != E or not bias.is_contiguous()):
         raise KernelError("router_logits: one contiguous float32 bias per output")
     if n * E * K <= ROUTER_DIRECT_MAX or n <= 64:
-        lib.call("ns_router_logits", x.data_ptr(), x.stride(0), w.data_ptr(), _ptr(bias), out.data_ptr(), n, E, K, dtype_code(x.dtype), _stream())
+        lib.call("ns_router_logits", x.data_ptr(), x.stride(0), w.data_ptr(), _ptr(bias), out.data_ptr(), n, E, K, dtype_code(x.dtype), sm_count(), _stream())
         return out
     x32 = x if x.dtype == torch.float32 else cast_f32(x, scratch(n, K))
     linear(x32, w, out)

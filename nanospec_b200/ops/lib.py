@@ -80,7 +80,7 @@ _SIGNATURES: dict[str, list] = {
     "ns_latent_gather": [_P, _P, _I, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P],
     "ns_attention_latent_flat": [_P, _I, _I, _P, _P, _P, _I, _I, _I, _P, _P, _I, _I, _P, _I, _P, _I, _I, _I, _F, _I, _P, _P, _I, _P, _P],
     "ns_cast_f32": [_P, _L, _P, _I, _I, _I, _P],
-    "ns_router_logits": [_P, _L, _P, _P, _P, _I, _I, _I, _I, _P],
+    "ns_router_logits": [_P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "ns_moe_route": [_P, _I, _I, _I, _I, _I, _F, _I, _P, _I, _P, _P, _P],
     "ns_moe_route_plan": [_P, _I, _I, _I, _I, _I, _F, _I, _P, _I, _P, _P, _I, _P, _P, _P, _P],
     "ns_moe_plan": [_P, _I, _I, _P, _P, _P, _P],

@@ -869,7 +869,8 @@ def test_command_line(tmp_path):
     assert (tmp_path / "o" / "0.f32").stat().st_size == 4 * full_config()["vocab"]
 
 
-@pytest.mark.parametrize("n,E", [(513, 5), (600, 16), (515, 33), (520, 40), (514, 41), (1000, 70)])  # the experts to a warp, and remainders of them
+@pytest.mark.parametrize("n,E", [(513, 5), (600, 16), (515, 33), (520, 40), (514, 41), (1000, 70),
+                                 (1190, 16), (1190, 24), (1190, 31), (1190, 33), (1190, 41), (1190, 70)])  # 1 to 5 experts to a warp, and remainders of them
 def test_router_of_long_steps(n, E):
     """Long steps give a warp several experts; the sums keep their order: the bits of the same rows in short steps."""
     from nanospec_b200 import ops
