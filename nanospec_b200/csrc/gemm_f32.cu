@@ -310,17 +310,16 @@ int launch_rows(const float* x, const float* w, float* y, int M, int N, int K, i
 
 }  // namespace
 
-// x: [M, K] with row stride ldx; w: [N, K] with row stride ldw; y: [M, N] with row stride ldy.
+// x: [M, K] with row stride ldx; w: [N, K] with row stride ldw; y: [M, N] with row stride ldy; n_sms: multiprocessors of the device.
 NS_API int ns_gemm_f32(const float* x, const float* w, float* y, int M, int N, int K, int ldx, int ldw, int ldy,
-                       cudaStream_t stream) {
+                       int n_sms, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return NS_OK;
     if (K <= 0) NS_FAIL(NS_ERR_ARGUMENT, "ns_gemm_f32: K=%d", K);
     if ((M + 63) / 64 > 65535) NS_FAIL(NS_ERR_UNSUPPORTED, "ns_gemm_f32: M=%d exceeds 65535 row tiles", M);
-    constexpr int kSMs = 148;
     const bool aligned = (ldx % 4 == 0) && (ldw % 4 == 0) && (((uintptr_t)x | (uintptr_t)w) % 16 == 0);
     // up to 16 rows, and up to 32 where the columns alone would not give every SM a tile (32 x 2048 x 8192: 169 us against about 280 in
     // tiles; 32 x 16384 x 2048: 133 against about 75)
-    if (aligned && K % 4 == 0 && (M <= 16 || (M <= 32 && N <= kBN * kSMs))) {
+    if (aligned && K % 4 == 0 && (M <= 16 || (M <= 32 && N <= (long long)kBN * n_sms))) {
         if (M <= 4) return launch_rows<1>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
         if (M <= 8) return launch_rows<2>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
         if (M <= 16) return launch_rows<4>(x, w, y, M, N, K, ldx, ldw, ldy, stream);
@@ -332,7 +331,7 @@ NS_API int ns_gemm_f32(const float* x, const float* w, float* y, int M, int N, i
     // 129, 1500 x 2048 314; small tiles filled by plain loads 190, 261, 632).
     const dim3 wide((N + kWideN - 1) / kWideN, (M + kWideM - 1) / kWideM), small((N + kBN - 1) / kBN, (M + kBM - 1) / kBM);
     const bool pieces = aligned && K % 4 == 0;
-    if (!pieces || (long long)wide.x * wide.y >= 6 * kSMs || small.y > 65535) {
+    if (!pieces || (long long)wide.x * wide.y >= 6LL * n_sms || small.y > 65535) {
         if (aligned) NS_LAUNCH((gemm_f32_wide_kernel<true>), wide, kWideThreads, 0, stream, x, w, y, M, N, K, ldx, ldw, ldy);
         else NS_LAUNCH((gemm_f32_wide_kernel<false>), wide, kWideThreads, 0, stream, x, w, y, M, N, K, ldx, ldw, ldy);
     } else {

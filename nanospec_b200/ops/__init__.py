@@ -411,7 +411,7 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, sink: NormSink | None = None):
         if x.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
             raise KernelError("linear: operands must be row-major")
         lib.call("ns_gemm_f32", x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), w.stride(0),
-                 out.stride(0), _stream())
+                 out.stride(0), sm_count(), _stream())
         return out
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise KernelError(f"linear: unsupported operand types {x.dtype}, {w.dtype}")
