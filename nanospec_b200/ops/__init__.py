@@ -539,15 +539,16 @@ F32_TILES: bool | None = None  # None: by the rule below (measurements and tests
 
 
 def f32_tiles_pay(ctx, nq: int, dim: int) -> bool:
-    """Whether a float32 step's portions take csrc/attention_f32.cu: us of the exact kernel (a warp's chain over its keys, or all pairs of rows and
-    keys) against those of a block's chain over groups of 32 keys (one request, 32 heads of 64 over 8: a prompt of 2 tokens 6.2 us against 13.4,
-    of 40 23.4 / 23.0, of 300 434 / 87; 2 tokens behind 1,500 488 / 312; 4 heads of 32 over 1, a prompt of 128 26 / 33; of 450 such points the
-    rule takes a kernel slower by more than 5 % at 27, by 4 us in the mean of all but one).  The bits are the same."""
+    """Whether a float32 step's portions take csrc/attention_f32.cu: us of the exact kernel (a warp's chain over its keys, and all pairs of rows and
+    keys) against those of a block's chain over groups of 32 keys (exact kernel, tiles; one request, 32 heads of 64 over 8: a prompt of 2 tokens 6.2
+    and 13.4, of 40 23.4 and 23.0, of 300 434 and 87; 2 tokens behind 1,500 488 and 312; 4 heads of 32 over 1, a prompt of 128 26 and 33).
+    Of 512 steps and layers the rule takes a kernel slower by more than 5 % at 10, by 5 us in the mean.  The bits are the same."""
     if F32_TILES is not None:
         return F32_TILES
     prompts = _prompts(ctx)
     keys = prompts["keys"]
-    by_row = max(2 + keys * (0.08 + 0.0032 * dim), 6e-6 * dim * nq * prompts["pairs"])
+    chain, pairs = 2 + keys * (0.08 + 0.0032 * dim), 6e-6 * dim * nq * prompts["pairs"]
+    by_row = (chain ** 1.5 + pairs ** 1.5) ** (2 / 3)  # (the longer of the two alone misses 47 of them, by up to 22 us)
     return by_row > 6 + 0.04 * dim + -(-keys // 32) * (5.5 + 0.01 * dim)
 
 

@@ -23,6 +23,8 @@ def _step(held, brings):
     ([0], [300], 4, 64, True),                       # 121, 72
     ([1500], [2], 32, 64, True),                     # 488, 312
     ([200] * 8, [60] * 8, 4, 32, True),              # 100, 63
+    ([0], [97], 16, 64, True),                       # 51, 30: the chain and the pairs take alike, neither hides the other
+    ([0] * 4, [40] * 4, 16, 64, True),               # 45, 22
     ([1500, 900], [2, 1], 8, 128, True),             # a request that brings one token does not count
 ])
 def test_float32_portions(held, brings, nq, dim, tiles):
