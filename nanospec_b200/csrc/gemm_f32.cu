@@ -1,4 +1,5 @@
-// True 32-bit matrix product on the CUDA cores: y[M, N] = x[M, K] * w[N, K]^T.
+// True 32-bit matrix product on the CUDA cores: y[M, N] = x[M, K] * w[N, K]^T.  Products of K below 1,024, and those whose w TMA cannot
+// address; the others run in gemm_f32_tc.cu.
 //
 // No tensor cores and no reduced-precision mode: every product and sum is an fp32 FMA.
 // Each output element is accumulated by one thread over k = 0..K-1 in ascending order, so

@@ -159,6 +159,13 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
           "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -222,7 +229,7 @@ inline NsEncodeTiledFn ns_encode_fn() {
     return fn;
 }
 
-// rows x cols bf16 matrix with row stride ld (elements); boxes of box_rows x 64 columns, 128-byte
+// rows x cols matrix of bfloat16 or float with row stride ld (elements); boxes of box_rows x 128 bytes, 128-byte
 // swizzle, zero fill outside the matrix.  A map depends on the address, the sizes and the box only, never on the
 // contents, and weights and scratch buffers keep their addresses from step to step: every map is encoded once and
 // kept (per host thread and per source file that asks; the table is emptied when it reaches 8,192 entries), so
@@ -245,8 +252,9 @@ struct NsMapKeyHash {
     }
 };
 
-inline int ns_make_map_bf16(CUtensorMap* map, const void* ptr, unsigned long long rows, int cols, long long ld,
-                            int box_rows, const char* who) {
+template <int kBytes>  // of an element: 2 (bfloat16) or 4 (float)
+inline int ns_make_map(CUtensorMap* map, const void* ptr, unsigned long long rows, int cols, long long ld, int box_rows, const char* who) {
+    static_assert(kBytes == 2 || kBytes == 4, "bfloat16 or float");
     static thread_local std::unordered_map<NsMapKey, CUtensorMap, NsMapKeyHash> known;
     const NsMapKey key{ptr, rows, ld, cols, box_rows};
     const auto hit = known.find(key);
@@ -259,16 +267,19 @@ inline int ns_make_map_bf16(CUtensorMap* map, const void* ptr, unsigned long lon
     // the kernels address rows with signed 32-bit TMA coordinates
     if (rows > 0x7fffffffull) NS_FAIL(NS_ERR_UNSUPPORTED, "%s: a tensor of %llu rows is beyond the 2^31 - 1 that a TMA coordinate holds", who, rows);
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * kBytes};
+    const cuuint32_t box[2] = {128u / kBytes, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    const CUresult r = fn(map, kBytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(ptr), dims,
+                          strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) NS_FAIL(NS_ERR_CUDA, "%s: cuTensorMapEncodeTiled failed with code %d", who, (int)r);
     if (known.size() >= 8192) known.clear();
     known.emplace(key, *map);
     return NS_OK;
+}
+inline int ns_make_map_bf16(CUtensorMap* map, const void* ptr, unsigned long long rows, int cols, long long ld, int box_rows, const char* who) {
+    return ns_make_map<2>(map, ptr, rows, cols, ld, box_rows, who);
 }
 
 }  // namespace

@@ -176,6 +176,12 @@ USE_TENSOR_CORE_GEMM = True  # the hand-written tcgen05 kernel; False hands ever
 TENSOR_CORE_GEMM_MAX_TOKENS: int | None = 64
 
 
+# float32 products of at least this K go to the tcgen05 kernel on parts (csrc/gemm_f32_tc.cu).  The rule looks at w alone, so that a row's
+# bits do not depend on the rows beside it: below this K many rows would gain (300 x 4096 x 512: 47 -> 17 us), but a few lose to the kernel that
+# takes x apart (8 x 1024 x 512: 7.0 -> 10.1); from here on both gain (1 x 1024 x 1024: 11.8 -> 11.2).
+F32_TC_MIN_K = 1024
+
+
 def _tc(device: torch.device) -> _TensorCoreGemmState:
     st = _tc_state.get(device)
     if st is None:
@@ -201,6 +207,9 @@ def check_kernel_errors(device: torch.device | None = None) -> None:
                     11: "prefill attention: the loader waited for a free stage", 12: "prefill attention: the MMA issuer waited",
                     13: "prefill attention: a softmax warp waited", 21: "decode attention: the loader waited for a free stage",
                     22: "decode attention: a warp waited for its keys",
+                    51: "float32 product: the TMA producer waited for a free stage", 52: "float32 product: the MMA issuer waited",
+                    53: "float32 product: the parts of w waited", 54: "float32 product: the parts of x waited",
+                    55: "float32 product: the sums waited for the accumulator", 56: "float32 product: copies in flight did not land",
                     41: "routed experts: the TMA producer waited for a free stage", 42: "routed experts: the MMA issuer waited for a tile",
                     43: "routed experts: the epilogue waited for the accumulator", 44: "routed experts: copies in flight did not land",
                     31: "wait probe: nobody arrives at its barrier"}.get(code, "?")
@@ -238,6 +247,39 @@ def gemm_splits(M: int, N: int, K: int) -> int:
         # after all (continuous batching at that shape: 13,290 against 13,200 output tokens / s)
         splits = splits_with(4)
     return splits
+
+
+def f32_tiles(M: int, N: int, K: int, sms: int) -> tuple[int, int]:
+    """(rows of x to a tile, blocks that share a tile's k) of the float32 product on the tensor cores.  A block of 64 k of a tile takes about
+    (120 + rows) units of 5 ns (0.70 us with 16 rows, 1.12 with 96: taking w's tile apart is a constant part); tiles come in rounds over the SMs, and
+    where they are few, a cluster of two or four divides the groups of k that the kernel adds up in order (8 x 2048 x 8192: 91 us alone, 50, 32, and
+    38 with eight).  The bits do not depend on the choice."""
+    blocks = -(-K // 64)
+    group = -(-blocks // min(8, -(-blocks // 8)))
+    groups = -(-blocks // group)
+    best = None
+    for rows in range(16, 97, 16):
+        tiles = -(-N // 128) * -(-M // rows)
+        for splits in (1, 2, 4):
+            held = -(-groups // splits)
+            if splits > 1 and (splits > groups or tiles * splits > sms or held * rows > 96):
+                continue
+            cost = -(-tiles // sms) * (held * group if splits > 1 else blocks) * (120 + rows) + (300 if splits > 1 else 0)
+            if best is None or cost < best[0]:
+                best = (cost, rows, splits)
+        if rows >= M:
+            break
+    return best[1:]
+
+
+def linear_f32_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tiles: tuple[int, int] | None = None) -> None:
+    """The float32 product on the tensor cores (csrc/gemm_f32_tc.cu)."""
+    M, K = x.shape
+    N = w.shape[0]
+    rows, splits = tiles or f32_tiles(M, N, K, sm_count())
+    parts = torch.empty((3, M, -(-K // 8) * 8), dtype=torch.bfloat16, device=x.device)
+    lib.call("ns_gemm_f32_tc", x.data_ptr(), w.data_ptr(), out.data_ptr(), parts.data_ptr(), M, N, K, x.stride(0), w.stride(0), out.stride(0),
+             rows, splits, sm_count(), _tc(x.device).error.data_ptr(), _stream())
 
 
 def linear_tensor_core(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, splits: int | None = None) -> bool:
@@ -379,7 +421,8 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, sink: NormSink | None = None):
     for the norm that follows is returned; otherwise `out` is returned and the caller runs the norm.  A `TanhSink` (a norm
     without statistics follows) likewise: the stream is updated and a `Normed` returned, or `out`.
 
-    float32: the CUDA-core kernel (true fp32, k-ascending sums, independent of M).
+    float32: from K = 1024 on the tensor cores on three bfloat16 parts of every float (24 bits kept, sums in blocks, closer to 64 bits than a
+    chain), below it the CUDA cores (k-ascending sums); either way independent of M.
     bfloat16: the tcgen05 kernel; operands that TMA cannot address (K or a row stride that is no
     multiple of 8) are a plain matrix product for cuBLAS, as the reference hands its `nn.Linear`
     calls to it (model/llama.py:175,184,195).  `out` may be bfloat16 or float32.
@@ -410,6 +453,9 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, sink: NormSink | None = None):
             raise KernelError("linear: a float32 product takes float32 weights and output")
         if x.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
             raise KernelError("linear: operands must be row-major")
+        if K >= F32_TC_MIN_K and K % 4 == 0 and w.stride(0) % 4 == 0 and w.data_ptr() % 16 == 0:
+            linear_f32_tc(x, w, out)
+            return out
         lib.call("ns_gemm_f32", x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, x.stride(0), w.stride(0),
                  out.stride(0), sm_count(), _stream())
         return out

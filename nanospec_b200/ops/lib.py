@@ -30,6 +30,7 @@ _SIGNATURES: dict[str, list] = {
     "ns_swiglu_rows": [_P, _L, _P, _L, _I, _I, _I, _I, _P],
     "ns_gate_mul_rows": [_P, _L, _P, _L, _I, _I, _I, _F, _F, _F, _I, _P],
     "ns_gemm_f32": [_P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
+    "ns_gemm_f32_tc": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "ns_rope_kv_write": [_P, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P],
     "ns_attention_generic": [_P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _I, _I, _F, _I, _P],
     "ns_add_layernorm": [_P, _P, _P, _P, _P, _I, _I, _F, _I, _I, _P],

@@ -1,0 +1,120 @@
+"""The float32 product on the tensor cores (csrc/gemm_f32_tc.cu) at the edges of its tiles, splits and groups."""
+
+from __future__ import annotations
+
+import random
+
+import pytest
+import torch
+
+DEV = "cuda"
+
+
+def test_f32_tiles_fit():
+    """What the kernel's entry demands of a split, over sizes spread by their logarithm."""
+    from nanospec_b200 import ops
+    rng = random.Random(5)
+    for _ in range(2000):
+        M, N, K = (int(2 ** rng.uniform(0, hi)) for hi in (14, 17, 14))
+        rows, splits = ops.f32_tiles(M, N, K, 148)
+        blocks = -(-K // 64)
+        groups = -(-blocks // -(-blocks // min(8, -(-blocks // 8))))
+        assert rows % 16 == 0 and 16 <= rows <= 96 and rows < M + 16
+        assert splits == 1 or (splits <= groups and -(-N // 128) * -(-M // rows) * splits <= 148 and -(-groups // splits) * rows <= 96)
+
+
+def _operands(M, N, K, seed, spread=0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
+    if spread:
+        x = x * torch.exp2(torch.randint(-spread, spread, (M, K), generator=g, device=DEV).float())
+    return x, w
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [1024, 1028, 1092, 4160])  # whole groups; four past a block; a ragged last block; groups of unlike lengths
+@pytest.mark.parametrize("M,N", [(1, 1), (15, 127), (16, 128), (17, 129), (33, 300), (97, 260), (130, 20000)])
+def test_f32_tc_product(M, N, K):
+    """Against 64 bits: an element's products lose 2^-25 of themselves; a block's 24 additions truncate (2^-23 of what they reach), the K / 64 sums of
+    blocks and groups round.  And no further off, in the 2-norm, than the chain of fmaf.  Every tile and split, rows alone and rows that
+    do not start on 16 bytes give the same bits; nothing beside the result is touched."""
+    from nanospec_b200 import ops
+    from nanospec_b200.ops import lib
+    x, w = _operands(M, N, K, M + N + K, spread=20 if M == 33 else 0)
+    out = torch.full((M, N + 3), 7.0, device=DEV)
+    ops.linear(x, w, out[:, :N])
+    ref, size = x.double() @ w.double().T, x.abs().double() @ w.abs().double().T
+    err = out[:, :N].double() - ref
+    assert bool((err.abs() <= size * (50 + K // 64 + 8) * 2.0 ** -24).all())
+    assert bool((out[:, N:] == 7.0).all())
+    if M * N > 1000:  # (a 2-norm of few elements is chance: here the chain's is five times as large or more)
+        chain = torch.empty(M, N, device=DEV)
+        lib.call("ns_gemm_f32", x.data_ptr(), w.data_ptr(), chain.data_ptr(), M, N, K, K, K, N, ops.sm_count(), ops._stream())
+        assert float(err.norm()) <= float((chain.double() - ref).norm())
+    got = torch.empty(M, N, device=DEV)
+    blocks = -(-K // 64)
+    groups = -(-blocks // -(-blocks // min(8, -(-blocks // 8))))
+    for rows in (16, 32, 48, 96):
+        for splits in (1, 2, 4):
+            if splits == 1 or (splits <= groups and -(-N // 128) * -(-M // rows) * splits <= ops.sm_count() and -(-groups // splits) * rows <= 96):
+                ops.linear_f32_tc(x, w, got.fill_(float("nan")), (rows, splits))
+                assert torch.equal(got, out[:, :N]), (rows, splits)
+    one = torch.empty(1, N, device=DEV)
+    for m in {0, M // 2, M - 1}:
+        ops.linear(x[m:m + 1], w, one)
+        assert torch.equal(one[0], out[m, :N])
+    wide = torch.zeros(M, K + 1, device=DEV)
+    wide[:, 1:] = x
+    ops.linear(wide[:, 1:], w, got)
+    assert torch.equal(got, out[:, :N])
+    ops.check_kernel_errors()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tiles", [(16, 1), (16, 2), (48, 1)])
+def test_f32_tc_infinities_and_ends_of_the_range(tiles):
+    """An element whose floats have no parts (an infinity, a NaN) or whose parts fall below the smallest numbers is what the floats themselves
+    give; every other element keeps its bits."""
+    from nanospec_b200 import ops
+    x, w = _operands(40, 200, 1024, 3)
+    clean = torch.empty(40, 200, device=DEV)
+    ops.linear_f32_tc(x, w, clean, tiles)
+    y = x.clone()
+    y[3, 7], y[5, 100], y[9] = float("nan"), float("inf"), 0.0
+    y[12] *= 2.0 ** -124  # parts of these are subnormal
+    y[14, 0] = 3.4e38     # rounds to an infinite bfloat16
+    v = w.clone()
+    v[:, 0] *= 2.0 ** -10
+    v[17, 5] = float("-inf")
+    got = torch.empty(40, 200, device=DEV)
+    ops.linear_f32_tc(y, v, got, tiles)
+    assert bool(got[3].isnan().all())
+    assert torch.equal(got[5, :17], torch.sign(v[:17, 100]) * float("inf"))
+    assert bool((got[9, :17] == 0).all()) and bool(got[9, 17].isnan())  # 0 * -inf
+    assert torch.equal(got[[0, 20, 39], 17], torch.sign(y[[0, 20, 39], 5]) * float("-inf"))
+    keep = [c for c in range(200) if c != 17]
+    for m in (12, 14):
+        ref, size = y[m].double() @ v.double().T, y[m].abs().double() @ v.abs().double().T
+        # a chain of 32 fmaf and five sums, or the bound above; numbers below 2^-126 are whole multiples of 2^-149
+        assert bool(((got[m].double() - ref).abs()[keep] <= size[keep] * 82 * 2.0 ** -24 + 2.0 ** -143).all())
+    same = torch.empty(40, 200, device=DEV)
+    ops.linear_f32_tc(x, v, same, tiles)
+    rows = [m for m in range(40) if m not in (3, 5, 9, 12, 14)]
+    assert torch.equal(got[rows][:, keep], same[rows][:, keep])
+    ops.check_kernel_errors()
+
+
+@pytest.mark.gpu
+def test_f32_tc_late_weights():
+    """Weights from DRAM, whose tiles land out of order: the bits of the first run again and again (odd and even rings of w's tiles)."""
+    from nanospec_b200 import ops
+    x, w = _operands(3, 32768, 2048, 1)
+    flush = torch.empty(64 << 20, device=DEV)
+    first, got = torch.empty(3, 32768, device=DEV), torch.empty(3, 32768, device=DEV)
+    for tiles in ((16, 1), (48, 1)):
+        ops.linear_f32_tc(x, w, first, tiles)
+        for _ in range(12):
+            flush.zero_()
+            ops.linear_f32_tc(x, w, got, tiles)
+            assert torch.equal(got, first)
+    ops.check_kernel_errors()
