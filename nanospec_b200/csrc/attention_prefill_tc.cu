@@ -181,7 +181,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     auto o_final = [&](int t) { return tile_bar(t, 7); };
     const uint32_t holder = bar0 + 8u * (1 + 2 * kStages + kTiles * 8);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // heads vary fastest: the host lists the tiles with the most keys first, and blocks are
     // scheduled in that order, so the long tiles do not end up alone at the tail
     const int req = tiles[2 * blockIdx.y], q_off = tiles[2 * blockIdx.y + 1];
@@ -230,6 +230,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     tc_fence_after();
     uint32_t tmem_base;
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(holder));
+    tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
     auto tmem_s = [&](int t, int b) { return tmem_base + (uint32_t)((t * 2 + b) * 64); };
     auto tmem_o = [&](int t) { return tmem_base + 256u + (uint32_t)(t * 128); };
 
@@ -523,7 +524,7 @@ attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __
     auto o_final = [&](int tt) { return tile_bar(tt, 3); };  // the P V of the tile's last block has completed
     const uint32_t holder = bar0 + 8u * (1 + 2 * kKvStages + kTiles4 * 4);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int req = tiles[2 * blockIdx.y], q_off = tiles[2 * blockIdx.y + 1];
     const int h0 = 2 * blockIdx.x;          // tiles 0, 1: head h0; tiles 2, 3: head h0 + 1 (the same kv head)
     const int hk = h0 / (nq / nkv);
@@ -566,6 +567,7 @@ attention_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __
     tc_fence_after();
     uint32_t tmem_base;
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(holder));
+    tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
     auto tmem_s = [&](int tt) { return tmem_base + (uint32_t)(tt * 64); };
     auto tmem_o = [&](int tt) { return tmem_base + 256u + (uint32_t)(tt * 64); };
 

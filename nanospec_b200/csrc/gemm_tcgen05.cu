@@ -154,7 +154,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     float* sq_s = stage_f32 + BN * BM;  // sink mode: [BN][BM + 1] squares, behind the partial tile
 
     ns_pdl_launch_dependents();  // the next kernel may be scheduled; it waits for this one before it reads
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * BM;      // first feature of the tile
     const int tok0 = blockIdx.y * BN;    // first token of the tile
     const int split = blockIdx.z;
@@ -182,6 +182,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     tc_fence_after();
     uint32_t tmem_base;
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(holder));
+    tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
 
     if (warp == 0) {
         // ---------------- TMA producer: the warp runs the loop converged, one elected lane issues ----------------

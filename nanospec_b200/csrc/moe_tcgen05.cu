@@ -48,7 +48,7 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
 
     ns_pdl_launch_dependents();
     ns_pdl_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int n0 = blockIdx.x * BM;
     if (warp == 0) {  // which expert's rows this block takes
         int before = 0, found = -1, row = 0, count = 0;
@@ -95,6 +95,7 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     tc_fence_after();
     uint32_t tmem_base;
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(holder));
+    tmem_base = __shfl_sync(0xffffffffu, tmem_base, 0);
 
     if (warp == 0) {
         int issued = 0;
