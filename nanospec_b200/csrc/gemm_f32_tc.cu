@@ -1,7 +1,6 @@
 // 32-bit matrix product on the 5th-generation tensor cores: y[M, N] = x[M, K] * w[N, K]^T, nothing rounded to less than 24 bits.
 //
-// A float is the sum of three bfloat16, each the rest of the one before rounded to nearest (8 + 8 + 8 bits), and a product of two floats is
-// kept as the six products of parts that reach 2^-24 of it (what is left out: below 2^-25).  The tensor core multiplies parts exactly and
+// Floats come apart into three bfloat16, a product of two into six products (csrc/float_parts.cuh).  The tensor core multiplies parts exactly and
 // adds them in float32, but it truncates, so its chains are kept short and small things go first: in every block of 64 k the five
 // products with a middle or a low part, then the four steps of high by high, into an accumulator that starts at zero; the block's sum
 // then joins its group's sum in registers, rounded to nearest, and the groups (eight at most, of at least 512 k, by K alone) are added in their order.
@@ -36,12 +35,12 @@
 // so that taking apart, multiplying and adding up do not wait for one another.
 #include <cfloat>
 
+#include "float_parts.cuh"
 #include "tcgen05_utils.cuh"
 
 namespace {
 
 constexpr int kBM = 128, kBK = 64, kMaxBN = 96;
-constexpr int kParts = 3;
 constexpr int kRingBytes = kBM * kBK * 4;        // a stage of floats of w: two boxes of 128 rows x 32 floats
 constexpr int kMaxRing = 6, kMaxStages = 4;      // stages of w's ring and of the parts at most
 constexpr int kSmemMax = 227 * 1024;
@@ -51,17 +50,6 @@ constexpr uint32_t kPartsCols = kParts * kBK / 2;
 constexpr float kTiny = 8.077935669463161e-28f;  // 2^-90
 
 enum F32TcError { kErrF32Loader = 51, kErrF32Mma = 52, kErrF32Weights = 53, kErrF32Rows = 54, kErrF32Sum = 55, kErrF32Drain = 56 };
-
-// a pair of floats as three pairs of bfloat16 (the first number in the low half)
-__device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    hi = *reinterpret_cast<uint32_t*>(&h);
-    const float ra = a - __uint_as_float(hi << 16), rb = b - __uint_as_float(hi & 0xffff0000u);
-    __nv_bfloat162 m = __floats2bfloat162_rn(ra, rb);
-    mid = *reinterpret_cast<uint32_t*>(&m);
-    __nv_bfloat162 l = __floats2bfloat162_rn(ra - __uint_as_float(mid << 16), rb - __uint_as_float(mid & 0xffff0000u));
-    lo = *reinterpret_cast<uint32_t*>(&l);
-}
 
 // an element from the floats themselves (every lane gets it); apart from the kernel's code, whose registers are counted
 __device__ __noinline__ float warp_dot(const float* __restrict__ x, const float* __restrict__ w, int K) {

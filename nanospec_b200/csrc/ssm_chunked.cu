@@ -8,15 +8,20 @@
 //     chunk_states   the sum over a chunk (a product over its tokens), every chunk and head at once, and the chunk's decay exp(L_end)
 //     chunk_pass     the chunks of a request in order, element by element of the state: S_in of every chunk, and the request's state
 //     chunk_outputs  y of a chunk: C B^T masked and weighted, times x, plus C S_in scaled
-// Everything is float (the same operands as the token walk's: csrc/recurrent.cu), L and its differences double, so that a difference of
-// two large sums keeps its digits.  A request's chunks start at its first token of the step; requests of fewer than min_len
+// Everything is float (the same operands as the token walk's: csrc/recurrent.cu), L and its differences double (or two floats), so that a
+// difference of two large sums keeps its digits.  A request's chunks start at its first token of the step; requests of fewer than min_len
 // tokens are left to the token walk.  Blocks find their (request, chunk) from the step's token offsets on the device.
+#include <type_traits>
+
 #include "chunks.cuh"
+#include "float_parts.cuh"
+#include "mma_utils.cuh"
 
 namespace {
 
 constexpr int kThreads = 128;  // 8 x 16 threads on a 64 x 64 tile, 8 x 4 results each
 constexpr int kLd = 68;        // floats of a staged row: 16-byte aligned, rows in different banks
+constexpr int kHeads = 4;      // of a group to a block on the tensor cores
 
 // running sums of l over the chunk (double) and the step sizes, by one warp, two tokens to a lane; tokens beyond the chunk have step 0
 __device__ __forceinline__ void chunk_logs(const float* __restrict__ step, int ld, int start, int count, float a, double* L, float* dt) {
@@ -306,12 +311,12 @@ chunk_outputs_kernel(const float* __restrict__ C, const float* __restrict__ B, c
 }
 
 // ---------------------------------------------------------------------------------------
-// The same two kernels for heads of 64 features in groups of a multiple of four and states of 64 or 128 rows: a block takes four heads of a
-// group, so that B, and C and the scores C B^T, are staged and made once for them, and threads of 8 x 8 results (16 words of shared memory to 64
-// FMAs; 12 to 32 above).  The same sums in the same order, bit for bit.  Prompts of 2,471 tokens in all, 64 heads of 64, a state of 128 rows, 8
-// groups: sums 103 us above, 80 here; read-out 242 above, 190 here.
+// The sums for heads of 64 features in groups of a multiple of four and states of 64 or 128 rows: a block takes four heads of a
+// group, so that B is staged once for them, and threads of 8 x 8 results (16 words of shared memory to 64 FMAs; 12 to 32 above).  The same
+// sums in the same order, bit for bit.  Prompts of 2,471 tokens in all, 64 heads of 64, a state of 128 rows, 8 groups: 103 us above, 80 here.
+// Not on the tensor cores (66 us): a head that forgets soon has sums of a few large terms, which a chain rounds to 5.5e-8 and truncation to 7e-8.
 // ---------------------------------------------------------------------------------------
-constexpr int kHeads = 4, kLd4 = 68;
+constexpr int kLd4 = 68;
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 16 : 0) : "memory");
@@ -397,25 +402,120 @@ chunk_states4_kernel(const float* __restrict__ B, const float* __restrict__ x, c
     }
 }
 
-// grid (chunk slots, H / 4), 256 threads, two warps to a head: the first tokens 0 .. 31, the second 32 .. 63
-template <int N>
-__global__ void __launch_bounds__(256, 2)
-chunk_outputs4_kernel(const float* __restrict__ C, const float* __restrict__ B, const float* __restrict__ x, const float* __restrict__ step,
-                      int ld, const float* __restrict__ a_log, const int* __restrict__ qo_indptr, int n_requests, int min_len,
-                      const float* __restrict__ states, float* __restrict__ out, int ld_out, int H, int G) {
+// ---------------------------------------------------------------------------------------
+// The read-out for heads of 64 features with states of 64 or 128 rows on the tensor cores (m16n8k16), every float as three bfloat16 parts
+// (csrc/float_parts.cuh).  What the tensor core truncates stays small: the five products with a middle or a low part have an accumulator of their
+// own, the four steps of high by high of 64 k another that starts at zero, and the two and the blocks of 64 k are added rounded to nearest.
+// What several heads of a group or several warps read (B, C, the weights of x) lies as parts in shared memory; x and the state go from
+// memory into the fragments of the one warp that multiplies them, a warp's columns of v dealt to its tiles in turn, so that a thread's
+// are neighbours.  A block takes four heads of a group where that still makes blocks enough, or one: the same sums, bit for bit.
+// Read-out of prompts of 2,471 tokens in all, 64 heads, a state of 128 rows: 191 us as FMAs, 123 here; 700 tokens, 8 heads: 31.6 / 12.0.  Error of y
+// against 64 bits 2.1e-7 / 1.2e-7.  Of a block's 44,000 cycles 18,000 are products (m16n8k16 at 8.2 cycles a sub-partition), 9,000 the weights of x,
+// 15,000 the way to the first product; one block an SM, whose two groups of warps overlap the first two.
+// ---------------------------------------------------------------------------------------
+constexpr int kPadQ = 8;             // bfloat16 behind a staged row: ldmatrix reads eight rows from different banks
+constexpr int kLdM = kQ + kPadQ;
+
+// A double as the sum of two floats, and the difference of two such numbers rounded to a float: within 2^-24 (1 + 2^-20) of it, as the
+// difference of the doubles rounded (what double arithmetic costs here: 12,400 of a block's 50,000 cycles).
+__device__ __forceinline__ float2 two_floats(double v) {
+    const float hi = (float)v;
+    return make_float2(hi, isfinite(hi) ? (float)(v - (double)hi) : 0.f);
+}
+__device__ __forceinline__ float difference(float2 a, float2 b) {
+    const float d = a.x - b.x, t = d - a.x, rest = (a.x - (d - t)) - (b.x + t);  // d + rest = a.x - b.x exactly
+    return d + (rest + (a.y - b.y));
+}
+
+// three parts of a staged tile: dst[part][r][c] of src[r * ld + c], zeros from `rows` on; by 128 threads
+template <int COLS>
+__device__ __forceinline__ void stage_parts(__nv_bfloat16* dst, const float* __restrict__ src, int ld, int rows) {
+    constexpr int kLdP = COLS + kPadQ, kEach = kQ * COLS / 4 / 128, kBatch = kEach < 16 ? kEach : 16;
+    const int id = threadIdx.x & 127;
+#pragma unroll 1
+    for (int i0 = 0; i0 < kEach; i0 += kBatch) {  // (a batch of reads in flight)
+        float4 v[kBatch];
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j) {
+            const int i = id + (i0 + j) * 128, r = i / (COLS / 4), c = (i % (COLS / 4)) * 4;
+            v[j] = r < rows ? ld4(src + (size_t)r * ld + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j) {
+            const int i = id + (i0 + j) * 128, r = i / (COLS / 4), c = (i % (COLS / 4)) * 4;
+            uint32_t p[kParts][2];
+            split_pair(v[j].x, v[j].y, p[0][0], p[1][0], p[2][0]);
+            split_pair(v[j].z, v[j].w, p[0][1], p[1][1], p[2][1]);
+#pragma unroll
+            for (int q = 0; q < kParts; ++q) *reinterpret_cast<uint2*>(dst + (q * kQ + r) * kLdP + c) = make_uint2(p[q][0], p[q][1]);
+        }
+    }
+}
+
+// sums of 64 k: main takes high by high, rest the five small products
+template <int MT, int NT>
+struct PartSums {
+    float main[MT][NT][4], rest[MT][NT][4];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) main[i][j][e] = rest[i][j][e] = 0.f;
+    }
+    // row tiles I0 .. MT - 1 of A (three parts each) by all column tiles of B; neighbouring products have sums of their own
+    template <int I0>
+    __device__ __forceinline__ void add(const uint32_t (&a)[MT][kParts][4], const uint32_t (&b)[kParts][NT][2]) {
+        constexpr int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+        for (int p = 0; p < 6; ++p)
+#pragma unroll
+            for (int i = I0; i < MT; ++i)
+#pragma unroll
+                for (int j = 0; j < NT; ++j) ns_mma_bf16(p < 5 ? rest[i][j] : main[i][j], a[i][pa[p]], b[pb[p]][j][0], b[pb[p]][j][1]);
+    }
+};
+
+// two column tiles of B from rows k = 2 q, 2 q + 1, 2 q + 8, 2 q + 9 (q = lane % 4) of a thread's two neighbouring columns
+__device__ __forceinline__ void column_parts(const float2 (&v)[4], uint32_t (&b)[kParts][2][2]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        split_pair(v[2 * h].x, v[2 * h + 1].x, b[0][0][h], b[1][0][h], b[2][0][h]);
+        split_pair(v[2 * h].y, v[2 * h + 1].y, b[0][1][h], b[1][1][h], b[2][1][h]);
+    }
+}
+
+// grid (chunk slots, H / HEADS): four warps to a head (64 tokens x 16 features each), HEADS / 2 heads one after the other to each of two such
+// groups (one to one).  The next head's state and x come by cp.async while this one's products run: what a warp can keep in flight in
+// registers is 2.4 TB/s over the GPU.
+constexpr int kLdSc = kQ + 2;
+template <int N, int HEADS>
+struct OutputsTc {
+    static constexpr int kGroups = HEADS == 1 ? 1 : 2, kThreads = kGroups * 128, kLdB = N + kPadQ;
+    static constexpr int kPartsB = kParts * kQ * kLdB, kPartsM = kParts * kQ * kLdM;                       // bfloat16
+    static constexpr int kShared = kPartsB > kGroups * kPartsM ? kPartsB : kGroups * kPartsM;              // B's place, then the weights'
+    static constexpr int kState = N * kLd, kX = kQ * kLd;                                                  // floats of a group's staged state and x
+    static constexpr int kSmem = 2 * (kPartsB + kShared) + 4 * (kQ * kLdSc + kGroups * (kState + kX));
+    static_assert(kSmem + HEADS * kQ * 12 + 64 <= 227 * 1024, "shared memory");
+};
+
+template <int N, int HEADS>
+__global__ void __launch_bounds__(OutputsTc<N, HEADS>::kThreads, 1)
+chunk_outputs_tc_kernel(const float* __restrict__ C, const float* __restrict__ B, const float* __restrict__ x, const float* __restrict__ step,
+                        int ld, const float* __restrict__ a_log, const int* __restrict__ qo_indptr, int n_requests, int min_len,
+                        const float* __restrict__ states, float* __restrict__ out, int ld_out, int H, int G) {
+    using O = OutputsTc<N, HEADS>;
     ns_pdl_wait();
-    constexpr int kRows = 16;  // rows of the state to a slice
-    constexpr int kSlices = 2 * kHeads * kRows * kLd4, kCt = N * kLd4;
-    extern __shared__ __align__(16) float outputs_smem[];
-    float* Sc = outputs_smem;       // the scores, [s][t]
-    float* Ct = Sc + kQ * kLd4;     // C transposed, [k][t]
-    float* slices = Ct + kCt;       // first B transposed, [k][s]; then slices of the heads' states, [2][head][16][68]
-    float* M = Ct;                  // at last, over both: the heads' weights of x, [head][s][t]
-    static_assert(kSlices >= kCt, "B transposed takes the slices' place");
-    __shared__ double L[kHeads][kQ];
-    __shared__ float dt[kHeads][kQ];
+    constexpr int kLdB = O::kLdB;
+    extern __shared__ __align__(16) __nv_bfloat16 parts_smem[];
+    __nv_bfloat16* Cp = parts_smem;                                   // C [part][t][n]
+    __nv_bfloat16* Bp = Cp + O::kPartsB;                              // B, then the heads' weights of x [group][part][t][s]
+    float* Sc = reinterpret_cast<float*>(Bp + O::kShared);            // the scores [t][s]
+    __shared__ float2 Lf[HEADS][kQ];
+    __shared__ float dt[HEADS][kQ];
     __shared__ Chunk chunk;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h0 = blockIdx.y * kHeads, g = h0 / (H / G);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, group = warp >> 2, h0 = blockIdx.y * HEADS, g = h0 / (H / G);
     if (warp == 0) {
         const Chunk c = find_chunk(blockIdx.x, qo_indptr, n_requests, min_len);
         if (lane == 0) chunk = c;
@@ -423,90 +523,190 @@ chunk_outputs4_kernel(const float* __restrict__ C, const float* __restrict__ B, 
     __syncthreads();
     const Chunk c = chunk;
     if (c.count == 0) return;
-    {
-        const float* C0 = C + (size_t)c.start * ld + (size_t)g * N;
-        const float* B0 = B + (size_t)c.start * ld + (size_t)g * N;
-#pragma unroll 4
-        for (int i = tid; i < kQ * (N / 4); i += 256) {
-            const int t = (i >> 2) % kQ, k = ((i >> 2) / kQ * 4 + (i & 3)) * 4;
-            float4 u = make_float4(0.f, 0.f, 0.f, 0.f), v = u;
-            if (t < c.count) {
-                u = ld4(C0 + (size_t)t * ld + k);
-                v = ld4(B0 + (size_t)t * ld + k);
-            }
-            float* a = Ct + k * kLd4 + t;
-            float* b = slices + k * kLd4 + t;
-            a[0] = u.x; a[kLd4] = u.y; a[2 * kLd4] = u.z; a[3 * kLd4] = u.w;
-            b[0] = v.x; b[kLd4] = v.y; b[2 * kLd4] = v.z; b[3 * kLd4] = v.w;
+    float* Ss = Sc + kQ * kLdSc + group * (O::kState + O::kX);        // this group's state [n][v] and x [t][v]
+    float* Xs = Ss + O::kState;
+    const int id = tid & 127;
+    auto load_state = [&](int hh) {
+        const float* src = states + ((size_t)c.slot * H + h0 + hh) * N * 64;
+        for (int i = id; i < N * 16; i += 128) cp_async16(Ss + (i >> 4) * kLd + (i & 15) * 4, src + i * 4, true);
+        cp_async_commit();
+    };
+    auto load_x = [&](int hh) {
+        const float* src = x + (size_t)c.start * ld + (size_t)(h0 + hh) * 64;
+        for (int i = id; i < kQ * 16; i += 128) {
+            const int t = i >> 4;
+            cp_async16(Xs + t * kLd + (i & 15) * 4, src + (size_t)(t < c.count ? t : 0) * ld + (i & 15) * 4, t < c.count);
         }
+        cp_async_commit();
+    };
+    auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + group) : "memory"); };
+    load_state(group);
+    load_x(group);
+    // one group C, the other B and the logarithms
+    if (group == 0) stage_parts<N>(Cp, C + (size_t)c.start * ld + (size_t)g * N, ld, c.count);
+    if (group == O::kGroups - 1) {
+        if ((warp & 3) < HEADS) {
+            const int hh = warp & 3;
+            double* L = reinterpret_cast<double*>(Sc) + hh * kQ;  // (the scores come later)
+            chunk_logs(step + h0 + hh, ld, c.start, c.count, expf(a_log[h0 + hh]), L, dt[hh]);
+            __syncwarp();
+            for (int t = lane; t < kQ; t += 32) Lf[hh][t] = two_floats(L[t]);
+        }
+        stage_parts<N>(Bp, B + (size_t)c.start * ld + (size_t)g * N, ld, c.count);
     }
-    if (warp < kHeads) chunk_logs(step + h0 + warp, ld, c.start, c.count, expf(a_log[h0 + warp]), L[warp], dt[warp]);
     __syncthreads();
-    {  // the scores: four tokens t and four s to a thread
-        const int t4 = (tid >> 4) * 4, s4 = (tid & 15) * 4;
-        float z[4][4] = {};
-#pragma unroll 4
-        for (int k = 0; k < N; ++k) {
-            const float4 a = ld4(Ct + k * kLd4 + t4), b = ld4(slices + k * kLd4 + s4);
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+    const int q = lane & 3, quad = lane >> 2, mi = lane >> 3, t0 = (warp & 3) * 16;
+    const __nv_bfloat16* c_at = Cp + (lane & 15) * kLdB + (lane >> 4) * 8;  // of ldmatrix: row t, column n of C
+    // the scores: 16 tokens t by 32 tokens s to a warp
+    for (int sh = group; sh < 2; sh += O::kGroups) {
+        float total[4][4] = {};
+        if (sh * 32 <= t0) {  // (the others are masked)
+#pragma unroll 1
+            for (int kb = 0; kb < N; kb += 64) {
+                PartSums<1, 4> z;
+                z.clear();
+#pragma unroll
+                for (int k0 = 0; k0 < 64; k0 += 16) {
+                    uint32_t a[1][kParts][4], b[kParts][4][2];
+#pragma unroll
+                    for (int p = 0; p < kParts; ++p) {
+                        ns_ldmatrix_x4(a[0][p], c_at + (p * kQ + t0) * kLdB + kb + k0);
+#pragma unroll
+                        for (int j = 0; j < 4; j += 2) {
+                            uint32_t r[4];
+                            ns_ldmatrix_x4(r, Bp + (p * kQ + sh * 32 + j * 8 + (mi >> 1) * 8 + (lane & 7)) * kLdB + kb + k0 + (mi & 1) * 8);
+                            b[p][j][0] = r[0]; b[p][j][1] = r[1]; b[p][j + 1][0] = r[2]; b[p][j + 1][1] = r[3];
+                        }
+                    }
+                    z.add<0>(a, b);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) total[j][e] += z.main[0][j][e] + z.rest[0][j][e];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+                *reinterpret_cast<float2*>(Sc + (t0 + quad + 8 * r) * kLdSc + sh * 32 + j * 8 + 2 * q) = make_float2(total[j][2 * r], total[j][2 * r + 1]);
+    }
+    __syncthreads();  // the scores are there, B has been read
+    const int v0 = (warp & 3) * 16, steps = (c.count + 15) >> 4;
+    __nv_bfloat16* Mp = Bp + group * O::kPartsM;
+    const __nv_bfloat16* m_at = Mp + (lane & 15) * kLdM + (lane >> 4) * 8;
+    const float *s_at = Ss + 2 * q * kLd + v0 + quad * 2, *x_at = Xs + 2 * q * kLd + v0 + quad * 2;
+    auto columns = [&](const float* at, int k0, uint32_t (&b)[kParts][2][2]) {  // rows k0 + 2 q, + 1, + 8, + 9 of a thread's two columns
+        float2 v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = *reinterpret_cast<const float2*>(at + (k0 + (e & 1) + (e >> 1) * 8) * kLd);
+        column_parts(v, b);
+    };
+#pragma unroll 1
+    for (int hh = group; hh < HEADS; hh += O::kGroups) {
+        const int h = h0 + hh;
+        const bool more = hh + O::kGroups < HEADS;
+        float y[4][2][4] = {};
+        PartSums<4, 2> sums;
+        auto take = [&] {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) z[i][j] = fmaf(av[i], bv[j], z[i][j]);
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) y[i][j][e] += sums.main[i][j][e] + sums.rest[i][j][e];
+        };
+        // the weights of x: a warp 16 tokens t, a lane two tokens s
+        auto weights = [&] {
+            constexpr int kBatch = 8;
+            const float2 l0 = Lf[hh][2 * lane], l1 = Lf[hh][2 * lane + 1];
+            const float d0 = dt[hh][2 * lane], d1 = dt[hh][2 * lane + 1];
+#pragma unroll 1
+            for (int r0 = 0; r0 < 16; r0 += kBatch) {  // (reads first, writes last: in turn each row would wait for the one before)
+                float2 z[kBatch], lt[kBatch];
+                uint32_t p[kBatch][kParts];
+#pragma unroll
+                for (int r = 0; r < kBatch; ++r) {
+                    z[r] = *reinterpret_cast<const float2*>(Sc + (t0 + r0 + r) * kLdSc + 2 * lane);
+                    lt[r] = Lf[hh][t0 + r0 + r];
+                }
+#pragma unroll
+                for (int r = 0; r < kBatch; ++r) {
+                    const bool in0 = 2 * lane <= t0 + r0 + r, in1 = 2 * lane + 1 <= t0 + r0 + r;
+                    const float e0 = expf(in0 ? difference(lt[r], l0) : 0.f), e1 = expf(in1 ? difference(lt[r], l1) : 0.f);  // (of all lanes: no branch)
+                    split_pair(in0 ? z[r].x * (e0 * d0) : 0.f, in1 ? z[r].y * (e1 * d1) : 0.f, p[r][0], p[r][1], p[r][2]);
+                }
+#pragma unroll
+                for (int r = 0; r < kBatch; ++r)
+#pragma unroll
+                    for (int k = 0; k < kParts; ++k) *reinterpret_cast<uint32_t*>(Mp + (k * kQ + t0 + r0 + r) * kLdM + 2 * lane) = p[r][k];
+            }
+        };
+        // The first group makes its weights before C S_in, the second after it: one is on the CUDA cores while the other is on the tensor cores.
+        if (group == 0) weights();
+        cp_async_wait<0>();
+        group_sync();  // the head's state and x are there
+        // C S_in
+#pragma unroll 1
+        for (int kb = 0; kb < N; kb += 64) {
+            sums.clear();
+#pragma unroll
+            for (int k = 0; k < 64; k += 16) {
+                uint32_t a[4][kParts][4], b[kParts][2][2];
+                columns(s_at, kb + k, b);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int p = 0; p < kParts; ++p) ns_ldmatrix_x4(a[i][p], c_at + (p * kQ + i * 16) * kLdB + kb + k);
+                sums.template add<0>(a, b);
+            }
+            take();
+        }
+        if (group == 1) weights();
+        group_sync();  // the state has been read, the weights are there
+        if (more) load_state(hh + O::kGroups);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const float f = expf(Lf[hh][i * 16 + quad + 8 * r].x);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) { y[i][j][2 * r] *= f; y[i][j][2 * r + 1] *= f; }
+            }
+        // the weights times x; a row tile ends at its own tokens
+        sums.clear();
+        auto row_tiles = [&](auto first_tile) {  // tokens 16 KS .. + 15 of x, for row tiles KS .. 3
+            constexpr int KS = decltype(first_tile)::value;
+            if (KS >= steps) return;
+            uint32_t a[4][kParts][4], b[kParts][2][2];
+            columns(x_at, KS * 16, b);
+#pragma unroll
+            for (int i = KS; i < 4; ++i)
+#pragma unroll
+                for (int p = 0; p < kParts; ++p) ns_ldmatrix_x4(a[i][p], m_at + (p * kQ + i * 16) * kLdM + KS * 16);
+            sums.template add<KS>(a, b);
+        };
+        row_tiles(std::integral_constant<int, 0>{});
+        row_tiles(std::integral_constant<int, 1>{});
+        row_tiles(std::integral_constant<int, 2>{});
+        row_tiles(std::integral_constant<int, 3>{});
+        take();
+        if (more) {
+            group_sync();  // x and the weights have been read
+            load_x(hh + O::kGroups);
+        } else {
+            ns_pdl_launch_dependents();
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(Sc + (s4 + j) * kLd4 + t4) = make_float4(z[0][j], z[1][j], z[2][j], z[3][j]);
-    }
-    __syncthreads();  // B has been read
-    const int hh = warp >> 1, h = h0 + hh, id = tid & 63;
-    const int ta = 32 * (warp & 1) + (lane >> 3) * 4, va = (lane & 7) * 4;  // tokens ta .. + 3 and ta + 16 .. + 19, features va .. + 3 and va + 32 .. + 35
-    const float* S0 = states + ((size_t)c.slot * H + h) * N * 64;
-    auto issue = [&](int sl) {
-        float* dst = slices + ((sl & 1) * kHeads + hh) * kRows * kLd4;
-        for (int i = id; i < kRows * 16; i += 64) cp_async16(dst + (i >> 4) * kLd4 + (i & 15) * 4, S0 + (size_t)(sl * kRows + (i >> 4)) * 64 + (i & 15) * 4, true);
-        cp_async_commit();
-    };
-    auto head_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + hh) : "memory"); };  // the two warps of a head
-    float y[8][8] = {};
-    issue(0);
-    for (int sl = 0; sl < N / kRows; ++sl) {
-        if (sl + 1 < N / kRows) { issue(sl + 1); cp_async_wait<1>(); }
-        else cp_async_wait<0>();
-        head_sync();
-        const float* Sl = slices + ((sl & 1) * kHeads + hh) * kRows * kLd4;
-        const float* Ck = Ct + sl * kRows * kLd4;
-#pragma unroll 4
-        for (int k = 0; k < kRows; ++k)
-            outer8(y, ld4(Ck + k * kLd4 + ta), ld4(Ck + k * kLd4 + ta + 16), ld4(Sl + k * kLd4 + va), ld4(Sl + k * kLd4 + va + 32));
-        head_sync();  // the slice may be filled again
-    }
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const float f = expf((float)L[hh][i < 4 ? ta + i : ta + 12 + i]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) y[i][j] *= f;
-    }
-    __syncthreads();  // C and the slices have been read by every head
-    float* Mh = M + hh * kQ * kLd4;
-    {
-        const double Lt = L[hh][id];
-#pragma unroll 4
-        for (int s = 0; s < kQ; ++s) Mh[s * kLd4 + id] = s <= id ? Sc[s * kLd4 + id] * (expf((float)(Lt - L[hh][s])) * dt[hh][s]) : 0.f;
-    }
-    head_sync();
-    const float* xh = x + (size_t)c.start * ld + (size_t)h * 64 + va;
-    const int s_end = min(c.count, 32 * (warp & 1) + 32);  // no weight of this warp's tokens lies beyond
-#pragma unroll 4
-    for (int s = 0; s < s_end; ++s)
-        outer8(y, ld4(Mh + s * kLd4 + ta), ld4(Mh + s * kLd4 + ta + 16), ld4(xh + (size_t)s * ld), ld4(xh + (size_t)s * ld + 32));
-    ns_pdl_launch_dependents();
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int t = i < 4 ? ta + i : ta + 12 + i;
-        if (t >= c.count) continue;
-        float* dst = out + (size_t)(c.start + t) * ld_out + (size_t)h * 64 + va;
-        *reinterpret_cast<float4*>(dst) = make_float4(y[i][0], y[i][1], y[i][2], y[i][3]);
-        *reinterpret_cast<float4*>(dst + 32) = make_float4(y[i][4], y[i][5], y[i][6], y[i][7]);
+            for (int r = 0; r < 2; ++r) {
+                const int t = i * 16 + quad + 8 * r;
+                if (t < c.count)
+                    *reinterpret_cast<float4*>(out + (size_t)(c.start + t) * ld_out + (size_t)h * 64 + v0 + q * 4) =
+                        make_float4(y[i][0][2 * r], y[i][1][2 * r], y[i][0][2 * r + 1], y[i][1][2 * r + 1]);
+            }
     }
 }
 
@@ -519,14 +719,13 @@ int launch_states4(const float* B, const float* x, const float* step, int ld, co
     NS_CHECK_LAUNCH("ns_ssm_chunked");
     return NS_OK;
 }
-template <int N>
-int launch_outputs4(const float* C, const float* B, const float* x, const float* step, int ld, const float* a_log, const int* qo_indptr, int n_requests,
-                    int min_len, int chunks, const float* states, float* out, int ld_out, int H, int G, cudaStream_t stream) {
-    constexpr int both = N * kLd4 + 2 * kHeads * 16 * kLd4, weights = kHeads * kQ * kLd4;
-    constexpr int smem = 4 * (kQ * kLd4 + (both > weights ? both : weights));
-    NS_CUDA(cudaFuncSetAttribute(chunk_outputs4_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    NS_LAUNCH(chunk_outputs4_kernel<N>, dim3(chunks, H / kHeads), 256, smem, stream, C, B, x, step, ld, a_log, qo_indptr, n_requests, min_len, states, out,
-              ld_out, H, G);
+template <int N, int HEADS>
+int launch_outputs_tc(const float* C, const float* B, const float* x, const float* step, int ld, const float* a_log, const int* qo_indptr, int n_requests,
+                      int min_len, int chunks, const float* states, float* out, int ld_out, int H, int G, cudaStream_t stream) {
+    using O = OutputsTc<N, HEADS>;
+    NS_CUDA(cudaFuncSetAttribute(chunk_outputs_tc_kernel<N, HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, O::kSmem));
+    NS_LAUNCH((chunk_outputs_tc_kernel<N, HEADS>), dim3(chunks, H / HEADS), O::kThreads, O::kSmem, stream, C, B, x, step, ld, a_log, qo_indptr, n_requests,
+              min_len, states, out, ld_out, H, G);
     NS_CHECK_LAUNCH("ns_ssm_chunked");
     return NS_OK;
 }
@@ -537,7 +736,7 @@ int launch_outputs4(const float* C, const float* B, const float* x, const float*
 // per head); a_log [H]; state [slots, state_floats] with S [H, N, V] at the start of a row; states: scratch for `chunks` chunks of
 // H * N * V floats, decays: H floats each, where `chunks` is at least the number of chunks of all requests of min_len tokens or more.
 // Requests of fewer tokens are not touched.  Four heads go to a block, where they can, once that makes more than
-// `four_from` blocks.
+// `four_from` blocks (half of that on the tensor cores).
 NS_API int ns_ssm_chunked(const float* C, const float* B, const float* x, const float* step, int ld, const float* a_log, float* state,
                           long long state_floats, const int* qo_indptr, const int* state_slot, float* out, int ld_out, int n_requests,
                           int min_len, int chunks, float* states, float* decays, int H, int G, int N, int Np, int V, int four_from, cudaStream_t stream) {
@@ -548,10 +747,10 @@ NS_API int ns_ssm_chunked(const float* C, const float* B, const float* x, const 
     const int n_tiles = (N + 63) / 64, v_tiles = (V + 63) / 64;
     if (H > 65535 || n_tiles * v_tiles > 65535) NS_FAIL(NS_ERR_UNSUPPORTED, "ns_ssm_chunked: %d heads, state of %d x %d exceed the grid", H, N, V);
     const bool many = (long long)chunks * H > (long long)four_from * kHeads;
-    const bool four = many && V == 64 && (N == 64 || N == 128) && Np == N && (H / G) % kHeads == 0 && ld_out % 4 == 0;
-#define NS_SSM_FOUR(F, ...) (N == 128 ? F<128>(__VA_ARGS__) : F<64>(__VA_ARGS__))
+    const bool tensor = V == 64 && (N == 64 || N == 128) && Np == N && ld_out % 4 == 0, group4 = tensor && (H / G) % kHeads == 0, four = many && group4;
     if (four) {
-        const int rc = NS_SSM_FOUR(launch_states4, B, x, step, ld, a_log, qo_indptr, n_requests, min_len, chunks, states, decays, H, G, stream);
+        auto* launch = N == 128 ? launch_states4<128> : launch_states4<64>;
+        const int rc = launch(B, x, step, ld, a_log, qo_indptr, n_requests, min_len, chunks, states, decays, H, G, stream);
         if (rc) return rc;
     } else {
         NS_LAUNCH(chunk_states_kernel, dim3(chunks, H, n_tiles * v_tiles), kThreads, 0, stream, B, x, step, ld, a_log, qo_indptr, n_requests, min_len,
@@ -569,9 +768,14 @@ NS_API int ns_ssm_chunked(const float* C, const float* B, const float* x, const 
     else { if (many) NS_SSM_PASS(1, true); else NS_SSM_PASS(1, false); }
 #undef NS_SSM_PASS
     NS_CHECK_LAUNCH("ns_ssm_chunked");
-    if (four)
-        return NS_SSM_FOUR(launch_outputs4, C, B, x, step, ld, a_log, qo_indptr, n_requests, min_len, chunks, states, out, ld_out, H, G, stream);
-#undef NS_SSM_FOUR
+    if (tensor) {
+        // a round of blocks of four heads takes 24 us with a state of 128 rows, one of a head each 11.7: four from two rounds of single heads on (500
+        // tokens, 64 heads: 24 against 47 us; 150 tokens, 32 heads: 22 against 12)
+        const bool fours = group4 && (long long)chunks * H > 2LL * four_from;
+        auto* launch = N == 128 ? (fours ? launch_outputs_tc<128, kHeads> : launch_outputs_tc<128, 1>)
+                                : (fours ? launch_outputs_tc<64, kHeads> : launch_outputs_tc<64, 1>);
+        return launch(C, B, x, step, ld, a_log, qo_indptr, n_requests, min_len, chunks, states, out, ld_out, H, G, stream);
+    }
     NS_LAUNCH(chunk_outputs_kernel, dim3(chunks, H, v_tiles), kThreads, 0, stream, C, B, x, step, ld, a_log, qo_indptr, n_requests, min_len,
               states, out, ld_out, H, G, N, Np, V);
     NS_CHECK_LAUNCH("ns_ssm_chunked");
