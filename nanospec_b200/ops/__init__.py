@@ -1642,6 +1642,15 @@ def moe_grouped(x: torch.Tensor, pair_of: torch.Tensor, offsets: torch.Tensor, w
 MOE_TILE: int | None = None  # rows of a tile in `moe_grouped_tc` (None: by the rows an expert holds on average)
 
 
+def moe_tile(E: int, n: int, ff: int) -> int:
+    """Rows of a tile of the experts' products: 256 on pairs of SMs where an expert holds enough to fill most of one (32 experts of 116 rows, width
+    2048: 90 us against 83 in tiles of 128; of 124: 91 / 96) and there is more than a tile for each pair (16 of 300 rows, 72 tiles: 41 / 33; 4 of 700,
+    80 tiles: 48 / 53)."""
+    if n >= 120 * E and max(E, n // 256) * -(-ff // 128) >= 80:
+        return 256
+    return 128 if n > 24 * E else 32
+
+
 def moe_grouped_tc(xs: torch.Tensor, offsets: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, act: torch.Tensor, ys: torch.Tensor,
                    unit: GatedUnit = SILU) -> torch.Tensor:
     """Every expert over its rows of the plan as tcgen05 products whose tiles are found from the offsets on the device
@@ -1654,9 +1663,9 @@ def moe_grouped_tc(xs: torch.Tensor, offsets: torch.Tensor, w_gate_up: torch.Ten
     if not all(t.is_contiguous() and t.dtype == torch.bfloat16 for t in (xs, w_gate_up, w_down, act, ys)) or w_gate_up.shape[2] != width \
             or w_down.shape != (E, width, ff) or act.shape != (n, ff) or ys.shape != (n, width) or offsets.numel() != E + 1:
         raise KernelError("moe_grouped_tc: contiguous bfloat16 operands of the sizes the experts have")
-    tile = MOE_TILE or (256 if n >= 300 * E else 128 if n > 24 * E else 32)
+    tile = MOE_TILE or moe_tile(E, n, ff)
     lib.call("ns_moe_grouped_tc", xs.data_ptr(), offsets.data_ptr(), w_gate_up.data_ptr(), w_down.data_ptr(), act.data_ptr(), ys.data_ptr(),
-             E, n, width, ff, tile, *unit.args, _tc(xs.device).error.data_ptr(), _stream())
+             E, n, width, ff, tile, sm_count(), *unit.args, _tc(xs.device).error.data_ptr(), _stream())
     return ys
 
 

@@ -98,3 +98,11 @@ def test_prefill_of_many_requests(nq, nkv, brings, entry, monkeypatch):
     ops.check_kernel_errors()
     assert names[0] == entry and names[0] != names[1]
     assert float((outs[0].double() - outs[1].double()).norm() / outs[1].double().norm()) < 2.0 ** -8
+
+
+def test_tiles_of_the_experts_products():
+    """By the rows that an expert holds, and pairs of SMs only where there are tiles for them."""
+    from nanospec_b200 import ops
+    assert [ops.moe_tile(32, 32 * per, 1024) for per in (1, 24, 25, 119, 120, 600)] == [32, 32, 128, 128, 256, 256]
+    assert [ops.moe_tile(E, 300 * E, 1024) for E in (1, 8, 9, 10)] == [128, 128, 256, 256]
+    assert ops.moe_tile(16, 300 * 16, 512) == 128 and ops.moe_tile(20, 300 * 20, 512) == 256
