@@ -22,18 +22,26 @@
 //        x alone
 //   4-12 add a finished block's accumulator to their sums in registers (32 columns to a thread), add up groups, write results
 //
-// Microseconds on a B200 in a graph of such products (w from DRAM), the kernels of gemm_f32.cu -> this one with its parts kernel:
-//     M x N x K         1 x 2048 x 2048   8 x 2048 x 8192   3 x 32768 x 2048   200 x 8192 x 1024   641 x 2048 x 8192   641 x 16384 x 2048   8 x 1024 x 512
-//     before / now         23 / 12            97 / 28           90 / 59            120 / 43             711 / 144           943 / 279          7 / 10
-// From K = 1024 on it was slower nowhere (1 x 1024 x 1024: 11.8 / 11.2); that line is the dispatch's (F32_TC_MIN_K).
+// Weights that a checkpoint held in 16 bits have neither middle nor low parts.  Where a block's 128 x 64 of w have none, the three products with
+// them are left out: they are zeros, so the bits stay (641 x 16384 x 2048 213 -> 167 us).  The eight warps see the parts as they make them.
+//
+// Microseconds on a B200 in a graph of such products (w from DRAM): the kernels of gemm_f32.cu, this one with its parts kernel on weights of 24 bits,
+// and on bfloat16's numbers
+//     M x N x K   1 x 2048 x 2048   8 x 2048 x 8192   3 x 32768 x 2048   200 x 8192 x 1024   641 x 2048 x 8192   641 x 16384 x 2048   8 x 1024 x 512
+//     fmaf               23                97                 89                 119                 709                 943                 7.0
+//     24 bits            11.5              26                 51                  32                 117                 213                 9.0
+//     bfloat16's         11.3              25                 51                  30                  94                 167                 9.0
+// From K = 1024 on it was slower nowhere (1 x 1024 x 1024: 11.8 / 10.5); that line is the dispatch's (F32_TC_MIN_K).  Groups that were added up in y
+// (a read-modify-write of the tile for each) took 244 us instead of 213 on 641 x 16384 x 2048, 128 instead of 117 on 641 x 2048 x 8192.
 // Error against 64 bits (2-norm, normal x and w), one chain of fmaf / this kernel, in 1e-7: K = 1024 5.7 / 1.0, 2048 8.1 / 1.0, 8192 16 / 1.2,
 // 14336 21 / 1.4; numbers over 60 powers of two 7.0 / 1.3; all of one sign 6.3 / 0.9.
-// Bound with 96 rows (1,700 cycles a block of k; its MMAs run for 1,190): shared memory, which the MMAs' operand, TMA's writes and the reads of w
-// keep at four fifths of its rate; with 16 rows (1,200 cycles) taking w apart.
+// Bound, with 96 rows, by shared memory, which the MMAs' operand, TMA's writes and the reads of w share (24 bits: 1,700 cycles a block of k, of which
+// the MMAs run for 1,190; bfloat16's numbers: 1,290 and 600); with 16 rows (990 cycles) by taking w apart.
 //
 // The accumulators are double buffered, both operands' parts have three or four stages (a warpgroup of the eight warps takes every other block),
 // so that taking apart, multiplying and adding up do not wait for one another.
 #include <cfloat>
+#include <type_traits>
 
 #include "float_parts.cuh"
 #include "tcgen05_utils.cuh"
@@ -44,7 +52,7 @@ constexpr int kBM = 128, kBK = 64, kMaxBN = 96;
 constexpr int kRingBytes = kBM * kBK * 4;        // a stage of floats of w: two boxes of 128 rows x 32 floats
 constexpr int kMaxRing = 6, kMaxStages = 4;      // stages of w's ring and of the parts at most
 constexpr int kSmemMax = 227 * 1024;
-constexpr int kBarBytes = 320, kSmemFixed = 1024 + kBarBytes;  // barriers; alignment
+constexpr int kBarBytes = 384, kSmemFixed = 1024 + kBarBytes;  // barriers; alignment
 constexpr uint32_t kTmemCols = 512;              // two accumulators, then the stages of w's parts (32 columns to a part)
 constexpr uint32_t kPartsCols = kParts * kBK / 2;
 constexpr float kTiny = 8.077935669463161e-28f;  // 2^-90
@@ -135,7 +143,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     auto acc_free = [&](int b) { return bar0 + 8u * (kRings + 2 + b); };                    // which has been read
     auto go = [&](int s) { return bar0 + 8u * (kRings + 4 + s); };                          // all that a block's MMAs wait for is there
     const uint32_t holder = bar0 + 8u * (kRings + 4 + kMaxStages);
-    static_assert(8 * (kRings + 5 + kMaxStages) <= kBarBytes, "barriers");
+    auto finer = [&](int s) { return bar0 + 8u * (kRings + 6 + kMaxStages) + 16u * s; };    // four warps' words: does w's tile have middle or low parts?
+    static_assert(8 * (kRings + 6 + kMaxStages) % 16 == 0 && 8 * (kRings + 6 + kMaxStages) + 16 * kMaxStages <= kBarBytes, "barriers");
     float* groups_smem = reinterpret_cast<float*>(smem_dyn + (bar0 + (uint32_t)kBarBytes - smem_u32(smem_dyn)));  // splits > 1: this block's groups [group][row of x][128]
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (known to be one number for the warp)
 
@@ -218,16 +227,29 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             tc_fence_after();
             const uint32_t d = tmem_base + (uint32_t)b * kBN, wp = tmem_base + 2 * kBN + (uint32_t)s * kPartsCols;
             const uint64_t xp = smem_desc(x_smem + (uint32_t)s * R::kXStage);
-            constexpr int pw[6] = {2, 0, 1, 1, 0, 0}, px[6] = {0, 2, 1, 0, 1, 0};
+            // Weights that bfloat16 holds exactly (a checkpoint of that type run in float32) have no middle or low parts: three of the six products
+            // are zeros, and adding zeros changes nothing.
+            uint32_t f[4];
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3]) : "r"(finer(s)) : "memory");
             // Unrolled, a lane elected for each, offsets known to the compiler: operands that are not in uniform registers cost an MMA more to
             // issue than it runs (it runs for 20 cycles with 16 columns, 55 with 96; issued from a branch of one lane it took 126).
+            auto products = [&](auto with_parts_of_w) {
+                constexpr bool kAll = decltype(with_parts_of_w)::value;
+                constexpr int pw[6] = {2, 0, 1, 1, 0, 0}, px[6] = {0, 2, 1, 0, 1, 0};
+                bool first = true;
 #pragma unroll
-            for (int p = 0; p < 6; ++p) {
+                for (int p = 0; p < 6; ++p) {
+                    if (!kAll && pw[p] != 0) continue;
 #pragma unroll
-                for (int k = 0; k < kBK / 16; ++k)
-                    if (elect_one())
-                        umma_bf16_ts(d, wp + pw[p] * 32 + k * 8, xp + ((px[p] * part_bytes + k * 32) >> 4), idesc, (p > 0 || k > 0) ? 1u : 0u);
-            }
+                    for (int k = 0; k < kBK / 16; ++k) {
+                        if (elect_one())
+                            umma_bf16_ts(d, wp + pw[p] * 32 + k * 8, xp + ((px[p] * part_bytes + k * 32) >> 4), idesc, first ? 0u : 1u);
+                        first = false;
+                    }
+                }
+            };
+            if (__any_sync(0xffffffffu, (f[0] | f[1] | f[2] | f[3]) != 0)) products(std::true_type{});
+            else products(std::false_type{});
             if (elect_one()) umma_commit(done(b));
             if (elect_one()) umma_commit(empty(s));
             if (++s == stages) { s = 0; s_turn ^= 1u; }
@@ -297,26 +319,39 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             }
             tc_fence_after();
             const uint32_t src = w_smem + (uint32_t)s * kRingBytes + row_off;
+            uint32_t rest = 0;
+            float4 v[2][4];  // 16 k at a time, the next ones on their way (read and taken apart in turn: 1,900 cycles a tile, most of them waiting)
+            auto read = [&](int q) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint32_t hi[16], mid[16], lo[16];
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    float4 v;
+                for (int c = 0; c < 4; ++c)
                     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(src + h * (kRingBytes / 2) + (((uint32_t)c ^ sw) << 4)));
-                    split_pair(v.x, v.y, hi[2 * c], mid[2 * c], lo[2 * c]);
-                    split_pair(v.z, v.w, hi[2 * c + 1], mid[2 * c + 1], lo[2 * c + 1]);
+                                 : "=f"(v[q & 1][c].x), "=f"(v[q & 1][c].y), "=f"(v[q & 1][c].z), "=f"(v[q & 1][c].w)
+                                 : "r"(src + (q >> 1) * (kRingBytes / 2) + (((uint32_t)((q & 1) * 4 + c) ^ sw) << 4)));
+            };
+            read(0);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (q < 3) read(q + 1);
+                uint32_t hi[8], mid[8], lo[8];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    split_pair(v[q & 1][c].x, v[q & 1][c].y, hi[2 * c], mid[2 * c], lo[2 * c]);
+                    split_pair(v[q & 1][c].z, v[q & 1][c].w, hi[2 * c + 1], mid[2 * c + 1], lo[2 * c + 1]);
                 }
-                if (h == 1) {
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(w_empty(s));
+#pragma unroll
+                for (int c = 0; c < 8; ++c) rest |= mid[c];  // (no middle part: no low one)
+                if (q == 3) {
+                    const bool any = __any_sync(0xffffffffu, (rest & 0x7fff7fffu) != 0);  // (a zero's sign is nothing)
+                    if (lane == 0) {
+                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(finer(p) + 4u * quarter), "r"((int)any) : "memory");
+                        mbar_arrive(w_empty(s));
+                    }
                     __syncwarp();
                 }
-                const uint32_t dst = t_row + (uint32_t)p * kPartsCols + h * 16;
-                tmem_st16(dst, hi);
-                tmem_st16(dst + 32, mid);
-                tmem_st16(dst + 64, lo);
+                const uint32_t dst = t_row + (uint32_t)p * kPartsCols + q * 8;
+                tmem_st8(dst, hi);
+                tmem_st8(dst + 32, mid);
+                tmem_st8(dst + 64, lo);
             }
             tmem_st_wait();
             tc_fence_before();
@@ -327,6 +362,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         // ---------------- sums: a thread owns a row of w and all or half of the tile's rows of x ----------------
         ns_pdl_wait();
         const int quarter = warp & 3, c0 = (warp - R::kSum) / 4 * 32, cols = min(32, bn - c0);  // (none left: the warp only keeps step)
+        constexpr int kLoad = kBN <= 32 ? 32 : 8;  // columns at a time: 64 sums leave no more registers
         const uint32_t t_acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0;
         int g = 0;
         bool ok = true;
@@ -334,6 +370,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             int m0, n0;
             tile_at(i, m0, n0);
             const int n_warp = n0 + quarter * 32, n = n_warp + lane;
+            float all[32];  // the groups so far
             for (int kb = kb0; kb < kb0 + n_kb;) {
                 float sum[32];
 #pragma unroll
@@ -348,11 +385,15 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     }
                     tc_fence_after();
                     if (cols > 0) {  // (columns past the tile's hold what other tiles left: added and not stored)
-                        uint32_t r[32];
-                        tmem_ld32(t_acc + (uint32_t)b * kBN, r);
-                        tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) sum[j] += __uint_as_float(r[j]);
+                        for (int c = 0; c < 32; c += kLoad) {
+                            uint32_t r[kLoad];
+                            if constexpr (kLoad == 8) tmem_ld8(t_acc + (uint32_t)b * kBN + c, r);
+                            else tmem_ld32(t_acc + (uint32_t)b * kBN + c, r);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < kLoad; ++j) sum[c + j] += __uint_as_float(r[j]);
+                        }
                     }
                     tc_fence_before();
                     __syncwarp();
@@ -364,44 +405,28 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
                     for (int j = 0; j < 32; ++j)
                         if (j < cols) dst[j * kBM] = sum[j];
-                    continue;
-                }
-                // the groups before wait in y: one thread reads and writes an element, in the groups' order
-                const bool last = group == a.groups - 1;
-                const int rows = n < a.N ? min(cols, a.M - m0 - c0) : 0;
-                bool odd = false;
-                float* out = a.y + (size_t)(m0 + c0) * a.ldy + n;
-                if (last && group > 0) {
-                    const float* o = out;
-                    float before[32];
+                } else {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        before[j] = j < rows ? __ldcg(o) : 0.f;
-                        o += a.ldy;
-                        asm volatile("" : "+l"(o));  // (a running pointer: 32 addresses kept through the sums would not leave them their registers)
-                    }
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) sum[j] = before[j] + sum[j];
+                    for (int j = 0; j < 32; ++j) all[j] = group == 0 ? sum[j] : all[j] + sum[j];
                 }
+            }
+            if (!ok) break;
+            if (splits > 1) continue;
+            const int rows = n < a.N ? min(cols, a.M - m0 - c0) : 0;
+            bool odd = false;
+            float* out = a.y + (size_t)(m0 + c0) * a.ldy + n;
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    if (j < rows) {
-                        if (last) {
-                            *out = sum[j];
-                            odd |= out_of_range(sum[j]);
-                        } else if (group == 0) {
-                            __stcg(out, sum[j]);
-                        } else {
-                            asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(out), "f"(sum[j]) : "memory");
-                        }
-                    }
-                    out += a.ldy;
-                    asm volatile("" : "+l"(out));
+            for (int j = 0; j < 32; ++j) {
+                if (j < rows) {
+                    *out = all[j];
+                    odd |= out_of_range(all[j]);
                 }
-                if (__any_sync(0xffffffffu, odd)) {
+                out += a.ldy;
+                asm volatile("" : "+l"(out));  // (a running pointer: 32 addresses kept through the sums would not leave them their registers)
+            }
+            if (__any_sync(0xffffffffu, odd)) {
 #pragma unroll 1
-                    for (int m = m0 + c0; m < min(m0 + c0 + cols, a.M); ++m) mend_row(a, m, n_warp);
-                }
+                for (int m = m0 + c0; m < min(m0 + c0 + cols, a.M); ++m) mend_row(a, m, n_warp);
             }
         }
     }

@@ -177,8 +177,8 @@ TENSOR_CORE_GEMM_MAX_TOKENS: int | None = 64
 
 
 # float32 products of at least this K go to the tcgen05 kernel on parts (csrc/gemm_f32_tc.cu).  The rule looks at w alone, so that a row's
-# bits do not depend on the rows beside it: below this K many rows would gain (300 x 4096 x 512: 47 -> 17 us), but a few lose to the kernel that
-# takes x apart (8 x 1024 x 512: 7.0 -> 10.1); from here on both gain (1 x 1024 x 1024: 11.8 -> 11.2).
+# bits do not depend on the rows beside it: below this K many rows would gain (300 x 4096 x 512: 47 -> 14 us), but a few lose to the kernel that
+# takes x apart (8 x 1024 x 512: 7.0 -> 9.0); from here on both gain (1 x 1024 x 1024: 11.8 -> 10.5).
 F32_TC_MIN_K = 1024
 
 
@@ -251,9 +251,9 @@ def gemm_splits(M: int, N: int, K: int) -> int:
 
 def f32_tiles(M: int, N: int, K: int, sms: int) -> tuple[int, int]:
     """(rows of x to a tile, blocks that share a tile's k) of the float32 product on the tensor cores.  A block of 64 k of a tile takes about
-    (120 + rows) units of 5 ns (0.70 us with 16 rows, 1.12 with 96: taking w's tile apart is a constant part); tiles come in rounds over the SMs, and
-    where they are few, a cluster of two or four divides the groups of k that the kernel adds up in order (8 x 2048 x 8192: 91 us alone, 50, 32, and
-    38 with eight).  The bits do not depend on the choice."""
+    (120 + rows) units of 4.3 ns (0.58 us with 16 rows, 0.93 with 96, less for weights of 16 bits: taking w's tile apart is a constant part); tiles come
+    in rounds over the SMs, and where they are few, a cluster of two or four divides the groups of k that the kernel adds up in order (8 x 2048 x
+    8192: 75 us alone, 43, 26; eight took longer than four).  The bits do not depend on the choice."""
     blocks = -(-K // 64)
     group = -(-blocks // min(8, -(-blocks // 8)))
     groups = -(-blocks // group)

@@ -105,6 +105,30 @@ def test_f32_tc_infinities_and_ends_of_the_range(tiles):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,tiles", [(1, 128, 1024, (16, 2)), (33, 300, 1092, (48, 1)), (97, 257, 2048, (96, 1)), (20, 20000, 1024, (32, 1))])
+def test_f32_tc_weights_of_16_bits(M, N, K, tiles):
+    """Products with parts of w that are zero are left out: such weights' elements stay within the bound, and keep their bits when another row of w's tile,
+    in its first or last block of k, has all three parts (then none are left out)."""
+    from nanospec_b200 import ops
+    x, w = _operands(M, N, K, M + N)
+    w = w.bfloat16().float()
+    got, other = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    ops.linear_f32_tc(x, w, got, tiles)
+    ref, size = x.double() @ w.double().T, x.abs().double() @ w.abs().double().T
+    assert bool(((got.double() - ref).abs() <= size * (50 + K // 64 + 8) * 2.0 ** -24).all())
+    for n, k in ((0, 0), (N // 2, K - 1), (N - 1, 64)):
+        v = w.clone()
+        v[n, k] += 2.0 ** -18
+        assert float(v[n, k]) != float(w[n, k])
+        ops.linear_f32_tc(x, v, other, tiles)
+        keep = [c for c in range(N) if c != n]
+        assert torch.equal(got[:, keep], other[:, keep])
+        ref = x.double() @ v[n].double()
+        assert bool(((other[:, n].double() - ref).abs() <= size[:, n] * 1.01 * (50 + K // 64 + 8) * 2.0 ** -24).all())
+    ops.check_kernel_errors()
+
+
+@pytest.mark.gpu
 def test_f32_tc_late_weights():
     """Weights from DRAM, whose tiles land out of order: the bits of the first run again and again (odd and even rings of w's tiles)."""
     from nanospec_b200 import ops
