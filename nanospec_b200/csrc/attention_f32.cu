@@ -5,8 +5,12 @@
 // A block takes a run of tokens of one request and one kv head: its rows are (token, query head of that kv head), 32 / (nq / nkv)
 // tokens of them, eight rows to each of four warps.  Keys and values come 32 at a time through two cp.async stages.  A lane is a key in the
 // scores (a chain of fmaf over the features in ascending order, as there) and a feature in the sums over the values (keys in
-// ascending order, as there); a warp's eight rows share every read of a key or a value.  Three prompts of 641 tokens in all, 32 heads of 64 over
-// 8, a whole step of two layers: 6242 us with the one-warp kernel, 5061 with this one.
+// ascending order, as there); a warp's eight rows share every read of a key or a value.
+//
+// Bound by the chain of a block's keys where few blocks share an SM (32 keys: 5,300 cycles, of them copies 650, scores 1,600, softmax 1,100, values 1,200), by
+// shared memory (1,450 of its cycles for the same) where many do.  Three prompts of 300, 200 and 141 tokens, 32 heads of 64 over 8: 92 -> 55 us; one
+// of 300 tokens, 4 heads over 1: 74 -> 32 us.  Of 11,000 cycles for 32 keys, 5,000 went into copies whose addresses shared registers, so that each
+// waited for the data of the one before it, and 1,800 into the rows' reductions, one after the other.
 #include "common.cuh"
 
 namespace {
@@ -46,17 +50,32 @@ attention_f32_kernel(const float* __restrict__ q, int q_stride, const float* __r
     const int key_end = positions[first + off_end - 1] + 1;  // of the block's last token
     const int n_blocks = (key_end + kKeys - 1) / kKeys;
 
+    // a lane's key of a block (beyond the end: the last one again, never used): where it is, found one block ahead of its copy
+    auto find = [&](int kb) {
+        const int key = min(kb * kKeys + lane, key_end - 1);
+        return ((size_t)bt[key / page_size] * nkv + hk) * page_size + key % page_size;
+    };
+    size_t slot = find(0);
     auto issue = [&](int kb) {
         if (kb < n_blocks) {
-            float* kd = ks + (kb & 1) * kKeys * ldk;
-            float* vd = vs + (kb & 1) * kKeys * dv;
-            // a warp takes the keys warp, warp + 4, ...: one look at the block table each
-            for (int j = warp; j < kKeys; j += kWarps) {
-                const int key = min(kb * kKeys + j, key_end - 1);  // (keys beyond the end: the last one again, never used)
-                const size_t slot = ((size_t)bt[key / page_size] * nkv + hk) * page_size + key % page_size;
-                for (int p = lane; p < pieces_k; p += 32) cp_async16(kd + j * ldk + 4 * p, k_cache + slot * d + 4 * p);
-                for (int p = lane; p < pieces_v; p += 32) cp_async16(vd + j * dv + 4 * p, v_cache + slot * dv + 4 * p);
+            float* kd = ks + (kb & 1) * kKeys * ldk + warp * (kKeys / kWarps) * ldk;
+            float* vd = vs + (kb & 1) * kKeys * dv + warp * (kKeys / kWarps) * dv;
+            // straight code and an address register to each copy: copies whose addresses shared registers waited for one another's data
+            const float *kg[kKeys / kWarps], *vg[kKeys / kWarps];
+#pragma unroll
+            for (int j = 0; j < kKeys / kWarps; ++j) {  // (a warp takes eight keys)
+                const size_t at = __shfl_sync(0xffffffffu, slot, warp * (kKeys / kWarps) + j);
+                kg[j] = k_cache + at * d + 4 * lane;
+                vg[j] = v_cache + at * dv + 4 * lane;
             }
+#pragma unroll
+            for (int j = 0; j < kKeys / kWarps; ++j) {
+                if (lane < pieces_k) cp_async16(kd + j * ldk + 4 * lane, kg[j]);
+                if (lane + 32 < pieces_k) cp_async16(kd + j * ldk + 4 * lane + 128, kg[j] + 128);
+                if (lane < pieces_v) cp_async16(vd + j * dv + 4 * lane, vg[j]);
+                if (DPL > 4 && lane + 32 < pieces_v) cp_async16(vd + j * dv + 4 * lane + 128, vg[j] + 128);
+            }
+            slot = find(kb + 1);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -95,33 +114,50 @@ attention_f32_kernel(const float* __restrict__ q, int q_stride, const float* __r
 #pragma unroll 4
             for (int e = 0; e < d; e += 4) {
                 const float4 b = *reinterpret_cast<const float4*>(kr + e);
+                float4 a[kQ];
 #pragma unroll
-                for (int i = 0; i < kQ; ++i) {
-                    const float4 a = *reinterpret_cast<const float4*>(qw + i * d + e);
-                    s[i] = fmaf(a.x, b.x, s[i]);
-                    s[i] = fmaf(a.y, b.y, s[i]);
-                    s[i] = fmaf(a.z, b.z, s[i]);
-                    s[i] = fmaf(a.w, b.w, s[i]);
-                }
+                for (int i = 0; i < kQ; ++i) a[i] = *reinterpret_cast<const float4*>(qw + i * d + e);
+#pragma unroll
+                for (int i = 0; i < kQ; ++i) s[i] = fmaf(a[i].x, b.x, s[i]);
+#pragma unroll
+                for (int i = 0; i < kQ; ++i) s[i] = fmaf(a[i].y, b.y, s[i]);
+#pragma unroll
+                for (int i = 0; i < kQ; ++i) s[i] = fmaf(a[i].z, b.z, s[i]);
+#pragma unroll
+                for (int i = 0; i < kQ; ++i) s[i] = fmaf(a[i].w, b.w, s[i]);
             }
+            // the eight rows' reductions side by side: one after the other they were most of the block's time
             const int key = kb * kKeys + lane;
+            float top[kQ], corr[kQ];
+#pragma unroll
+            for (int i = 0; i < kQ; ++i) s[i] *= scale;
+            if (softcap > 0.f) {
+#pragma unroll
+                for (int i = 0; i < kQ; ++i) s[i] = softcap * tanhf(s[i] / softcap);
+            }
+#pragma unroll
+            for (int i = 0; i < kQ; ++i) top[i] = s[i] = key < kend[i] ? s[i] : -INFINITY;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < kQ; ++i) top[i] = fmaxf(top[i], __shfl_xor_sync(0xffffffffu, top[i], o));
 #pragma unroll
             for (int i = 0; i < kQ; ++i) {
-                float p = 0.f;
-                if (kb * kKeys < kend[i]) {  // (uniform in the warp; a row that has seen all its keys stays as it is)
-                    const bool valid = key < kend[i];
-                    float z = s[i] * scale;
-                    if (softcap > 0.f) z = softcap * tanhf(z / softcap);
-                    z = valid ? z : -INFINITY;
-                    const float m_new = fmaxf(m[i], ns_warp_max(z));
-                    const float corr = expf(m[i] - m_new);
-                    p = valid ? expf(z - m_new) : 0.f;
-                    l[i] = l[i] * corr + ns_warp_sum(p);
+                const float m_new = fmaxf(m[i], top[i]);
+                corr[i] = expf(m[i] - m_new);  // (1 for a row that has seen all its keys)
+                s[i] = expf(s[i] - m_new);
+                m[i] = m_new;
+                top[i] = s[i];
+            }
 #pragma unroll
-                    for (int u = 0; u < DPL; ++u) acc[i][u] *= corr;
-                    m[i] = m_new;
-                }
-                s[i] = p;
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < kQ; ++i) top[i] += __shfl_xor_sync(0xffffffffu, top[i], o);
+#pragma unroll
+            for (int i = 0; i < kQ; ++i) {
+                l[i] = l[i] * corr[i] + top[i];
+#pragma unroll
+                for (int u = 0; u < DPL; ++u) acc[i][u] *= corr[i];
             }
 #pragma unroll
             for (int i = 0; i < kQ; i += 4) *reinterpret_cast<float4*>(pw + lane * kQ + i) = make_float4(s[i], s[i + 1], s[i + 2], s[i + 3]);
@@ -143,6 +179,7 @@ attention_f32_kernel(const float* __restrict__ q, int q_stride, const float* __r
                 for (int j = 0; j < kKeys; ++j) add_values(j, true);
             } else {
                 const int cnt = min(kKeys, kend_max - kb * kKeys);
+#pragma unroll 4
                 for (int j = 0; j < cnt; ++j) add_values(j, false);
             }
         }

@@ -588,7 +588,8 @@ def f32_tiles_pay(ctx, nq: int, dim: int) -> bool:
     """Whether a float32 step's portions take csrc/attention_f32.cu: us of the exact kernel (a warp's chain over its keys, and all pairs of rows and
     keys) against those of a block's chain over groups of 32 keys (exact kernel, tiles; one request, 32 heads of 64 over 8: a prompt of 2 tokens 6.2
     and 13.4, of 40 23.4 and 23.0, of 300 434 and 87; 2 tokens behind 1,500 488 and 312; 4 heads of 32 over 1, a prompt of 128 26 and 33).
-    Of 512 steps and layers the rule takes a kernel slower by more than 5 % at 10, by 5 us in the mean.  The bits are the same."""
+    Those are the times that the line was fitted to.  The tiles have since become up to twice as fast (300 tokens, 32 heads of 64: 51 us) and pay
+    somewhat earlier than the line says; the bits are the same on both sides of it."""
     if F32_TILES is not None:
         return F32_TILES
     prompts = _prompts(ctx)
