@@ -81,13 +81,21 @@ __device__ __forceinline__ void gate_logs(const float* __restrict__ gate, int ld
     L[t1] = sum;
 }
 
-// x[t][e] = src[(start + t) * ld + e] for t < count, zeros beyond; D floats to a row, `ldx` apart
-template <int THREADS>
-__device__ __forceinline__ void stage(float* x, int ldx, const float* __restrict__ src, int ld, int count, int cols) {
-    const int pieces = cols / 4;
-    for (int i = threadIdx.x; i < kQ * pieces; i += THREADS) {
-        const int t = i / pieces, e = (i - t * pieces) * 4;
-        cp_async16(x + t * ldx + e, src + (size_t)(t < count ? t : 0) * ld + e, t < count);
+// x[t][e] = src[(start + t) * ld + e] for t < count, zeros beyond; COLS floats to a row, `ldx` apart.  Every copy has an address register of its own:
+// copies that share one wait for one another's data (reads of a prompt of 2,048 tokens 79 -> 75 us)
+template <int THREADS, int COLS>
+__device__ __forceinline__ void stage(float* x, int ldx, const float* __restrict__ src, int ld, int count) {
+    constexpr int kPieces = COLS / 4, kCopies = (kQ * kPieces + THREADS - 1) / THREADS;
+    const float* from[kCopies];
+#pragma unroll
+    for (int j = 0; j < kCopies; ++j) {
+        const int i = threadIdx.x + j * THREADS, t = i / kPieces;
+        from[j] = src + (size_t)(t < count ? t : 0) * ld + (i - t * kPieces) * 4;
+    }
+#pragma unroll
+    for (int j = 0; j < kCopies; ++j) {
+        const int i = threadIdx.x + j * THREADS, t = i / kPieces;
+        if (kQ * kPieces % THREADS == 0 || t < kQ) cp_async16(x + t * ldx + (i - t * kPieces) * 4, from[j], t < count);
     }
 }
 
@@ -128,7 +136,7 @@ chunk_solve_kernel(const float* __restrict__ k, const float* __restrict__ v, con
     if (!k) return;
     const float* k0 = k + (size_t)c.start * ld + (size_t)(h / (H / G)) * D;
     const float* v0 = v + (size_t)c.start * ld + (size_t)h * V;
-    stage<256>(Ks, kLdK, k0, ld, c.count, D);
+    stage<256, D>(Ks, kLdK, k0, ld, c.count);
     cp_async_commit();
     if (tid < kQ) bt[tid] = tid < c.count ? beta[(size_t)(c.start + tid) * ld + h] : 0.f;
     cp_async_wait<0>();
@@ -287,12 +295,12 @@ chunk_walk_kernel(const float* __restrict__ k, const float* __restrict__ v, int 
             float* st = stages + (c & 1) * kStage;
             const size_t item = (size_t)(first_slot + c) * H + h;
             const int n0 = start + c * kQ, count = min(kQ, len - c * kQ);
-            stage<kThreads>(st, D, kh + (size_t)n0 * ld, ld, count, D);
+            stage<kThreads, D>(st, D, kh + (size_t)n0 * ld, ld, count);
             if (DELTA) {
-                stage<kThreads>(st + kQ * D, kVC, U + item * kQ * V + v0, V, kQ, kVC);
-                stage<kThreads>(st + kQ * D + kQ * kVC, D, W + item * kQ * D, D, kQ, D);
+                stage<kThreads, kVC>(st + kQ * D, kVC, U + item * kQ * V + v0, V, kQ);
+                stage<kThreads, D>(st + kQ * D + kQ * kVC, D, W + item * kQ * D, D, kQ);
             } else {
-                stage<kThreads>(st + kQ * D, kVC, v + (size_t)n0 * ld + (size_t)h * V + v0, ld, count, kVC);
+                stage<kThreads, kVC>(st + kQ * D, kVC, v + (size_t)n0 * ld + (size_t)h * V + v0, ld, count);
             }
             if (tid < kQ) fs[c & 1][tid] = fade[item * kQ + tid];
             if (tid == 0) es[c & 1] = whole[item];
@@ -445,8 +453,8 @@ chunk_read_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
     const Chunk c = chunk;
     if (c.count == 0) return;
     const size_t item = (size_t)c.slot * H + h, head = (size_t)(h / (H / G)) * D;
-    stage<256>(Qs, kLdQ, q + (size_t)c.start * ld + head, ld, c.count, D);
-    stage<256>(Xs, kLdQ, k + (size_t)c.start * ld + head, ld, c.count, D);
+    stage<256, D>(Qs, kLdQ, q + (size_t)c.start * ld + head, ld, c.count);
+    stage<256, D>(Xs, kLdQ, k + (size_t)c.start * ld + head, ld, c.count);
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
@@ -481,8 +489,8 @@ chunk_read_kernel(const float* __restrict__ q, const float* __restrict__ k, cons
         for (int j = 0; j < kTN; ++j) y[i][j] *= f;
     }
     __syncthreads();
-    if (U) stage<256>(Xs, kLdU, U + item * kQ * V + v0, V, kQ, VT);
-    else stage<256>(Xs, kLdU, v + (size_t)c.start * ld + (size_t)h * V + v0, ld, c.count, VT);
+    if (U) stage<256, VT>(Xs, kLdU, U + item * kQ * V + v0, V, kQ);
+    else stage<256, VT>(Xs, kLdU, v + (size_t)c.start * ld + (size_t)h * V + v0, ld, c.count);
     cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();

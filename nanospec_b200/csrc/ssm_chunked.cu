@@ -313,7 +313,7 @@ chunk_outputs_kernel(const float* __restrict__ C, const float* __restrict__ B, c
 // ---------------------------------------------------------------------------------------
 // The sums for heads of 64 features in groups of a multiple of four and states of 64 or 128 rows: a block takes four heads of a
 // group, so that B is staged once for them, and threads of 8 x 8 results (16 words of shared memory to 64 FMAs; 12 to 32 above).  The same
-// sums in the same order, bit for bit.  Prompts of 2,471 tokens in all, 64 heads of 64, a state of 128 rows, 8 groups: 103 us above, 80 here.
+// sums in the same order, bit for bit.  Prompts of 2,471 tokens in all, 64 heads of 64, a state of 128 rows, 8 groups: 103 us above, 77 here.
 // Not on the tensor cores (66 us): a head that forgets soon has sums of a few large terms, which a chain rounds to 5.5e-8 and truncation to 7e-8.
 // ---------------------------------------------------------------------------------------
 constexpr int kLd4 = 68;
@@ -323,6 +323,24 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) 
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int G> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(G) : "memory"); }
+// a chunk's rows of COLS floats by 256 threads, zeros beyond `count`.  Every copy has an address register of its own: copies that share one wait for
+// one another's data (chunk sums 81 -> 77 us)
+template <int COLS>
+__device__ __forceinline__ void rows_in(float* dst, int ldd, const float* __restrict__ src, int ld, int count) {
+    constexpr int kPieces = COLS / 4, kCopies = kQ * kPieces / 256;
+    static_assert(kQ * kPieces % 256 == 0, "a whole number of copies to a thread");
+    const float* from[kCopies];
+#pragma unroll
+    for (int j = 0; j < kCopies; ++j) {
+        const int i = threadIdx.x + j * 256, t = i / kPieces;
+        from[j] = src + (size_t)(t < count ? t : 0) * ld + (i % kPieces) * 4;
+    }
+#pragma unroll
+    for (int j = 0; j < kCopies; ++j) {
+        const int i = threadIdx.x + j * 256, t = i / kPieces;
+        cp_async16(dst + t * ldd + (i % kPieces) * 4, from[j], t < count);
+    }
+}
 
 // acc += a b^T, 8 x 8
 __device__ __forceinline__ void outer8(float (&acc)[8][8], const float4& a0, const float4& a1, const float4& b0, const float4& b1) {
@@ -356,16 +374,11 @@ chunk_states4_kernel(const float* __restrict__ B, const float* __restrict__ x, c
     const Chunk c = chunk;
     if (c.count == 0) return;
     const float* B0 = B + (size_t)c.start * ld + (size_t)g * N;
-    for (int i = tid; i < kQ * (N / 4); i += 256) {
-        const int t = i / (N / 4), e = (i % (N / 4)) * 4;
-        cp_async16(Bs + t * kLdB + e, B0 + (size_t)(t < c.count ? t : 0) * ld + e, t < c.count);
-    }
+    rows_in<N>(Bs, kLdB, B0, ld, c.count);
     const float* x0 = x + (size_t)c.start * ld + (size_t)h0 * 64;
     for (int p = 0; p < kPasses; ++p) {  // a group of copies to a pass, so that the first heads do not wait for the others
-        for (int i = tid; i < kAtOnce * kQ * 16; i += 256) {
-            const int hh = p * kAtOnce + i / (kQ * 16), t = (i >> 4) % kQ, e = (i & 15) * 4;
-            cp_async16(xs + (hh * kQ + t) * kLd4 + e, x0 + (size_t)(t < c.count ? t : 0) * ld + hh * 64 + e, t < c.count);
-        }
+#pragma unroll
+        for (int h = p * kAtOnce; h < (p + 1) * kAtOnce; ++h) rows_in<64>(xs + h * kQ * kLd4, kLd4, x0 + h * 64, ld, c.count);
         cp_async_commit();
     }
     if (warp < kHeads) {
