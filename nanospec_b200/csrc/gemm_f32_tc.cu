@@ -1,14 +1,14 @@
 // 32-bit matrix product on the 5th-generation tensor cores: y[M, N] = x[M, K] * w[N, K]^T, nothing rounded to less than 24 bits.
 //
-// Floats come apart into three bfloat16, a product of two into six products (csrc/float_parts.cuh).  The tensor core multiplies parts exactly and
+// Floats come apart into three bfloat16, exactly, a product of two into six products (csrc/float_parts.cuh).  The tensor core multiplies parts exactly and
 // adds them in float32, but it truncates, so its chains are kept short and small things go first: in every block of 64 k the five
 // products with a middle or a low part, then the four steps of high by high, into an accumulator that starts at zero; the block's sum
 // then joins its group's sum in registers, rounded to nearest, and the groups (eight at most, of at least 512 k, by K alone) are added in their order.
 //
 // An element's value depends on its row of x, its row of w and K: the order of its sums is the same for every M, every tile and every split, so
-// rows alone and in a batch give the same bits.  Parts of an infinity or a NaN make a NaN, and parts of numbers near the ends of the exponent's
-// range are lost; so an element that comes out infinite, NaN, or tiny and not zero is formed again from the floats themselves by its warp (32
-// chains of fmaf and their sum).
+// rows alone and in a batch give the same bits.  Parts are 2^24 times the floats, so that small ones keep all their bits; an infinity or a NaN among
+// them, numbers from 2^104 and sums from 2^80 on come out infinite or NaN, and such an element is formed again from the floats themselves by
+// its warp (32 chains of fmaf and their sum).
 //
 // The product is computed transposed, as in gemm_tcgen05.cu: 128 rows of w are the M side of tcgen05.mma, bn rows of x (16 to 96) its N side.
 // A block owns an SM and walks over tiles (blockIdx.x, + gridDim.x, ...; the tiles of the same rows of w are neighbours, so that w comes from DRAM
@@ -55,7 +55,6 @@ constexpr int kSmemMax = 227 * 1024;
 constexpr int kBarBytes = 384, kSmemFixed = 1024 + kBarBytes;  // barriers; alignment
 constexpr uint32_t kTmemCols = 512;              // two accumulators, then the stages of w's parts (32 columns to a part)
 constexpr uint32_t kPartsCols = kParts * kBK / 2;
-constexpr float kTiny = 8.077935669463161e-28f;  // 2^-90
 
 enum F32TcError { kErrF32Loader = 51, kErrF32Mma = 52, kErrF32Weights = 53, kErrF32Rows = 54, kErrF32Sum = 55, kErrF32Drain = 56 };
 
@@ -75,7 +74,7 @@ struct F32Gemm {
     int ring;  // stages of w's ring
 };
 
-__device__ __forceinline__ bool out_of_range(float v) { return !(fabsf(v) <= FLT_MAX) || (v != 0.f && fabsf(v) < kTiny); }
+__device__ __forceinline__ bool out_of_range(float v) { return !(fabsf(v) <= FLT_MAX); }
 // a warp's 32 results of row m (rows n_warp + lane of w), which it has written: those that the parts cannot give come from the floats
 __device__ __forceinline__ void mend_row(const F32Gemm& a, int m, int n_warp) {
     const int lane = threadIdx.x & 31;
@@ -418,7 +417,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
                 if (j < rows) {
-                    *out = all[j];
+                    *out = all[j] * kPartsBack;
                     odd |= out_of_range(all[j]);
                 }
                 out += a.ldy;
@@ -446,7 +445,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 const float p = ld_cluster_f32(mine + (uint32_t)(((q % per_rank) * bn + r) * kBM + at) * 4u, (uint32_t)(q / per_rank));
                 v = q == 0 ? p : v + p;
             }
-            if (n_warp + lane < a.N) a.y[(size_t)m * a.ldy + n_warp + lane] = v;
+            if (n_warp + lane < a.N) a.y[(size_t)m * a.ldy + n_warp + lane] = v * kPartsBack;
             if (__any_sync(0xffffffffu, out_of_range(v))) mend_row(a, m, n_warp);
         }
         cluster_sync();  // nobody leaves while its shared memory is read

@@ -603,7 +603,7 @@ chunk_outputs_tc_kernel(const float* __restrict__ C, const float* __restrict__ B
         for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int r = 0; r < 2; ++r)
-                *reinterpret_cast<float2*>(Sc + (t0 + quad + 8 * r) * kLdSc + sh * 32 + j * 8 + 2 * q) = make_float2(total[j][2 * r], total[j][2 * r + 1]);
+                *reinterpret_cast<float2*>(Sc + (t0 + quad + 8 * r) * kLdSc + sh * 32 + j * 8 + 2 * q) = make_float2(total[j][2 * r] * kPartsBack, total[j][2 * r + 1] * kPartsBack);
     }
     __syncthreads();  // the scores are there, B has been read
     const int v0 = (warp & 3) * 16, steps = (c.count + 15) >> 4;
@@ -718,7 +718,8 @@ chunk_outputs_tc_kernel(const float* __restrict__ C, const float* __restrict__ B
                 const int t = i * 16 + quad + 8 * r;
                 if (t < c.count)
                     *reinterpret_cast<float4*>(out + (size_t)(c.start + t) * ld_out + (size_t)h * 64 + v0 + q * 4) =
-                        make_float4(y[i][0][2 * r], y[i][1][2 * r], y[i][0][2 * r + 1], y[i][1][2 * r + 1]);
+                        make_float4(y[i][0][2 * r] * kPartsBack, y[i][1][2 * r] * kPartsBack, y[i][0][2 * r + 1] * kPartsBack,
+                                    y[i][1][2 * r + 1] * kPartsBack);
             }
     }
 }

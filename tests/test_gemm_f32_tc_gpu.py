@@ -35,7 +35,7 @@ def _operands(M, N, K, seed, spread=0):
 @pytest.mark.parametrize("K", [1024, 1028, 1092, 4160])  # whole groups; four past a block; a ragged last block; groups of unlike lengths
 @pytest.mark.parametrize("M,N", [(1, 1), (15, 127), (16, 128), (17, 129), (33, 300), (97, 260), (130, 20000)])
 def test_f32_tc_product(M, N, K):
-    """Against 64 bits: an element's products lose 2^-25 of themselves; a block's 24 additions truncate (2^-23 of what they reach), the K / 64 sums of
+    """Against 64 bits: an element's products lose 2^-24 of themselves; a block's 24 additions truncate (2^-23 of what they reach), the K / 64 sums of
     blocks and groups round.  And no further off, in the 2-norm, than the chain of fmaf.  Every tile and split, rows alone and rows that
     do not start on 16 bytes give the same bits; nothing beside the result is touched."""
     from nanospec_b200 import ops
@@ -73,15 +73,15 @@ def test_f32_tc_product(M, N, K):
 @pytest.mark.gpu
 @pytest.mark.parametrize("tiles", [(16, 1), (16, 2), (48, 1)])
 def test_f32_tc_infinities_and_ends_of_the_range(tiles):
-    """An element whose floats have no parts (an infinity, a NaN) or whose parts fall below the smallest numbers is what the floats themselves
-    give; every other element keeps its bits."""
+    """An element whose floats have no parts (an infinity, a NaN, the largest numbers) is what the floats themselves give, subnormal results are
+    as near as their spacing lets them be; every other element keeps its bits."""
     from nanospec_b200 import ops
     x, w = _operands(40, 200, 1024, 3)
     clean = torch.empty(40, 200, device=DEV)
     ops.linear_f32_tc(x, w, clean, tiles)
     y = x.clone()
     y[3, 7], y[5, 100], y[9] = float("nan"), float("inf"), 0.0
-    y[12] *= 2.0 ** -124  # parts of these are subnormal
+    y[12] *= 2.0 ** -124  # results of these are subnormal or nearly
     y[14, 0] = 3.4e38     # rounds to an infinite bfloat16
     v = w.clone()
     v[:, 0] *= 2.0 ** -10
@@ -101,6 +101,24 @@ def test_f32_tc_infinities_and_ends_of_the_range(tiles):
     ops.linear_f32_tc(x, v, same, tiles)
     rows = [m for m in range(40) if m not in (3, 5, 9, 12, 14)]
     assert torch.equal(got[rows][:, keep], same[rows][:, keep])
+    ops.check_kernel_errors()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tiles", [(16, 1), (16, 2), (48, 1)])
+@pytest.mark.parametrize("small,large", [(-109, 40), (-112, 60), (-124, 60), (-136, 80), (-146, 100), (50, 50), (-100, -20)])
+def test_f32_tc_small_and_large_operands(small, large, tiles):
+    """Small numbers on either side lose nothing, whatever the results are, zeros among them stay zeros, and sums beyond the parts' range come
+    from the floats: the bounds above (a chain of 32 fmaf and its five sums is below them)."""
+    from nanospec_b200 import ops
+    x, w = _operands(40, 200, 1024, 4)
+    x[7], w[11] = 0.0, 0.0
+    got = torch.empty(40, 200, device=DEV)
+    for a, b in ((small, large), (large, small)):
+        u, v = torch.ldexp(x, torch.tensor(a, device=DEV)), torch.ldexp(w, torch.tensor(b, device=DEV))
+        ops.linear_f32_tc(u, v, got, tiles)
+        ref, size = u.double() @ v.double().T, u.abs().double() @ v.abs().double().T
+        assert bool(((got.double() - ref).abs() <= size * 82 * 2.0 ** -24 + 2.0 ** -149).all())
     ops.check_kernel_errors()
 
 
