@@ -98,8 +98,8 @@ struct Roles {
 
 // x[M, K] -> parts[3][M][ldp]: high, middle, low; eight k to a thread, zeros from K to ldp
 __global__ void __launch_bounds__(256) f32_parts_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ parts, int M, int K, int ldx, int ldp, int pieces) {
-    ns_pdl_launch_dependents();
     ns_pdl_wait();
+    ns_pdl_launch_dependents();  // in this order: the product loads w without a wait of its own, and a kernel before this one may have written it
     const int per_row = ldp / 8;
     const size_t plane = (size_t)M * ldp;
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < (long long)M * per_row; i += (long long)gridDim.x * 256) {
@@ -186,7 +186,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     };
 
     if (warp == 0) {
-        // ---------------- w's floats (weights: no kernel of this stream writes them, so the loads need not wait for the predecessor) ----------------
+        // ---------------- w's floats: the predecessor, f32_parts_kernel, does not write them and has waited for all before it ----------------
         int g = 0;
         bool ok = true;
         for (int i = 0; ok && i < my_tiles; ++i) {

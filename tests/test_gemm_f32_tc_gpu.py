@@ -160,3 +160,24 @@ def test_f32_tc_late_weights():
             ops.linear_f32_tc(x, w, got, tiles)
             assert torch.equal(got, first)
     ops.check_kernel_errors()
+
+
+@pytest.mark.gpu
+def test_f32_tc_weights_just_written():
+    """w from this library's kernel directly before the product, one that starts its successor at once: the product sees all of it."""
+    from nanospec_b200 import ops
+    rounds = [_operands(8, 4096, 2048, seed) for seed in range(6)]
+    rounds = [(x, w.bfloat16()) for x, w in rounds]
+    want = []
+    for x, w in rounds:
+        want.append(torch.empty(8, 4096, device=DEV))
+        w32 = w.float()
+        torch.cuda.synchronize()
+        ops.linear(x, w32, want[-1])
+    w32, got = torch.empty(4096, 2048, device=DEV), [torch.empty(8, 4096, device=DEV) for _ in rounds]
+    torch.cuda.synchronize()
+    for (x, w), out in zip(rounds, got):
+        ops.cast_f32(w, w32)
+        ops.linear(x, w32, out)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    ops.check_kernel_errors()
