@@ -251,10 +251,10 @@ qk_norm_rope_once_kernel(__nv_bfloat16* __restrict__ qkv, int row_stride, const 
     const int e = turns ? it * 8 : 2 * rot_pairs + (it - rot_items) * 8;              // the piece's first feature
     __nv_bfloat16* row = qkv + (size_t)n * row_stride;
     const float* gain = is_k ? k_gain : q_gain;
-    const float freq = w < rot_pairs ? inv_freq[w] : 0.f;
     uint4 lo_raw, hi_raw, v_raw;  // (as they lie: registers decide how many blocks an SM holds)
     ns_pdl_wait();
     const int req = token_req[n], pos = positions[n];
+    const float freq = w < rot_pairs ? inv_freq[w] : 0.f;
     if (mine) {
         lo_raw = *reinterpret_cast<const uint4*>(row + h * d + e);
         if (rot) hi_raw = *reinterpret_cast<const uint4*>(row + h * d + e + rot_pairs);

@@ -51,3 +51,24 @@ def test_one_reading(nq, nkv, d, dv, pairs, write, gains, interleaved):
     assert torch.equal(got[0][0][:, width:], rows[:, width:]) and torch.equal(got[0][0][8], rows[8])
     if write:
         assert torch.equal(got[0][2], got[1][2]) and bool((got[0][2] != 7.0).any())
+
+
+def test_frequencies_just_written():
+    """Frequencies from this library's kernel directly before: the rotation sees them."""
+    from nanospec_b200 import ops
+    n, heads, d = 64, 8, 64
+    ctx = SimpleNamespace(positions=torch.arange(n, dtype=torch.int32, device=DEV), token_req=torch.zeros(n, dtype=torch.int32, device=DEV))
+    rows = torch.randn(n, heads * d, device=DEV).to(torch.bfloat16)
+    lane = SimpleNamespace(k=None, v=None, block_table=None, page_size=1)
+    tables = [(1e4 ** (-torch.arange(32, device=DEV) / (8.0 + i))).to(torch.bfloat16).view(1, 32) for i in range(8)]
+    freq, got, want = torch.empty(1, 32, device=DEV), [], []
+    for out, late in ((want, False), (got, True)):
+        for t in tables:
+            x = rows.clone()
+            torch.cuda.synchronize()
+            ops.cast_f32(t, freq)
+            if not late:
+                torch.cuda.synchronize()
+            ops.qk_norm_rope_store(x, ctx, lane, freq[0], 1.0, False, heads, 0, d, d, None, None, 1e-6, False)
+            out.append(x)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
