@@ -272,14 +272,30 @@ def f32_tiles(M: int, N: int, K: int, sms: int) -> tuple[int, int]:
     return best[1:]
 
 
+F32_PARTS_MAX = 1 << 28  # bytes of x's parts (one and a half times x): more rows go in runs, each of which reads w again
+
+
+def f32_runs(M: int, K: int, limit: int) -> list[tuple[int, int]]:
+    """(first row, rows) of the runs of a float32 product on the tensor cores: whole tiles of 96 rows while the parts stay within
+    `limit` bytes, at least one tile."""
+    step = max(96, limit // (48 * -(-K // 8)) // 96 * 96)
+    return [(m, min(step, M - m)) for m in range(0, M, step)]
+
+
+def _f32_plan(M: int, N: int, K: int, sms: int, limit: int) -> list[tuple[int, int, int, int]]:
+    """(first row, rows, rows of a tile, blocks to a tile) of every run."""
+    return [(m, rows, *f32_tiles(rows, N, K, sms)) for m, rows in f32_runs(M, K, limit)]
+
+
 def linear_f32_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tiles: tuple[int, int] | None = None) -> None:
     """The float32 product on the tensor cores (csrc/gemm_f32_tc.cu)."""
-    M, K = x.shape
-    N = w.shape[0]
-    rows, splits = tiles or f32_tiles(M, N, K, sm_count())
-    parts = torch.empty((3, M, -(-K // 8) * 8), dtype=torch.bfloat16, device=x.device)
-    lib.call("ns_gemm_f32_tc", x.data_ptr(), w.data_ptr(), out.data_ptr(), parts.data_ptr(), M, N, K, x.stride(0), w.stride(0), out.stride(0),
-             rows, splits, sm_count(), _tc(x.device).error.data_ptr(), _stream())
+    N, K = w.shape
+    ldx, ldy, sms = x.stride(0), out.stride(0), sm_count()
+    plan = _f32_plan(x.shape[0], N, K, sms, F32_PARTS_MAX)
+    parts = torch.empty(24 * plan[0][1] * -(-K // 8) if plan else 0, dtype=torch.bfloat16, device=x.device)
+    for m, M, *chosen in plan:
+        lib.call("ns_gemm_f32_tc", x.data_ptr() + 4 * m * ldx, w.data_ptr(), out.data_ptr() + 4 * m * ldy, parts.data_ptr(), M, N, K,
+                 ldx, w.stride(0), ldy, *(tiles or chosen), sms, _tc(x.device).error.data_ptr(), _stream())
 
 
 def linear_tensor_core(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, splits: int | None = None) -> bool:

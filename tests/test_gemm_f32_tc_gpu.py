@@ -23,6 +23,18 @@ def test_f32_tiles_fit():
         assert splits == 1 or (splits <= groups and -(-N // 128) * -(-M // rows) * splits <= 148 and -(-groups // splits) * rows <= 96)
 
 
+def test_f32_runs():
+    """The runs cover the rows once, in whole tiles but for the last, and their parts stay below the limit; a product of few rows is one run."""
+    from nanospec_b200 import ops
+    for M, K in ((1, 1024), (641, 8192), (16384, 14336), (100000, 1028), (500, 1 << 20), (200, 1 << 24)):
+        runs = ops.f32_runs(M, K, ops.F32_PARTS_MAX)
+        assert [m for m, _ in runs] == [0, *(m + n for m, n in runs[:-1])] and sum(n for _, n in runs) == M
+        assert all(n % 96 == 0 for _, n in runs[:-1])
+        assert runs[0][1] <= 96 or 6 * runs[0][1] * K <= ops.F32_PARTS_MAX
+        assert len(runs) == 1 or 6 * M * K > ops.F32_PARTS_MAX // 2
+    assert ops.f32_runs(0, 1024, 1) == []
+
+
 def _operands(M, N, K, seed, spread=0):
     g = torch.Generator(device=DEV).manual_seed(seed)
     x, w = torch.randn(M, K, generator=g, device=DEV), torch.randn(N, K, generator=g, device=DEV)
@@ -180,4 +192,22 @@ def test_f32_tc_weights_just_written():
         ops.cast_f32(w, w32)
         ops.linear(x, w32, out)
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+    ops.check_kernel_errors()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [97, 192, 300])
+def test_f32_tc_rows_in_runs(M, monkeypatch):
+    """More rows than the parts' limit go in runs, with the same bits, rows of x apart and on odd addresses too."""
+    from nanospec_b200 import ops
+    x, w = _operands(M, 260, 1028, M)
+    want, got = torch.empty(M, 260, device=DEV), torch.full((M, 263), 7.0, device=DEV)
+    ops.linear(x, w, want)
+    monkeypatch.setattr(ops, "F32_PARTS_MAX", 1 << 20)
+    assert len(ops.f32_runs(M, 1028, ops.F32_PARTS_MAX)) > 1
+    wide = torch.zeros(M, 1033, device=DEV)
+    wide[:, 3:1031] = x
+    for rows in (x, wide[:, 3:1031]):
+        ops.linear(rows, w, got[:, :260].fill_(float("nan")))
+        assert torch.equal(got[:, :260], want) and bool((got[:, 260:] == 7.0).all())
     ops.check_kernel_errors()
