@@ -5,6 +5,7 @@ except `linear` in bfloat16, which may hand a plain matrix product to cuBLAS.
 
 from __future__ import annotations
 
+import functools
 import math
 import threading
 from dataclasses import dataclass
@@ -282,8 +283,9 @@ def f32_runs(M: int, K: int, limit: int) -> list[tuple[int, int]]:
     return [(m, min(step, M - m)) for m in range(0, M, step)]
 
 
+@functools.lru_cache(maxsize=1024)
 def _f32_plan(M: int, N: int, K: int, sms: int, limit: int) -> list[tuple[int, int, int, int]]:
-    """(first row, rows, rows of a tile, blocks to a tile) of every run."""
+    """(first row, rows, rows of a tile, blocks to a tile) of every run.  Kept, since working it out takes the host as long as a launch."""
     return [(m, rows, *f32_tiles(rows, N, K, sms)) for m, rows in f32_runs(M, K, limit)]
 
 
