@@ -58,11 +58,41 @@ constexpr uint32_t kPartsCols = kParts * kBK / 2;
 
 enum F32TcError { kErrF32Loader = 51, kErrF32Mma = 52, kErrF32Weights = 53, kErrF32Rows = 54, kErrF32Sum = 55, kErrF32Drain = 56 };
 
-// an element from the floats themselves (every lane gets it); apart from the kernel's code, whose registers are counted
-__device__ __noinline__ float warp_dot(const float* __restrict__ x, const float* __restrict__ w, int K) {
-    float p = 0.f;
-    for (int k = threadIdx.x & 31; k < K; k += 32) p = fmaf(x[k], w[k], p);
-    return ns_warp_sum(p);
+// Elements from the floats themselves: a lane whose `mine` is set gets the product of x and row `lane` of w.  Four rows of w at a time; a NaN in x is
+// the result of them all, found in one reading of it.  Apart from the kernel's code, whose registers are counted.
+__device__ __noinline__ float warp_dots(const float* __restrict__ x, const float* __restrict__ w, int ldw, int K, bool mine) {
+    const int lane = threadIdx.x & 31;
+    unsigned who = __ballot_sync(0xffffffffu, mine);
+    bool nan = false;
+    for (int k = lane; k < K; k += 32) nan |= x[k] != x[k];
+    if (__any_sync(0xffffffffu, nan)) return __int_as_float(0x7fffffff);
+    float result = 0.f;
+    int last = 0;
+    while (who) {
+        int src[4];
+        float p[4];
+        const float* row[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {  // (fewer than four left: the last one again)
+            if (who) last = __ffs(who) - 1;
+            src[i] = last;
+            who &= who - 1;
+            row[i] = w + (size_t)src[i] * ldw;
+            p[i] = 0.f;
+        }
+#pragma unroll 4
+        for (int k = lane; k < K; k += 32) {
+            const float v = x[k];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) p[i] = fmaf(v, row[i][k], p[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            p[i] = ns_warp_sum(p[i]);
+            if (lane == src[i]) result = p[i];
+        }
+    }
+    return result;
 }
 
 struct F32Gemm {
@@ -80,11 +110,9 @@ __device__ __forceinline__ void mend_row(const F32Gemm& a, int m, int n_warp) {
     const int lane = threadIdx.x & 31;
     float* out = a.y + (size_t)m * a.ldy + n_warp + lane;
     const bool odd = n_warp + lane < a.N && out_of_range(*out);
-    for (unsigned who = __ballot_sync(0xffffffffu, odd); who; who &= who - 1) {
-        const int src = __ffs(who) - 1;
-        const float p = warp_dot(a.x + (size_t)m * a.ldx, a.w + (size_t)(n_warp + src) * a.ldw, a.K);
-        if (lane == src) *out = p;
-    }
+    if (!__any_sync(0xffffffffu, odd)) return;
+    const float p = warp_dots(a.x + (size_t)m * a.ldx, a.w + (size_t)n_warp * a.ldw, a.ldw, a.K, odd);
+    if (odd) *out = p;
 }
 
 // tiles of up to kBN rows of x: the roles' first warps, stages of both operands' parts
