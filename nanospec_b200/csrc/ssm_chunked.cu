@@ -11,6 +11,7 @@
 // Everything is float (the same operands as the token walk's: csrc/recurrent.cu), L and its differences double (or two floats), so that a
 // difference of two large sums keeps its digits.  A request's chunks start at its first token of the step; requests of fewer than min_len
 // tokens are left to the token walk.  Blocks find their (request, chunk) from the step's token offsets on the device.
+#include <cfloat>
 #include <type_traits>
 
 #include "chunks.cuh"
@@ -499,6 +500,35 @@ __device__ __forceinline__ void column_parts(const float2 (&v)[4], uint32_t (&b)
     }
 }
 
+// A token's 16 features from the floats themselves, by one warp: what the parts cannot give (infinities, the largest numbers), and tokens that a
+// later one's infinity or NaN reached through a weight of zero.  C, x, S, out: the token's, the chunk's and the head's first of these features.
+template <int N>
+__device__ __noinline__ void row_from_floats(const float* __restrict__ C, const float* __restrict__ B, const float* __restrict__ x,
+                                             const float* __restrict__ step, int ld, float a, const float* __restrict__ S, int t, float* out) {
+    const int lane = threadIdx.x & 31, f = lane & 15;
+    double whole = 0.0, after[2] = {0.0, 0.0};  // of the logarithms: all up to t, those behind tokens lane and lane + 32
+    for (int u = t; u >= 0; --u) {
+        const double l = -(double)(a * step[(size_t)u * ld]);
+        whole += l;
+        if (u > lane) after[0] += l;
+        if (u > lane + 32) after[1] += l;
+    }
+    float m[2] = {0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int s = lane + 32 * j;
+        if (s > t) continue;
+        float z = 0.f;
+        for (int n = 0; n < N; ++n) z = fmaf(C[n], B[(size_t)s * ld + n], z);
+        m[j] = z * (expf((float)after[j]) * step[(size_t)s * ld]);
+    }
+    float y = 0.f;
+    for (int n = 0; n < N; ++n) y = fmaf(C[n], S[n * 64 + f], y);
+    y *= expf((float)whole);
+    for (int s = 0; s <= t; ++s) y = fmaf(__shfl_sync(0xffffffffu, s < 32 ? m[0] : m[1], s & 31), x[(size_t)s * ld + f], y);
+    if (lane < 16) out[f] = y;
+}
+
 // grid (chunk slots, H / HEADS): four warps to a head (64 tokens x 16 features each), HEADS / 2 heads one after the other to each of two such
 // groups (one to one).  The next head's state and x come by cp.async while this one's products run: what a warp can keep in flight in
 // registers is 2.4 TB/s over the GPU.
@@ -616,6 +646,7 @@ chunk_outputs_tc_kernel(const float* __restrict__ C, const float* __restrict__ B
         for (int e = 0; e < 4; ++e) v[e] = *reinterpret_cast<const float2*>(at + (k0 + (e & 1) + (e >> 1) * 8) * kLd);
         column_parts(v, b);
     };
+    unsigned odd = 0;  // bit by head: something that this thread wrote is not finite
 #pragma unroll 1
     for (int hh = group; hh < HEADS; hh += O::kGroups) {
         const int h = h0 + hh;
@@ -711,16 +742,39 @@ chunk_outputs_tc_kernel(const float* __restrict__ C, const float* __restrict__ B
         } else {
             ns_pdl_launch_dependents();
         }
+        float zero = 0.f;  // as long as everything is finite
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 const int t = i * 16 + quad + 8 * r;
-                if (t < c.count)
-                    *reinterpret_cast<float4*>(out + (size_t)(c.start + t) * ld_out + (size_t)h * 64 + v0 + q * 4) =
-                        make_float4(y[i][0][2 * r] * kPartsBack, y[i][1][2 * r] * kPartsBack, y[i][0][2 * r + 1] * kPartsBack,
-                                    y[i][1][2 * r + 1] * kPartsBack);
+                const float4 v = make_float4(y[i][0][2 * r] * kPartsBack, y[i][1][2 * r] * kPartsBack, y[i][0][2 * r + 1] * kPartsBack,
+                                             y[i][1][2 * r + 1] * kPartsBack);
+                if (t < c.count) *reinterpret_cast<float4*>(out + (size_t)(c.start + t) * ld_out + (size_t)h * 64 + v0 + q * 4) = v;
+                zero = fmaf(v.x, 0.f, fmaf(v.y, 0.f, fmaf(v.z, 0.f, fmaf(v.w, 0.f, zero))));
             }
+        odd |= (unsigned)(zero != 0.f) << hh;
+    }
+    odd = __reduce_or_sync(0xffffffffu, odd);
+#pragma unroll 1
+    for (; odd; odd &= odd - 1) {  // rows that are not finite, from the floats
+        const int h = h0 + __ffs(odd) - 1;
+#pragma unroll 1
+        for (int k = 0; k < 8; ++k) {
+            const int first = (k >> 1) * 16 + 8 * (k & 1);
+            bool mine = false;
+            if (first + quad < c.count) {
+                const float4 v = *reinterpret_cast<const float4*>(out + (size_t)(c.start + first + quad) * ld_out + (size_t)h * 64 + v0 + q * 4);
+                mine = !(fabsf(v.x + v.y + (v.z + v.w)) <= FLT_MAX);  // (numbers are below 2^80 here: their sum is one)
+            }
+            for (unsigned who = __ballot_sync(0xffffffffu, mine); who;) {
+                const int row = (__ffs(who) - 1) >> 2, t = first + row;
+                who &= ~(15u << (4 * row));
+                row_from_floats<N>(C + (size_t)(c.start + t) * ld + (size_t)g * N, B + (size_t)c.start * ld + (size_t)g * N,
+                                   x + (size_t)c.start * ld + (size_t)h * 64 + v0, step + (size_t)c.start * ld + h, ld, expf(a_log[h]),
+                                   states + ((size_t)c.slot * H + h) * N * 64 + v0, t, out + (size_t)(c.start + t) * ld_out + (size_t)h * 64 + v0);
+            }
+        }
     }
 }
 
