@@ -295,12 +295,13 @@ moe_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                 }
             }
         }
-        if (rank == 0)
-            for (int i = max(0, g - kStages); i < g; ++i)  // both blocks' copies have landed before either leaves
-                if (!mbar_wait_warp(full_bar(i % kStages), (uint32_t)(i / kStages) & 1u)) {
-                    if (lane == 0) atomicExch(error_flag, kErrDrainWait);
-                    break;
-                }
+        // Before either block leaves, both blocks' copies have landed (the leader's barriers count them) and the leader's last commits have arrived
+        // at the other block's barriers (at its own: warp 1 below).
+        for (int i = max(0, g - kStages); i < g; ++i)
+            if (!mbar_wait_warp(rank == 0 ? full_bar(i % kStages) : empty_bar(i % kStages), (uint32_t)(i / kStages) & 1u)) {
+                if (lane == 0) atomicExch(error_flag, kErrDrainWait);
+                break;
+            }
     } else if (warp == 1) {
         if (rank == 0) {
             int g = 0, n = 0;
