@@ -23,18 +23,22 @@
 //   4-12 add a finished block's accumulator to their sums in registers (32 columns to a thread), add up groups, write results
 //
 // Weights that a checkpoint held in 16 bits have neither middle nor low parts.  Where a block's 128 x 64 of w have none, the three products with
-// them are left out: they are zeros, so the bits stay (641 x 16384 x 2048 213 -> 167 us).  The eight warps see the parts as they make them.
+// them are left out: they are zeros, so the bits stay (641 x 16384 x 2048 213 -> 163 us).  The eight warps see the parts as they make them.
 //
 // Microseconds on a B200 in a graph of such products (w from DRAM): the kernels of gemm_f32.cu, this one with its parts kernel on weights of 24 bits,
 // and on bfloat16's numbers
 //     M x N x K   1 x 2048 x 2048   8 x 2048 x 8192   3 x 32768 x 2048   200 x 8192 x 1024   641 x 2048 x 8192   641 x 16384 x 2048   8 x 1024 x 512
 //     fmaf               23                97                 89                 119                 709                 943                 7.0
-//     24 bits            11.5              26                 51                  32                 117                 213                 9.0
-//     bfloat16's         11.3              25                 51                  30                  94                 167                 9.0
-// From K = 1024 on it was slower nowhere (1 x 1024 x 1024: 11.8 / 10.5); that line is the dispatch's (F32_TC_MIN_K).  Groups that were added up in y
+//     24 bits            11.0              25                 51                  30                 120                 213                 9.0
+//     bfloat16's         10.8              24                 50                  27                  92                 163                 9.0
+// From K = 1024 on the GPU was slower nowhere (1 x 1024 x 1024: 11.6 / 10.5); that line is the dispatch's (F32_TC_MIN_K).  The host is: an eager product
+// of a few rows takes it 15 us, two launches and the parts' buffer, where one launch took 9.  Groups that were added up in y
 // (a read-modify-write of the tile for each) took 244 us instead of 213 on 641 x 16384 x 2048, 128 instead of 117 on 641 x 2048 x 8192.
 // Error against 64 bits (2-norm, normal x and w), one chain of fmaf / this kernel, in 1e-7: K = 1024 5.7 / 1.0, 2048 8.1 / 1.0, 8192 16 / 1.2,
-// 14336 21 / 1.4; numbers over 60 powers of two 7.0 / 1.3; all of one sign 6.3 / 0.9.
+// 14336 21 / 1.4; numbers over 60 powers of two 7.0 / 1.3; all of one sign 6.3 / 0.9.  Rows of x with few numbers that are not zero are the other way
+// round, since a chain of n fmaf rounds n times: with one 0.25 / 0.46, 4 0.41 / 0.59, 8 0.54 / 0.66, 16 0.74 / 0.72, 128 2.0 / 0.9.
+// Elements formed from the floats cost what they are: 641 x 16384 x 2048 with an infinity in every row 13 ms, with a NaN in every row (found once for
+// 32 elements) 0.75.
 // Bound, with 96 rows, by shared memory, which the MMAs' operand, TMA's writes and the reads of w share (24 bits: 1,700 cycles a block of k, of which
 // the MMAs run for 1,190; bfloat16's numbers: 1,290 and 600); with 16 rows (990 cycles) by taking w apart.
 //

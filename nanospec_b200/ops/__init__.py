@@ -1663,8 +1663,9 @@ MOE_TILE: int | None = None  # rows of a tile in `moe_grouped_tc` (None: by the 
 
 def moe_tile(E: int, n: int, ff: int) -> int:
     """Rows of a tile of the experts' products: 256 on pairs of SMs where an expert holds enough to fill most of one (32 experts of 116 rows, width
-    2048: 90 us against 83 in tiles of 128; of 124: 91 / 96) and there is more than a tile for each pair (16 of 300 rows, 72 tiles: 41 / 33; 4 of 700,
-    80 tiles: 48 / 53)."""
+    2048: 90 us against 83 in tiles of 128; of 124: 91 / 96) and the first product has a tile for each of the 74 pairs of 148 SMs and some to spare
+    (16 of 300 rows, 72 tiles: 41 / 33; 4 of 700, 80 tiles: 48 / 53).  A whole layer of experts in tiles of 256 on single SMs, as it was, and by this
+    rule: 16 experts of 500 rows 226 / 194 us, 4 of 1,000 140 / 132, 4 of 350 (tiles of 128 now) 120 / 122."""
     if n >= 120 * E and max(E, n // 256) * -(-ff // 128) >= 80:
         return 256
     return 128 if n > 24 * E else 32

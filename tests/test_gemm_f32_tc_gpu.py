@@ -135,6 +135,22 @@ def test_f32_tc_small_and_large_operands(small, large, tiles):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("terms", [1, 2, 8])
+def test_f32_tc_rows_of_few_terms(terms):
+    """Rows of x that are zero but for a few numbers: a product leaves out 2^-24 of itself, each of its high by high steps truncates once (2^-23 of
+    what is reached) and its block's sum joins with a rounding; what the small products truncate is a sixteenth of that."""
+    from nanospec_b200 import ops
+    x, w = _operands(70, 300, 2048, terms)
+    order = torch.rand(70, 2048, generator=torch.Generator().manual_seed(terms)).argsort(1).to(DEV)
+    x = torch.where(order < terms, x, 0.0)
+    got = torch.empty(70, 300, device=DEV)
+    ops.linear(x, w, got)
+    ref, size = x.double() @ w.double().T, x.abs().double() @ w.abs().double().T
+    assert bool(((got.double() - ref).abs() <= size * (1 + 3.2 * terms) * 2.0 ** -24).all())
+    ops.check_kernel_errors()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K,tiles", [(1, 128, 1024, (16, 2)), (33, 300, 1092, (48, 1)), (97, 257, 2048, (96, 1)), (20, 20000, 1024, (32, 1))])
 def test_f32_tc_weights_of_16_bits(M, N, K, tiles):
     """Products with parts of w that are zero are left out: such weights' elements stay within the bound, and keep their bits when another row of w's tile,
