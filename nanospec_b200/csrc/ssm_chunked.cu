@@ -423,7 +423,8 @@ chunk_states4_kernel(const float* __restrict__ B, const float* __restrict__ x, c
 // What several heads of a group or several warps read (B, C, the weights of x) lies as parts in shared memory; x and the state lie there as floats
 // and come apart on their way into the fragments of the one warp that multiplies them, a warp's columns of v dealt to its tiles in turn, so
 // that a thread's are neighbours.  A block takes four heads of a group where that still makes blocks enough, or one: the same sums, bit for bit.
-// Read-out of prompts of 2,471 tokens in all, 64 heads, a state of 128 rows: 191 us as FMAs, 123 here; 700 tokens, 8 heads: 31.6 / 12.0.  Error of y
+// Read-out of prompts of 2,471 tokens in all, 64 heads, a state of 128 rows: 191 us as FMAs, 125 here (2 of them to keep small
+// operands' bits and to look for rows that are not finite); 700 tokens, 8 heads: 31.6 / 12.0.  Error of y
 // against 64 bits 2.1e-7 / 1.2e-7.  Of a block's 44,000 cycles 18,000 are products (m16n8k16 at 8.2 cycles a sub-partition), 9,000 the weights of x,
 // 15,000 the way to the first product; one block an SM, whose two groups of warps overlap the first two.
 // ---------------------------------------------------------------------------------------
